@@ -14,6 +14,17 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// True in exactly one thread of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok));
+  return ok != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -145,26 +156,30 @@ __device__ __forceinline__ constexpr uint32_t umma_desc_hi_sw128(uint32_t sbo_by
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
   return ((smem_addr & 0x3FFFFu) >> 4) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
 }
-// `issue` selects the one lane that issues; the other lanes of the warp execute the instruction
-// predicated off, so the call can sit in warp-uniform code.
+// Call from code that one thread runs, selected with elect_one(): the compiler then knows that the
+// operands are uniform and issues back to back at the tensor pipe's own rate.  Measured, cycles per
+// instruction seen by one issuing thread (M = 128, K = 16; SS = A from shared memory, TS = A from
+// TMEM): SS N = 64 / 128 / 256: 48 / 64 / 128; TS N = 32 / 64 / 128: 16 / 32 / 64, and the same
+// next to busy FP32 warps on every scheduler.  A warp-wide loop with the instruction predicated on
+// `lane == 0` costs 93 whatever N is, and 200 next to busy warps.
 __device__ __forceinline__ void umma_ss_split(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi,
-                                              uint32_t idesc, uint32_t accumulate, bool issue = true) {
+                                              uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
       "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
-      "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(issue))
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void umma_ts_split(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi,
-                                              uint32_t idesc, uint32_t accumulate, bool issue = true) {
+                                              uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
       "mov.b64 db, {%2, %3};\n\t"
-      "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(issue))
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // Arrives on `bar` once every tcgen05.mma this thread issued so far has completed.

@@ -62,13 +62,13 @@ constexpr uint32_t kDescHi = umma_desc_hi_sw128(1024);
 // words of the tiles; a K=16 step advances 32 bytes inside a 64-column box, the second box of a
 // D=128 tile starts A_BOX / B_BOX bytes after the first.  The number of B rows (N) is in idesc.
 template <int D, int A_BOX, int B_BOX, int KS0 = 0, int KS1 = D / 16>
-__device__ __forceinline__ void gemm_ss(bool leader, uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+__device__ __forceinline__ void gemm_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
                                         bool accumulate) {
 #pragma unroll
   for (int ks = KS0; ks < KS1; ++ks) {
     const uint32_t a = a_lo + (((ks / 4) * A_BOX + (ks % 4) * 32) >> 4);
     const uint32_t b = b_lo + (((ks / 4) * B_BOX + (ks % 4) * 32) >> 4);
-    umma_ss_split(d_tmem, a, b, kDescHi, idesc, (accumulate || ks > 0) ? 1u : 0u, leader);
+    umma_ss_split(d_tmem, a, b, kDescHi, idesc, (accumulate || ks > 0) ? 1u : 0u);
   }
 }
 
@@ -77,13 +77,13 @@ __device__ __forceinline__ void gemm_ss(bool leader, uint32_t d_tmem, uint32_t a
 // 2048 bytes per step.  b_lo must carry the leading byte offset (distance between the tile's two
 // 64-column boxes; not used when the tile has a single box).
 template <int BN>
-__device__ __forceinline__ void gemm_ts(bool leader, uint32_t d_tmem, uint32_t a_region, uint32_t b_lo,
+__device__ __forceinline__ void gemm_ts(uint32_t d_tmem, uint32_t a_region, uint32_t b_lo,
                                         uint32_t idesc, bool accumulate) {
   constexpr int CH = BN / 32;
 #pragma unroll
   for (int s = 0; s < BN / 16; ++s) {
     const uint32_t a = a_region + (s / CH) * (BN / 2) + 8 * (s % CH);
-    umma_ts_split(d_tmem, a, b_lo + ((s * 2048) >> 4), kDescHi, idesc, (accumulate || s > 0) ? 1u : 0u, leader);
+    umma_ts_split(d_tmem, a, b_lo + ((s * 2048) >> 4), kDescHi, idesc, (accumulate || s > 0) ? 1u : 0u);
   }
 }
 

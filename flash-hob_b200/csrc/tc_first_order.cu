@@ -106,7 +106,7 @@ __device__ __forceinline__ void fo_split_pack(float x, float y, uint32_t& hi, ui
 }
 
 template <int A_BOX, int B_BOX>
-__device__ __forceinline__ void fo_gemm_ss_split(bool leader, uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo,
+__device__ __forceinline__ void fo_gemm_ss_split(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo,
                                                  uint32_t idesc, bool accumulate) {
 #pragma unroll
   for (int term = 0; term < 3; ++term) {   // (hi, hi), (hi, lo), (lo, hi)
@@ -114,7 +114,7 @@ __device__ __forceinline__ void fo_gemm_ss_split(bool leader, uint32_t d_tmem, u
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks)
       umma_ss_split(d_tmem, a_lo + ((ab * A_BOX + ks * 32) >> 4), b_lo + ((bb * B_BOX + ks * 32) >> 4), kDescHi, idesc,
-                    (accumulate || term > 0 || ks > 0) ? 1u : 0u, leader);
+                    (accumulate || term > 0 || ks > 0) ? 1u : 0u);
   }
 }
 
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
 
   if (warp == TMA_WARP) {
     // ================================================= TMA producer
-    if (lane == 0 && n_iter > 0) {
+    if (n_iter > 0 && elect_one()) {
       const int head_b = head / p.heads, head_h = head - head_b * p.heads;   // batch entry and head within it
       mbar_arrive_expect_tx(&bars->stat_full, C::STAT_BYTES);
 #pragma unroll
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
       }
     }
   } else if (warp == MMA_WARP || (warp == MMA_WARP2 && MODE != FO_LSE)) {
-    // ================================================= MMA issuers (whole warp runs the loop, one lane issues)
+    // ================================================= MMA issuers (one elected thread of each warp)
     // One thread cannot issue the products of a tile fast enough, so two warps share them.
     // Backward modes: warp 0 issues the S products and the output products, warp 1 the dP products;
     // warp 1 reuses the dP columns of a stage (they hold dS by then) only after warp 0 has issued
@@ -232,13 +232,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
     // issued the product that reads it.  The tensor pipe runs MMAs in the order they arrive.
     constexpr bool kSplitOutputs = C::kForward && MODE != FO_LSE;  // warp 1 issues the outputs
     const int role = warp == MMA_WARP ? 0 : 1;
-    if (n_iter > 0) {
-      const bool leader = lane == 0;
+    if (n_iter > 0 && elect_one()) {
       auto wait_all = [&](uint64_t* bar, uint32_t parity) {
-        return __all_sync(0xffffffffu, wait_bar(bar, parity, bars, status)) != 0;
+        return wait_bar(bar, parity, bars, status);
       };
       auto commit = [&](uint64_t* bar) {
-        if (leader) umma_commit(bar);
+        umma_commit(bar);
       };
       constexpr uint32_t idesc_s = umma_idesc_bf16(BM, BN, false, false, F16);
       constexpr uint32_t idesc_o0 = umma_idesc_bf16(BM, C::OUT0_COLS ? C::OUT0_COLS : 64, false, true, F16);  // O | dQ | dK
@@ -255,13 +254,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
       };
       // score product over KD columns (or over the hi/lo boxes of split operands)
       auto scores_mma = [&](auto kd, uint32_t d, uint32_t a, uint32_t b, bool accumulate) {
-        if constexpr (SPLIT) fo_gemm_ss_split<kStatBox, kStrmBox>(leader, d, a, b, idesc_s, accumulate);
-        else gemm_ss<decltype(kd)::value, kStatBox, kStrmBox>(leader, d, a, b, idesc_s, accumulate);
+        if constexpr (SPLIT) fo_gemm_ss_split<kStatBox, kStrmBox>(d, a, b, idesc_s, accumulate);
+        else gemm_ss<decltype(kd)::value, kStatBox, kStrmBox>(d, a, b, idesc_s, accumulate);
       };
       // output product, A = 16-bit tile in TMEM; split operands: A_hi . [B_hi | B_lo], then A_lo . B_hi
       auto outputs_mma = [&](uint32_t out, uint32_t a_region, uint32_t b, uint32_t idesc, bool accumulate) {
-        gemm_ts<BN>(leader, out, a_region, b, idesc, accumulate);
-        if constexpr (SPLIT) gemm_ts<BN>(leader, out, a_region + kLoTile, b, idesc_o64, true);
+        gemm_ts<BN>(out, a_region, b, idesc, accumulate);
+        if constexpr (SPLIT) gemm_ts<BN>(out, a_region + kLoTile, b, idesc_o64, true);
       };
       using KQ = std::integral_constant<int, DQK>;
       using KV = std::integral_constant<int, DV>;
@@ -286,7 +285,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
             outputs_mma(tmem_base, acc, mn_lo(sl, 1), idesc_o0, it > 0);  // O += P . V
             commit(&bars->strm_free[slot]);
             if (MODE == FO_ONE) commit(&bars->o_done);
-            if (leader) mbar_arrive(&bars->go[stage]);
+            mbar_arrive(&bars->go[stage]);
           }
         }
       } else if (role == 1) {
@@ -339,7 +338,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
               outputs_mma(tmem_base, acc + BN, mn_lo(sl, 0), idesc_o0, accum);                // dK += dS^T . Q
             }
             commit(&bars->strm_free[slot]);
-            if (C::NACC == 2 && leader) mbar_arrive(&bars->go[stage]);
+            if (C::NACC == 2) mbar_arrive(&bars->go[stage]);
           }
         }
       }
@@ -670,6 +669,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
   }
 
   // ---- teardown
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == MMA_WARP) {

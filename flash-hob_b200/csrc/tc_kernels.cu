@@ -209,7 +209,7 @@ __device__ __forceinline__ void split_pack(float x, float y, uint32_t& hi, uint3
 
 // D (+)= A . B^T for split operands: boxes (hi, hi), (hi, lo), (lo, hi), four K = 16 steps each.
 template <int A_BOX, int B_BOX>
-__device__ __forceinline__ void gemm_ss_split(bool leader, uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo,
+__device__ __forceinline__ void gemm_ss_split(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo,
                                               uint32_t idesc, bool accumulate) {
 #pragma unroll
   for (int term = 0; term < 3; ++term) {
@@ -218,7 +218,7 @@ __device__ __forceinline__ void gemm_ss_split(bool leader, uint32_t d_tmem, uint
     for (int ks = 0; ks < 4; ++ks) {
       const uint32_t a = a_lo + ((ab * A_BOX + ks * 32) >> 4);
       const uint32_t b = b_lo + ((bb * B_BOX + ks * 32) >> 4);
-      umma_ss_split(d_tmem, a, b, kDescHi, idesc, (accumulate || term > 0 || ks > 0) ? 1u : 0u, leader);
+      umma_ss_split(d_tmem, a, b, kDescHi, idesc, (accumulate || term > 0 || ks > 0) ? 1u : 0u);
     }
   }
 }
@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
 
   if (warp == TMA_WARP) {
     // ================================================= TMA producer
-    if (lane == 0 && n_iter > 0) {
+    if (n_iter > 0 && elect_one()) {
       const int head_b = head / p.heads, head_h = head - head_b * p.heads;   // batch entry and head within it
       mbar_arrive_expect_tx(&bars->stat_full, C::STAT_BYTES);
 #pragma unroll
@@ -487,17 +487,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
     }
   } else if (warp == MMA_WARP || warp == MMA_WARP2) {
     // ================================================= MMA issuers
-    // The whole warp runs the loop so that addresses and descriptors stay warp-uniform; one lane
-    // issues the MMAs and commits.  chain 0 = group A side, chain 1 = group B side.
+    // One elected thread waits, issues and commits.  chain 0 = group A side, chain 1 = group B side.
     const int chain = warp == MMA_WARP ? 0 : 1;
     const bool has_work = n_iter > 0 && (chain == 0 || PASS >= 2);
-    if (has_work) {
-      const bool leader = lane == 0;
+    if (has_work && elect_one()) {
       auto wait_all = [&](uint64_t* bar, uint32_t parity) {
-        return __all_sync(0xffffffffu, wait_bar(bar, parity, bars, p.status)) != 0;
+        return wait_bar(bar, parity, bars, p.status);
       };
       auto commit = [&](uint64_t* bar) {
-        if (leader) umma_commit(bar);
+        umma_commit(bar);
       };
       constexpr uint32_t idesc_s1 = umma_idesc_bf16(BM, BN, false, false, F16);      // one streamed tile
       constexpr uint32_t idesc_s2 = umma_idesc_bf16(BM, 2 * BN, false, false, F16);  // a stacked pair
@@ -518,8 +516,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
       bool ok = wait_all(&bars->stat_full, 0);
       // one score-shaped product: contraction over KD columns, or over hi/lo boxes for split operands
       auto scores = [&](auto kd, auto b_box, uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, bool accumulate) {
-        if constexpr (SPLIT) gemm_ss_split<kStatBox, decltype(b_box)::value>(leader, d, a, b, idesc, accumulate);
-        else gemm_ss<decltype(kd)::value, kStatBox, decltype(b_box)::value>(leader, d, a, b, idesc, accumulate);
+        if constexpr (SPLIT) gemm_ss_split<kStatBox, decltype(b_box)::value>(d, a, b, idesc, accumulate);
+        else gemm_ss<decltype(kd)::value, kStatBox, decltype(b_box)::value>(d, a, b, idesc, accumulate);
       };
       using KQ = std::integral_constant<int, DQK>;
       using KV = std::integral_constant<int, DV>;
@@ -539,7 +537,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
           if (kThirdIssuer) {
             // A2 += stat1 . strm0^T is issued by the third warp, strictly behind the stacked product
             // so that the order of the fp32 accumulation (and with it every result bit) is fixed
-            if (leader) mbar_arrive(&bars->a2_go);
+            mbar_arrive(&bars->a2_go);
           } else {
             if (early_s(PASS)) commit(&bars->s_ready);
             scores(KQ{}, Box0{}, acc + BN, stat_i(1), k_lo(sl, 0), idesc_s1, true);
@@ -581,8 +579,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
           // both 64-column halves of the accumulator (they are added in the epilogue), then
           // A_lo . B_hi goes on top of the first half
           auto outputs = [&](uint32_t out, uint32_t a_region, uint32_t b, uint32_t idesc, bool accumulate) {
-            gemm_ts<BN>(leader, out, a_region, b, idesc, accumulate);
-            if constexpr (SPLIT) gemm_ts<BN>(leader, out, a_region + 16, b, idesc_o64, true);
+            gemm_ts<BN>(out, a_region, b, idesc, accumulate);
+            if constexpr (SPLIT) gemm_ts<BN>(out, a_region + 16, b, idesc_o64, true);
           };
           if (chain == 0) {
             outputs(out1, acc + 1 * BN, mn_lo(sl, 2), idesc_o1, accum);              // ddP . V | dO
@@ -604,7 +602,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
             if (!ok) break;
             commit(&bars->s_full[chain]);
           }
-          if (chain == 0 && leader) mbar_arrive(&bars->chain_go);
+          if (chain == 0) mbar_arrive(&bars->chain_go);
         }
       }
       if (ok) {
@@ -620,10 +618,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
     }
   } else if (warp == MMA_WARP3) {
     // ================================================= third issuer: A2 += stat1 . strm0^T
-    if (kThirdIssuer && n_iter > 0) {
-      const bool leader = lane == 0;
+    if (kThirdIssuer && n_iter > 0 && elect_one()) {
       auto wait_all = [&](uint64_t* bar, uint32_t parity) {
-        return __all_sync(0xffffffffu, wait_bar(bar, parity, bars, p.status)) != 0;
+        return wait_bar(bar, parity, bars, p.status);
       };
       constexpr uint32_t idesc_s1 = umma_idesc_bf16(BM, BN, false, false, F16);
       constexpr int kStatBox = BM * 128;
@@ -640,17 +637,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
         tc_fence_after();
         const uint32_t acc = tmem_base + C::OUT_COLS + (PASS <= 2 ? stage * C::STAGE_COLS : 0);
         if constexpr (SPLIT)
-          gemm_ss_split<kStatBox, C::strm_box(0)>(leader, acc + BN, stat_lo + (C::stat_off(1) >> 4),
+          gemm_ss_split<kStatBox, C::strm_box(0)>(acc + BN, stat_lo + (C::stat_off(1) >> 4),
                                                   strm_lo + slot * kSlot16 + (C::strm_base(0) >> 4), idesc_s1, true);
         else
-          gemm_ss<DQK, kStatBox, C::strm_box(0)>(leader, acc + BN, stat_lo + (C::stat_off(1) >> 4),
+          gemm_ss<DQK, kStatBox, C::strm_box(0)>(acc + BN, stat_lo + (C::stat_off(1) >> 4),
                                                  strm_lo + slot * kSlot16 + (C::strm_base(0) >> 4), idesc_s1, true);
-        if (leader) {
-          umma_commit(&bars->s_full[stage]);
-          umma_commit(&bars->strm_free[slot]);
-        }
+        umma_commit(&bars->s_full[stage]);
+        umma_commit(&bars->strm_free[slot]);
       }
-      if (!ok && leader) {
+      if (!ok) {
         umma_commit(&bars->teardown[2]);
         const long long start = clock64();
         while (!mbar_try_wait(&bars->teardown[2], 0)) {
@@ -851,6 +846,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
   }
 
   // ---- teardown
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == MMA_WARP) {
