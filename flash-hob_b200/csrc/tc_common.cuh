@@ -23,7 +23,6 @@ constexpr int EW_THREADS = 256;
 constexpr int MMA_WARP = 0;   // issues the products of chain 1 (group A and the outputs it feeds); owns TMEM
 constexpr int MMA_WARP2 = 1;  // issues the products of chain 2 (group B and the outputs it feeds)
 constexpr int TMA_WARP = 2;
-constexpr int MMA_WARP3 = 3;  // issues A2 += stat1 . strm0^T behind chain 1's stacked product
 constexpr int EW_WARP0 = 4;   // elementwise warps 4..11
 constexpr int NTHREADS = 384;
 constexpr int TMEM_COLS = 512;

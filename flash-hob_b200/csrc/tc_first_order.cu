@@ -88,8 +88,7 @@ struct FoBars {
   uint64_t out_full;
   uint64_t o_done;      // ONE: the P V product of a tile has finished (O may be rescaled)
   uint64_t pair[4];     // ONE: the two warps that share 32 rows have both published their maximum
-  uint64_t go[2];       // BQ, BK: the outputs that read stage [i] have been issued (its dP columns may be reused)
-  uint64_t teardown[2];
+  uint64_t teardown;
   uint32_t tmem_base;
   int abort_flag;
   float red[2][2][BM];  // exchange of maxima / sums between the two column halves: [tile parity][half][row]
@@ -151,12 +150,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
       mbar_init(&bars->strm_free[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&bars->s_full[i], C::NACC);  // one commit per issuing warp
+      mbar_init(&bars->s_full[i], 1);
       mbar_init(&bars->s_free[i], EW_THREADS);
       mbar_init(&bars->p_full[i], EW_THREADS);
-      mbar_init(&bars->go[i], 1);
-      mbar_init(&bars->teardown[i], 1);
     }
+    mbar_init(&bars->teardown, 1);
     mbar_init(&bars->out_full, 1);
     mbar_init(&bars->o_done, 1);
     for (int i = 0; i < 4; ++i) mbar_init(&bars->pair[i], 64);
@@ -222,16 +220,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
         }
       }
     }
-  } else if (warp == MMA_WARP || (warp == MMA_WARP2 && MODE != FO_LSE)) {
-    // ================================================= MMA issuers (one elected thread of each warp)
-    // One thread cannot issue the products of a tile fast enough, so two warps share them.
-    // Backward modes: warp 0 issues the S products and the output products, warp 1 the dP products;
-    // warp 1 reuses the dP columns of a stage (they hold dS by then) only after warp 0 has issued
-    // the outputs that read them.  Forward modes with an output: warp 0 issues the S products,
-    // warp 1 the P V products; warp 0 reuses a stage (it holds P by then) only after warp 1 has
-    // issued the product that reads it.  The tensor pipe runs MMAs in the order they arrive.
-    constexpr bool kSplitOutputs = C::kForward && MODE != FO_LSE;  // warp 1 issues the outputs
-    const int role = warp == MMA_WARP ? 0 : 1;
+  } else if (warp == MMA_WARP) {
+    // ================================================= MMA issuer
+    // One elected thread issues every product: the tensor pipe runs the products of one thread in
+    // order, which is what makes overwriting a stage safe (its 16-bit tiles have been read by then).
     if (n_iter > 0 && elect_one()) {
       auto wait_all = [&](uint64_t* bar, uint32_t parity) {
         return wait_bar(bar, parity, bars, status);
@@ -266,41 +258,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
       using KV = std::integral_constant<int, DV>;
       bool ok = wait_all(&bars->stat_full, 0);
 
-      if (kSplitOutputs) {
-        for (int it = 0; ok && it < n_iter; ++it) {
-          const int slot = it % C::NSLOT, stage = it & 1;
-          const uint32_t acc = tmem_base + C::OUT_COLS + stage * C::STAGE_COLS;
-          const uint32_t sl = strm_lo + slot * kSlot16;
-          if (role == 0) {
-            if (it >= 2) ok = wait_all(&bars->go[stage], ((it - 2) >> 1) & 1);
-            ok = ok && wait_all(&bars->strm_full[slot], (it / C::NSLOT) & 1);
-            if (!ok) break;
-            tc_fence_after();
-            scores_mma(KQ{}, acc, stat_lo, sl, false);  // S
-            commit(&bars->s_full[stage]);
-          } else {
-            ok = wait_all(&bars->p_full[stage], (it >> 1) & 1) && wait_all(&bars->strm_full[slot], (it / C::NSLOT) & 1);
-            if (!ok) break;
-            tc_fence_after();
-            outputs_mma(tmem_base, acc, mn_lo(sl, 1), idesc_o0, it > 0);  // O += P . V
-            commit(&bars->strm_free[slot]);
-            if (MODE == FO_ONE) commit(&bars->o_done);
-            mbar_arrive(&bars->go[stage]);
-          }
-        }
-      } else if (role == 1) {
-        for (int it = 0; ok && it < n_iter; ++it) {
-          const int slot = it % C::NSLOT, stage = it & 1;
-          if (it >= 2) ok = wait_all(&bars->go[stage], ((it - 2) >> 1) & 1);
-          ok = ok && wait_all(&bars->strm_full[slot], (it / C::NSLOT) & 1);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t acc = tmem_base + C::OUT_COLS + stage * C::STAGE_COLS;
-          const uint32_t sl = strm_lo + slot * kSlot16;
-          scores_mma(KV{}, acc + BN, stat_lo + kStat16, sl + kStrm16, false);  // dP
-          commit(&bars->s_full[stage]);
-        }
-      } else {
+      {
         auto scores = [&](int it) -> bool {
           const int slot = it % C::NSLOT, stage = it & 1;
           if (!wait_all(&bars->strm_full[slot], (it / C::NSLOT) & 1)) return false;
@@ -309,6 +267,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
           const uint32_t acc = tmem_base + C::OUT_COLS + stage * C::STAGE_COLS;
           const uint32_t sl = strm_lo + slot * kSlot16;
           scores_mma(KQ{}, acc, stat_lo, sl, false);  // S
+          if (C::NACC == 2) scores_mma(KV{}, acc + BN, stat_lo + kStat16, sl + kStrm16, false);  // dP
           commit(&bars->s_full[stage]);
           if (MODE == FO_LSE) commit(&bars->strm_free[slot]);
           return true;
@@ -338,17 +297,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
               outputs_mma(tmem_base, acc + BN, mn_lo(sl, 0), idesc_o0, accum);                // dK += dS^T . Q
             }
             commit(&bars->strm_free[slot]);
-            if (C::NACC == 2) mbar_arrive(&bars->go[stage]);
           }
         }
       }
       if (ok) {
-        if (MODE != FO_LSE && role == (kSplitOutputs ? 1 : 0)) commit(&bars->out_full);
+        if (MODE != FO_LSE) commit(&bars->out_full);
       } else {
         // abort path: no tcgen05.mma may still be reading shared memory or TMEM at exit
-        commit(&bars->teardown[role]);
+        commit(&bars->teardown);
         const long long start = clock64();
-        while (!mbar_try_wait(&bars->teardown[role], 0)) {
+        while (!mbar_try_wait(&bars->teardown, 0)) {
           if (clock64() - start > kTimeoutCycles) break;
         }
       }

@@ -18,18 +18,23 @@
 //     pass 3: ddO += ddP . V + P . ddV   (after group A)     dQ2 += dS . ddK + dS2 . K     (after group B)
 //     pass 4: dV2 += ddP^T . dO          (after group A)     dK2 += dS^T . ddQ + dS2^T . Q (after group B)
 //
-// Warp roles (384 threads): warps 0, 1 and 3 = MMA issuers (one lane each; warp 0 also allocates
-// TMEM), warp 2 = TMA producer (one lane), warps 4-11 elementwise (warp w owns TMEM lanes
-// 32*(w%4).., column half (w-4)/4).  The products of a tile fall into two chains that never touch
-// the same TMEM columns - chain 1: group A -> P, ddP -> ddO | dV2; chain 2: group B -> dS, dS2 ->
-// dQ2 | dK2 - so each chain has its own issuing warp, on its own warp scheduler.  Issuing a
-// tcgen05.mma keeps a thread busy for about 51 cycles and the elementwise warps of the same
-// scheduler delay it further; one thread cannot feed 64-cycle products under that load.  For the
-// same reason, in passes 1 and 2 the second product of group A (A2 += stat1 . strm0^T) is issued
-// by a third warp, strictly behind chain 1's stacked product (the tensor pipe runs MMAs in the
-// order they arrive, so the accumulation order stays fixed and results stay bit-reproducible).
+// Warp roles (384 threads): warps 0 and 1 = MMA issuers (one elected thread each; warp 0 also
+// allocates TMEM), warp 2 = TMA producer (one thread), warp 3 idle, warps 4-11 elementwise (warp w
+// owns TMEM lanes 32*(w%4).., column half (w-4)/4).  The products of a tile fall into two chains -
+// chain 1: group A -> P, ddP -> ddO | dV2; chain 2: group B -> dS, dS2 -> dQ2 | dK2 - and each has
+// its own issuing thread, so that waiting for one chain's tiles never holds the other's products up.
+// Products of different threads reach the tensor pipe in no fixed order (an mbarrier arrival after
+// the issue does not order them), so all products that touch the same TMEM columns come from one
+// thread: that keeps the accumulation order fixed (results are bit-reproducible) and the reuse of
+// columns safe.
 //   passes 1, 2: two score stages in TMEM; the MMA warp runs one tile ahead.
-//   passes 3, 4: TMEM is full with one stage (2*D + 4*64 columns), so the tile is pipelined in
+//   passes 3, 4, head dims up to 64: three pairs of accumulators fit beside the outputs.  Group A
+//   has two pairs in turn and its products are issued two tiles ahead; group B has one, which is
+//   free again as soon as the elementwise warps have it in registers, because all four 16-bit tiles
+//   go into group A's pair (P, ddP into the first and dS, dS2 into the second half of each thread's
+//   columns).  The elementwise warps then never wait for a product that waits for them: N=2048,
+//   64 heads pass 3 335 -> 295 us, pass 4 359 -> 340 us.
+//   passes 3, 4 otherwise: TMEM is full with one stage (2*D + 4*64 columns), so the tile is pipelined in
 //   two halves instead: while the elementwise warps turn group A into P / ddP, the tensor core
 //   computes group B; while they turn group B into dS / dS2, it runs the group-A outputs and
 //   group A of the next tile.  The bf16 tiles overwrite their own accumulators in place.
@@ -62,6 +67,9 @@ struct Cfg {
   static constexpr int OUT1_COLS = NOUT ? DV : 0;    // ddO | dV2
   static constexpr int OUT_COLS = OUT0_COLS + OUT1_COLS;
   static constexpr int STAGE_COLS = NACC * BN;
+  // Passes 3, 4 with room for three pairs of score accumulators beside the outputs (both head dims
+  // up to 64): group A has two pairs in turn, group B one (see the kernel's header comment).
+  static constexpr bool DEEP_FITS = PASS >= 3 && OUT_COLS + 6 * BN <= TMEM_COLS;
   // score stages in TMEM: two for the reducing passes, one (pipelined in halves) for passes 3, 4
   static constexpr int NSS = PASS <= 2 ? ((TMEM_COLS - OUT_COLS) / STAGE_COLS >= 2 ? 2 : 1) : 1;
   __host__ __device__ static constexpr int stat_bytes(int i) { return BM * tile_d(i) * 2; }
@@ -120,12 +128,12 @@ struct Bars {
   uint64_t strm_free[4];
   uint64_t s_full[2];   // passes 1, 2: per score stage; passes 3, 4: [0] = group A done, [1] = group B done
   uint64_t s_free[2];   // passes 1, 2: stage consumed by the elementwise warps
-  uint64_t p_full[2];   // passes 3, 4: [0] = P/ddP written, [1] = dS/dS2 written
+  uint64_t p_full[2];   // passes 3, 4: [0] = P/ddP written, [1] = dS/dS2 written (deep: P/ddP of group-A stage [i])
+  uint64_t q_full[2];   // passes 3, 4 deep: dS/dS2 written into group-A stage [i]
   uint64_t out_full;
   uint64_t s_ready;      // passes 3, 4: the stacked product [S | Q.ddK^T] of a tile has finished
   uint64_t chain_go;     // passes 3, 4: chain 1 has issued its products of this round (chain 2 may follow)
-  uint64_t teardown[3];
-  uint64_t a2_go;        // chain 1 has issued the stacked product of a tile: the A2 product may follow
+  uint64_t teardown[2];
   uint32_t tmem_base;
   int abort_flag;
   float red[BM];
@@ -233,12 +241,12 @@ __device__ __forceinline__ void gemm_ss_split(uint32_t d_tmem, uint32_t a_lo, ui
 // (measured: pass 3 3-4 % faster; pass 4, which is at the register limit, up to 8 % slower).
 __host__ __device__ constexpr bool early_s(int pass) { return FHOB_EARLY_S && pass == 3; }
 
-template <int PASS, bool MASKED, bool F16, bool SPLIT, class B>
+template <int PASS, bool EARLY, bool MASKED, bool F16, bool SPLIT, class B>
 __device__ __forceinline__ bool ew_half_a(uint32_t acc, int col_base, int col_in_tile, const EwCtx& c,
                                           float2 (&ps)[16], float2 (&tt)[16], uint64_t* a2_full, uint32_t parity,
                                           B* bars, int* status) {
   constexpr bool kQStat = PASS != 4;
-  constexpr bool kEarlyS = early_s(PASS);
+  constexpr bool kEarlyS = EARLY;
   constexpr int BN = 64;
   uint32_t s[32], a2[32];
   tmem_ld32(acc + 0 * BN, s);
@@ -319,15 +327,22 @@ __device__ __forceinline__ bool ew_half_a(uint32_t acc, int col_base, int col_in
 
 // Second half: dP' = dP - D, X' = X - D*dd - b; writes P dP' and P (dP' t + X'), i.e. dS/scale and
 // dS2/scale: the factor `scale` is applied once to the finished dQ2 / dK2 accumulator instead.
+// `acc_b` holds [dP | X]; the two 16-bit tiles go to `dst_ds` and `dst_ds2`.  `loaded` (or NULL) is
+// arrived on as soon as dP and X are in registers.
 template <int PASS, bool MASKED, bool F16, bool SPLIT>
-__device__ __forceinline__ void ew_half_b(uint32_t acc, int col_base, int col_in_tile, const EwCtx& c,
-                                          const float2 (&ps)[16], const float2 (&tt)[16]) {
+__device__ __forceinline__ void ew_half_b(uint32_t acc_b, uint32_t dst_ds, uint32_t dst_ds2, uint64_t* loaded, int col_base,
+                                          int col_in_tile, const EwCtx& c, const float2 (&ps)[16],
+                                          const float2 (&tt)[16]) {
   constexpr bool kQStat = PASS != 4;
   constexpr int BN = 64;
   uint32_t dp[32], x[32];
-  tmem_ld32(acc + 2 * BN, dp);
-  tmem_ld32(acc + 3 * BN, x);
+  tmem_ld32(acc_b, dp);
+  tmem_ld32(acc_b + BN, x);
   tmem_wait_ld();
+  if (loaded) {
+    tc_fence_before();
+    mbar_arrive(loaded);
+  }
   uint32_t w_ds[16], w_ds2[16], w_ds_lo[16], w_ds2_lo[16];
 #pragma unroll
   for (int j4 = 0; j4 < 8; ++j4) {
@@ -362,11 +377,11 @@ __device__ __forceinline__ void ew_half_b(uint32_t acc, int col_base, int col_in
       }
     }
   }
-  tmem_st16(acc + 2 * BN, w_ds);
-  tmem_st16(acc + 3 * BN, w_ds2);
+  tmem_st16(dst_ds, w_ds);
+  tmem_st16(dst_ds2, w_ds2);
   if constexpr (SPLIT) {
-    tmem_st16(acc + 2 * BN + 16, w_ds_lo);
-    tmem_st16(acc + 3 * BN + 16, w_ds2_lo);
+    tmem_st16(dst_ds + 16, w_ds_lo);
+    tmem_st16(dst_ds2 + 16, w_ds2_lo);
   }
 }
 
@@ -376,9 +391,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
   static_assert(!SPLIT || (DQK == 128 && DV == 128 && !F16), "split fp32 operands are [hi(64) | lo(64)] bf16 rows");
   using C = Cfg<PASS, DQK, DV, BN>;
   constexpr bool kQStat = PASS != 4;
-  // passes 1, 2: a third warp issues the second product of group A (their tensor pipe has the room;
-  // in passes 3, 4 the extra issuer only delayed group A)
-  constexpr bool kThirdIssuer = PASS <= 2;
+  constexpr bool kDeep = C::DEEP_FITS && !SPLIT;
+  constexpr bool kEarly = early_s(PASS) && !kDeep;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* stat_tiles = smem;
   uint8_t* strm_tiles = smem + C::STAT_BYTES;
@@ -404,19 +418,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
     mbar_init(&bars->stat_full, 1);
     for (int i = 0; i < 4; ++i) {
       mbar_init(&bars->strm_full[i], 1);
-      mbar_init(&bars->strm_free[i], PASS == 1 ? 2 : (PASS == 2 ? 3 : 2));  // one commit per issuing warp
+      mbar_init(&bars->strm_free[i], PASS == 1 ? 1 : 2);  // one commit per issuing warp
     }
     for (int i = 0; i < 2; ++i) {
-      // commits per phase: in passes 1, 2 group A comes from two warps; pass 2 adds group B to the stage
-      mbar_init(&bars->s_full[i], PASS == 1 ? 2 : (PASS == 2 ? 3 : 1));
+      mbar_init(&bars->s_full[i], PASS == 2 ? 2 : 1);   // pass 2: groups A and B share a stage
       mbar_init(&bars->s_free[i], EW_THREADS);
       mbar_init(&bars->p_full[i], EW_THREADS);
+      mbar_init(&bars->q_full[i], EW_THREADS);
     }
     mbar_init(&bars->out_full, 2);
     mbar_init(&bars->chain_go, 1);
     mbar_init(&bars->s_ready, 1);
-    mbar_init(&bars->a2_go, 1);
-    mbar_init(&bars->teardown[2], 1);
     mbar_init(&bars->teardown[0], 1);
     mbar_init(&bars->teardown[1], 1);
     bars->abort_flag = 0;
@@ -527,26 +539,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
       // score-shaped products of this chain for tile `it` (waits for the tile's shared-memory slot)
       //   chain 0, group A: [S | stat0.strm1^T] as one N = 2*BN product, then A2 += stat1.strm0^T
       //   chain 1, group B: [dP | X] (one stacked product in passes 2, 3; two products in pass 4)
-      auto issue_scores = [&](int it, uint32_t acc) -> bool {
+      auto issue_scores = [&](int it, uint32_t acc, uint32_t acc_b) -> bool {
         const int slot = it % C::NSLOT;
         if (!wait_all(&bars->strm_full[slot], (it / C::NSLOT) & 1)) return false;
         tc_fence_after();
         const uint32_t sl = strm_lo + slot * kSlot16;
         if (chain == 0) {
           scores(KQ{}, Box0{}, acc, stat_lo, k_lo(sl, 0), idesc_s2, false);
-          if (kThirdIssuer) {
-            // A2 += stat1 . strm0^T is issued by the third warp, strictly behind the stacked product
-            // so that the order of the fp32 accumulation (and with it every result bit) is fixed
-            mbar_arrive(&bars->a2_go);
-          } else {
-            if (early_s(PASS)) commit(&bars->s_ready);
-            scores(KQ{}, Box0{}, acc + BN, stat_i(1), k_lo(sl, 0), idesc_s1, true);
-          }
+          if (kEarly) commit(&bars->s_ready);
+          scores(KQ{}, Box0{}, acc + BN, stat_i(1), k_lo(sl, 0), idesc_s1, true);
         } else if (PASS == 4) {
-          scores(KV{}, Box2{}, acc + 2 * BN, stat_i(2), k_lo(sl, 2), idesc_s1, false);
-          scores(KV{}, Box2{}, acc + 3 * BN, stat_i(3), k_lo(sl, 2), idesc_s1, false);
+          scores(KV{}, Box2{}, acc_b, stat_i(2), k_lo(sl, 2), idesc_s1, false);
+          scores(KV{}, Box2{}, acc_b + BN, stat_i(3), k_lo(sl, 2), idesc_s1, false);
         } else {
-          scores(KV{}, Box2{}, acc + 2 * BN, stat_i(2), k_lo(sl, 2), idesc_s2, false);
+          scores(KV{}, Box2{}, acc_b, stat_i(2), k_lo(sl, 2), idesc_s2, false);
         }
         return true;
       };
@@ -556,10 +562,49 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
           const int stage = it % C::NSS;
           const uint32_t acc = tmem_base + C::OUT_COLS + stage * C::STAGE_COLS;
           ok = wait_all(&bars->s_free[stage], ((it / C::NSS) & 1) ^ 1);
-          ok = ok && issue_scores(it, acc);
+          ok = ok && issue_scores(it, acc, acc + 2 * BN);
           if (!ok) break;
           commit(&bars->s_full[stage]);
           commit(&bars->strm_free[it % C::NSLOT]);
+        }
+      } else if (kDeep) {
+        // chain 0: group A two tiles ahead, and the output products; chain 1: group B, as soon as the
+        // elementwise warps have the previous [dP | X] in registers.
+        const uint32_t a_stages = tmem_base + C::OUT_COLS, acc_b = a_stages + 4 * BN;
+        const uint32_t out0 = tmem_base, out1 = tmem_base + C::OUT0_COLS;
+        if (chain == 0) {
+          for (int it = 0; ok && it < 2 && it < n_iter; ++it) {
+            ok = issue_scores(it, a_stages + it * 2 * BN, acc_b);
+            if (ok) commit(&bars->s_full[it]);
+          }
+          for (int it = 0; ok && it < n_iter; ++it) {
+            const uint32_t sl = strm_lo + (it % C::NSLOT) * kSlot16;
+            const uint32_t acc = a_stages + (it & 1) * 2 * BN;
+            const bool accum = it > 0;
+            ok = wait_all(&bars->p_full[it & 1], (it >> 1) & 1);
+            if (!ok) break;
+            tc_fence_after();
+            gemm_ts<BN>(out1, acc + BN, mn_lo(sl, 2), idesc_o1, accum);             // ddP . V | dO
+            if (kQStat) gemm_ts<BN>(out1, acc, mn_lo(sl, 3), idesc_o1, true);       // P . ddV
+            ok = wait_all(&bars->q_full[it & 1], (it >> 1) & 1);
+            if (!ok) break;
+            tc_fence_after();
+            gemm_ts<BN>(out0, acc + 16, mn_lo(sl, 1), idesc_o0, accum);             // dS  . ddK | ddQ
+            gemm_ts<BN>(out0, acc + BN + 16, mn_lo(sl, 0), idesc_o0, true);         // dS2 . K   | Q
+            commit(&bars->strm_free[it % C::NSLOT]);
+            if (it + 2 < n_iter) {
+              ok = issue_scores(it + 2, acc, acc_b);
+              if (ok) commit(&bars->s_full[it & 1]);
+            }
+          }
+        } else {
+          for (int it = 0; ok && it < n_iter; ++it) {
+            if (it > 0) ok = wait_all(&bars->s_free[0], (it - 1) & 1);
+            ok = ok && issue_scores(it, 0, acc_b);
+            if (!ok) break;
+            commit(&bars->s_ready);
+            commit(&bars->strm_free[it % C::NSLOT]);
+          }
         }
       } else {
         // One TMEM stage, pipelined per chain: scores(t) -> [elementwise half] -> outputs(t) ->
@@ -567,7 +612,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
         // MMAs execute in issue order, so scores(t+1) cannot overtake outputs(t).
         const uint32_t acc = tmem_base + C::OUT_COLS;
         const uint32_t out0 = tmem_base, out1 = tmem_base + C::OUT0_COLS;
-        ok = ok && issue_scores(0, acc);
+        ok = ok && issue_scores(0, acc, acc + 2 * BN);
         if (ok) commit(&bars->s_full[chain]);
         for (int it = 0; ok && it < n_iter; ++it) {
           const uint32_t sl = strm_lo + (it % C::NSLOT) * kSlot16;
@@ -598,7 +643,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
             if (!ok) break;
           }
           if (it + 1 < n_iter) {
-            ok = issue_scores(it + 1, acc);
+            ok = issue_scores(it + 1, acc, acc + 2 * BN);
             if (!ok) break;
             commit(&bars->s_full[chain]);
           }
@@ -616,44 +661,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
         }
       }
     }
-  } else if (warp == MMA_WARP3) {
-    // ================================================= third issuer: A2 += stat1 . strm0^T
-    if (kThirdIssuer && n_iter > 0 && elect_one()) {
-      auto wait_all = [&](uint64_t* bar, uint32_t parity) {
-        return wait_bar(bar, parity, bars, p.status);
-      };
-      constexpr uint32_t idesc_s1 = umma_idesc_bf16(BM, BN, false, false, F16);
-      constexpr int kStatBox = BM * 128;
-      const uint32_t stat_lo = umma_desc_lo(smem_u32(stat_tiles), 16);
-      const uint32_t strm_lo = umma_desc_lo(smem_u32(strm_tiles), 16);
-      constexpr uint32_t kSlot16 = C::SLOT_BYTES >> 4;
-      bool ok = wait_all(&bars->stat_full, 0);
-      for (int it = 0; ok && it < n_iter; ++it) {
-        const int slot = it % C::NSLOT;
-        const int stage = PASS <= 2 ? it % C::NSS : 0;
-        // chain 1 has waited for the stage and issued [S | stat0.strm1^T], which zero-initialises A2
-        ok = wait_all(&bars->a2_go, it & 1) && wait_all(&bars->strm_full[slot], (it / C::NSLOT) & 1);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t acc = tmem_base + C::OUT_COLS + (PASS <= 2 ? stage * C::STAGE_COLS : 0);
-        if constexpr (SPLIT)
-          gemm_ss_split<kStatBox, C::strm_box(0)>(acc + BN, stat_lo + (C::stat_off(1) >> 4),
-                                                  strm_lo + slot * kSlot16 + (C::strm_base(0) >> 4), idesc_s1, true);
-        else
-          gemm_ss<DQK, kStatBox, C::strm_box(0)>(acc + BN, stat_lo + (C::stat_off(1) >> 4),
-                                                 strm_lo + slot * kSlot16 + (C::strm_base(0) >> 4), idesc_s1, true);
-        umma_commit(&bars->s_full[stage]);
-        umma_commit(&bars->strm_free[slot]);
-      }
-      if (!ok) {
-        umma_commit(&bars->teardown[2]);
-        const long long start = clock64();
-        while (!mbar_try_wait(&bars->teardown[2], 0)) {
-          if (clock64() - start > kTimeoutCycles) break;
-        }
-      }
-    }
-  } else {
+  } else if (warp >= EW_WARP0) {
     // ================================================= elementwise warps
     const int quad = warp & 3, half = (warp - EW_WARP0) >> 2;
     const int row = quad * 32 + lane;
@@ -722,23 +730,30 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
           if (!ok) break;
           c.sv = smem_u32(strm_tiles + slot * C::SLOT_BYTES + C::STRM_BYTES);
         }
-        ok = __all_sync(0xffffffffu, wait_bar(early_s(PASS) ? &bars->s_ready : &bars->s_full[0], it & 1, bars, p.status));
+        // deep: group A of tile `it` in stage it & 1, group B in its own pair, dS and dS2 go to the
+        // unused halves of the thread's own S and A2 columns (P and ddP take the first 16 of 32)
+        const int st = kDeep ? it & 1 : 0;
+        const uint32_t phase = kDeep ? (it >> 1) & 1 : it & 1;
+        const uint32_t acc_a = acc + st * 2 * BN, acc_b = acc + (kDeep ? 4 : 2) * BN;
+        const uint32_t dst_ds = kDeep ? acc_a + 16 : acc_b, dst_ds2 = kDeep ? acc_a + BN + 16 : acc_b + BN;
+        ok = __all_sync(0xffffffffu, wait_bar(kEarly ? &bars->s_ready : &bars->s_full[st], phase, bars, p.status));
         if (!ok) break;
         tc_fence_after();
-        if (masked) ok = ew_half_a<PASS, true, F16, SPLIT>(acc, col_base, half * (BN / 2), c, ps, tt, &bars->s_full[0], it & 1, bars, p.status);
-        else ok = ew_half_a<PASS, false, F16, SPLIT>(acc, col_base, half * (BN / 2), c, ps, tt, &bars->s_full[0], it & 1, bars, p.status);
+        if (masked) ok = ew_half_a<PASS, kEarly, true, F16, SPLIT>(acc_a, col_base, half * (BN / 2), c, ps, tt, &bars->s_full[0], it & 1, bars, p.status);
+        else ok = ew_half_a<PASS, kEarly, false, F16, SPLIT>(acc_a, col_base, half * (BN / 2), c, ps, tt, &bars->s_full[0], it & 1, bars, p.status);
         if (!ok) break;
         tmem_wait_st();
         tc_fence_before();
-        mbar_arrive(&bars->p_full[0]);
-        ok = __all_sync(0xffffffffu, wait_bar(&bars->s_full[1], it & 1, bars, p.status));
+        mbar_arrive(&bars->p_full[st]);
+        ok = __all_sync(0xffffffffu, wait_bar(kDeep ? &bars->s_ready : &bars->s_full[1], it & 1, bars, p.status));
         if (!ok) break;
         tc_fence_after();
-        if (masked) ew_half_b<PASS, true, F16, SPLIT>(acc, col_base, half * (BN / 2), c, ps, tt);
-        else ew_half_b<PASS, false, F16, SPLIT>(acc, col_base, half * (BN / 2), c, ps, tt);
+        uint64_t* loaded = kDeep ? &bars->s_free[0] : nullptr;
+        if (masked) ew_half_b<PASS, true, F16, SPLIT>(acc_b, dst_ds, dst_ds2, loaded, col_base, half * (BN / 2), c, ps, tt);
+        else ew_half_b<PASS, false, F16, SPLIT>(acc_b, dst_ds, dst_ds2, loaded, col_base, half * (BN / 2), c, ps, tt);
         tmem_wait_st();
         tc_fence_before();
-        mbar_arrive(&bars->p_full[1]);
+        mbar_arrive(kDeep ? &bars->q_full[st] : &bars->p_full[1]);
       }
     }
 
