@@ -280,7 +280,7 @@ int fhob_pass12(const FhobProblem* p, void* stream) {
   int st = validate(p, false, true, true);
   if (st != FHOB_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (use_tc(*p)) return tc_pass(p->o ? 12 : 13, *p, s);
+  if (use_tc(*p)) return tc_pass(12, *p, s);
   st = simt_pass(1, *p, s);
   return st != FHOB_OK ? st : simt_pass(2, *p, s);
 }
@@ -290,18 +290,12 @@ int fhob_pass4(const FhobProblem* p, void* stream) { return run_pass(4, p, strea
 int fhob_bwdbwd(const FhobProblem* p, void* stream) {
   int st = validate(p, true, true, true);
   if (st != FHOB_OK) return st;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // tensor cores: dd and b come out of one sweep (sum_j P dP = D makes b linear in sums that need no
+  // dd), which also computes D and clears the status word, so there is no pre-pass
+  if (use_tc(*p)) return tc_operator(*p, s);
   st = run_prepass(p, stream);
   if (st != FHOB_OK) return st;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (use_tc(*p)) {
-    // dd and b come out of one sweep (sum_j P dP = D makes b linear in sums that need no dd)
-    const int kPasses[3] = {p->o ? 12 : 13, 3, 4};
-    for (int pass : kPasses) {
-      st = tc_pass(pass, *p, s);
-      if (st != FHOB_OK) return st;
-    }
-    return FHOB_OK;
-  }
   for (int pass = 1; pass <= 4; ++pass) {
     st = simt_pass(pass, *p, s);
     if (st != FHOB_OK) return st;
@@ -379,7 +373,6 @@ int fhob_forward(const FhobProblem* p, void* o_out, float* lse_out, void* stream
       int st = own_status_word(&status);
       if (st != FHOB_OK) return st;
     }
-    FHOB_CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), s));  // every call starts with a clean status word
     return tc_forward(*p, o_out, lse_out, status, s);
   }
   return simt_forward(*p, o_out, lse_out, s);

@@ -177,6 +177,7 @@ bool tc_split_supported(const FhobProblem& p);            // fp32 on the tensor 
 enum { kSplitQ = 1, kSplitDDQ = 2, kSplitDO = 4, kSplitK = 8, kSplitDDK = 16, kSplitV = 32, kSplitDDV = 64, kSplitAll = 127 };
 int tc_split_inputs(const FhobProblem& p, cudaStream_t s, int which = kSplitAll);  // writes hi/lo copies into the workspace
 int tc_pass(int pass, const FhobProblem& p, cudaStream_t s);
+int tc_operator(const FhobProblem& p, cudaStream_t s);   // the whole double backward
 
 // tensor-core forward (O, L) and first backward (dQ, dK, dV): tc_first_order.cu
 bool tc_first_order_supported(const FhobProblem& p);

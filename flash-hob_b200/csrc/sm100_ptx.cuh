@@ -25,6 +25,15 @@ __device__ __forceinline__ bool elect_one() {
   return ok != 0;
 }
 
+// ---------------------------------------------------------------- programmatic dependent launch
+// Blocks until the kernels this one was launched behind have completed and their memory is visible
+// (returns at once when the launch carries no such dependency).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel of the stream start its CTAs once every CTA of this one has come by here.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Orders this thread's view of global memory (generic proxy) before its later TMA and bulk copies.
+__device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <utility>
 
 #include "fhob_common.cuh"
 #include "sm100_ptx.cuh"
@@ -19,6 +20,7 @@ namespace {
 using namespace ptx;
 
 constexpr int BM = 128;
+constexpr int BOX_ROWS = 64;  // rows of a TMA box
 constexpr int EW_THREADS = 256;
 constexpr int MMA_WARP = 0;   // issues the products of chain 1 (group A and the outputs it feeds); owns TMEM
 constexpr int MMA_WARP2 = 1;  // issues the products of chain 2 (group B and the outputs it feeds)
@@ -94,7 +96,36 @@ __device__ __forceinline__ float2 f2(uint32_t lo, uint32_t hi) {
   return make_float2(__uint_as_float(lo), __uint_as_float(hi));
 }
 
+// Loads `ROWS` rows x D columns starting at row `y` of one head: boxes of 64 columns x 64 rows; a
+// tile's 64-column blocks are BOX bytes apart, rows are 128 bytes inside a block.
+template <int ROWS, int D, int BOX>
+__device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int y, int head, int batch) {
+  static_assert(ROWS % BOX_ROWS == 0, "whole boxes");
+#pragma unroll
+  for (int bx = 0; bx < D / 64; ++bx)
+#pragma unroll
+    for (int by = 0; by < ROWS / BOX_ROWS; ++by)
+      tma_load_4d(dst + bx * BOX + by * (BOX_ROWS * 128), map, bar, bx * 64, y + by * BOX_ROWS, head, batch);
+}
+
 // ------------------------------------------------------------------ host side
+// Launches with programmatic stream serialization: the kernel's CTAs may start while the kernel in
+// front of it drains (it says pdl_launch_dependents), and wait in pdl_wait before they touch memory.
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -112,20 +143,21 @@ EncodeTiledFn encode_fn() {
 }
 
 // 16-bit matrix of `n` rows x `d` columns per head, heads and batch entries at the strides of `v`:
-// a 4-D map (d, n, heads, batches), box = 64 columns x `rows` rows of one head, 128-byte swizzle.
+// a 4-D map (d, n, heads, batches), box = 64 columns x 64 rows of one head, 128-byte swizzle.  Taller
+// tiles take several boxes, so one map per tensor serves every kernel of a call.
 // Encoded maps are kept in a small per-thread table: a training step calls the operator with the
 // same tensors again and again, and an encode costs a few microseconds of host time per map.
 struct MapKey {
   const void* base;
-  int n, d, rows, f16, heads, batches;
+  int n, d, f16, heads, batches;
   long long row, head, batch;
   bool operator==(const MapKey& o) const {
-    return base == o.base && n == o.n && d == o.d && rows == o.rows && f16 == o.f16 && heads == o.heads &&
+    return base == o.base && n == o.n && d == o.d && f16 == o.f16 && heads == o.heads &&
            batches == o.batches && row == o.row && head == o.head && batch == o.batch;
   }
 };
 
-int make_map(CUtensorMap* m, const void* base, const View& v, int n, int d, int rows, bool f16) {
+int make_map(CUtensorMap* m, const void* base, const View& v, int n, int d, bool f16) {
   constexpr int kSlots = 64;
   struct Entry {
     MapKey key;
@@ -133,7 +165,7 @@ int make_map(CUtensorMap* m, const void* base, const View& v, int n, int d, int 
   };
   static thread_local Entry table[kSlots];
   static thread_local int used = 0, next = 0;
-  const MapKey key{base, n, d, rows, f16 ? 1 : 0, v.heads, v.batches, v.row, v.head, v.batch};
+  const MapKey key{base, n, d, f16 ? 1 : 0, v.heads, v.batches, v.row, v.head, v.batch};
   for (int i = 0; i < used; ++i)
     if (table[i].key == key) {
       *m = table[i].map;
@@ -150,7 +182,7 @@ int make_map(CUtensorMap* m, const void* base, const View& v, int n, int d, int 
                         static_cast<cuuint64_t>(v.batches)};
   cuuint64_t strides[3] = {static_cast<cuuint64_t>(v.row) * 2, static_cast<cuuint64_t>(v.head) * 2,
                            static_cast<cuuint64_t>(v.batch) * 2};
-  cuuint32_t box[4] = {64, static_cast<cuuint32_t>(rows), 1, 1};
+  cuuint32_t box[4] = {64, BOX_ROWS, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(m, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

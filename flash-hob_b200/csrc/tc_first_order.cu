@@ -63,18 +63,20 @@ struct FoCfg {
   static_assert((DQK == 64 || DQK == 128) && (DV == 64 || DV == 128), "head dims");
 };
 
+enum { kFoQ = 0, kFoDO, kFoK, kFoV, kFoMaps };
+
 struct FoParams {
-  CUtensorMap stat[2];
-  CUtensorMap strm[2];
+  CUtensorMap map[kFoMaps];
   const float* nlc;   // BQ, BK: -L*log2(e) per query
   const float* k1;    // BQ, BK: -D per query
-  float* lse_out;     // LSE
-  uint16_t* out0;     // ONE: O;  BQ: dQ;  BK: dK
-  uint16_t* out1;     // BK: dV
+  float* lse_out;     // ONE, LSE
+  void *o, *dq, *dk, *dv;
   int* status;
-  int n_q, n_k, causal, window, tiles_per_head;
-  int heads;            // heads per batch entry of the input tensor maps (4-D: columns, rows, head, batch)
-  int d_out0, d_out1;   // columns of the results in memory (<= the tile widths; see fo_launch)
+  int n_q, n_k, causal, window;
+  int tiles_q, tiles_k;   // 128-row tiles of a head
+  int q_blocks;           // BQ and BK in one launch: the first q_blocks CTAs are BQ
+  int heads;              // heads per batch entry of the input tensor maps (4-D: columns, rows, head, batch)
+  int d, d_v;             // columns in memory (<= the tile widths; see fo_fill)
   float scale;
 };
 
@@ -117,8 +119,9 @@ __device__ __forceinline__ void fo_gemm_ss_split(uint32_t d_tmem, uint32_t a_lo,
   }
 }
 
-template <int MODE, int DQK, int DV, bool F16, bool SPLIT = false>
-__global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__ FoParams p) {
+// One mode over one 128-row tile of one head; `block` numbers the (head, tile) pairs of the mode.
+template <int MODE, int DQK, int DV, bool F16, bool SPLIT>
+__device__ __forceinline__ void fo_body(const FoParams& p, int block) {
   using C = FoCfg<MODE, DQK, DV>;
   static_assert(!SPLIT || (DQK == 128 && DV == 128 && !F16), "split fp32 operands are [hi(64) | lo(64)] bf16 rows");
   constexpr bool kQStat = C::kQStat;
@@ -131,9 +134,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
   int* status = p.status;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int head = blockIdx.x / p.tiles_per_head;
-  const int tile_in_head = blockIdx.x - head * p.tiles_per_head;
-  const int tile = kQStat ? p.tiles_per_head - 1 - tile_in_head : tile_in_head;  // causal: longest first
+  const int tiles_per_head = kQStat ? p.tiles_q : p.tiles_k;
+  const int head = block / tiles_per_head;
+  const int tile_in_head = block - head * tiles_per_head;
+  const int tile = kQStat ? tiles_per_head - 1 - tile_in_head : tile_in_head;  // causal: longest first
   const int m0 = tile * BM;
   const int n_stat = kQStat ? p.n_q : p.n_k;
   const int n_strm = kQStat ? p.n_k : p.n_q;
@@ -142,8 +146,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
   visible_tiles(kQStat, m0, BM, BN, n_strm, off, p.causal, p.window, t_begin, t_end);
   const int n_iter = t_end - t_begin;
 
+  auto stat_map = [&](int i) { return &p.map[kQStat ? kFoQ + i : kFoK + i]; };   // Q, dO | K, V
+  auto strm_map = [&](int i) { return &p.map[kQStat ? kFoK + i : kFoQ + i]; };
+
+  int fault = 0;   // thread 0: what to report at the end
   if (threadIdx.x == 0) {
-    if (smem_u32(smem) & 1023u) atomicOr(status, FHOB_ERR_SMEM_ALIGN);
+    if (smem_u32(smem) & 1023u) fault |= FHOB_ERR_SMEM_ALIGN;
     mbar_init(&bars->stat_full, 1);
     for (int i = 0; i < 4; ++i) {
       mbar_init(&bars->strm_full[i], 1);
@@ -166,8 +174,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
     tmem_relinquish();
   }
   if (warp == TMA_WARP && lane == 0) {
-    for (int i = 0; i < C::NSTAT; ++i) prefetch_tensormap(&p.stat[i]);
-    for (int i = 0; i < C::NSTRM; ++i) prefetch_tensormap(&p.strm[i]);
+    for (int i = 0; i < C::NSTAT; ++i) prefetch_tensormap(stat_map(i));
+    for (int i = 0; i < C::NSTRM; ++i) prefetch_tensormap(strm_map(i));
   }
   tc_fence_before();
   __syncthreads();
@@ -175,18 +183,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
   // the CTA allocates all 512 columns, so the allocation starts at column 0 (checked)
   constexpr uint32_t tmem_base = 0;
   if (threadIdx.x == 0 && *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base) != 0)
-    atomicOr(status, FHOB_ERR_TMEM_BASE);
+    fault |= FHOB_ERR_TMEM_BASE;
+  // Everything up to here overlaps the end of the kernel in front; from here on memory is touched.
+  pdl_wait();
+  if (threadIdx.x == 0) {
+    pdl_launch_dependents();
+    if (C::kForward && block == 0) *status = 0;   // every call starts clean (the backward's pre-pass has done it)
+  }
 
   if (warp == TMA_WARP) {
     // ================================================= TMA producer
     if (n_iter > 0 && elect_one()) {
       const int head_b = head / p.heads, head_h = head - head_b * p.heads;   // batch entry and head within it
+      if (MODE == FO_BK) fence_proxy_async_global();   // the row vectors the bulk copies read were written by a kernel in front
       mbar_arrive_expect_tx(&bars->stat_full, C::STAT_BYTES);
 #pragma unroll
-      for (int i = 0; i < C::NSTAT; ++i)
-        for (int bx = 0; bx < C::tile_d(i) / 64; ++bx)
-          tma_load_4d(stat_tiles + C::stat_off(i) + bx * (BM * 128), &p.stat[i], &bars->stat_full, bx * 64, m0,
-                      head_h, head_b);
+      for (int i = 0; i < C::NSTAT; ++i) {
+        if (i == 0) load_tile<BM, DQK, BM * 128>(stat_tiles, stat_map(0), &bars->stat_full, m0, head_h, head_b);
+        else load_tile<BM, DV, BM * 128>(stat_tiles + C::stat_off(1), stat_map(1), &bars->stat_full, m0, head_h, head_b);
+      }
       int issued = 0;
       for (int it = 0; it < n_iter; ++it) {
         const int slot = it % C::NSLOT;
@@ -195,10 +210,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
         uint8_t* dst = strm_tiles + slot * C::SLOT_BYTES;
         const int n0 = (t_begin + it) * BN;
 #pragma unroll
-        for (int i = 0; i < C::NSTRM; ++i)
-          for (int bx = 0; bx < C::tile_d(i) / 64; ++bx)
-            tma_load_4d(dst + C::strm_off(i) + bx * (BN * 128), &p.strm[i], &bars->strm_full[slot], bx * 64, n0,
-                        head_h, head_b);
+        for (int i = 0; i < C::NSTRM; ++i) {
+          if (i == 0) load_tile<BN, DQK, BN * 128>(dst, strm_map(0), &bars->strm_full[slot], n0, head_h, head_b);
+          else load_tile<BN, DV, BN * 128>(dst + C::strm_off(1), strm_map(1), &bars->strm_full[slot], n0, head_h, head_b);
+        }
         if (MODE == FO_BK) {
           const size_t vo = static_cast<size_t>(head) * row_stride(p.n_q) + n0;
           uint8_t* sv = dst + C::STRM_BYTES;
@@ -562,9 +577,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
       if (ok) {
         // result o: `width` columns starting at TMEM column col0; dS was stored without the scale; the
         // single-sweep forward divides by the row sum here
-        auto store_out = [&](auto width, int d_mem, uint32_t col0, uint16_t* base, float mul) {
+        auto store_out = [&](auto width, int d_mem, uint32_t col0, void* base, float mul) {
           constexpr int DO = decltype(width)::value;   // columns of the accumulator; d_mem <= DO of them exist in memory
-          uint16_t* dst = base + (static_cast<size_t>(head) * n_stat + (g_row < n_stat ? g_row : 0)) * d_mem + half * (DO / 2);
+          uint16_t* dst = static_cast<uint16_t*>(base) + (static_cast<size_t>(head) * n_stat + (g_row < n_stat ? g_row : 0)) * d_mem + half * (DO / 2);
 #pragma unroll
           for (int ch = 0; ch < DO / 32; ++ch) {
             uint32_t v[16];
@@ -588,8 +603,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
           }
         };
         // split operands: 64 fp32 columns, the sum of the two 64-column halves of the accumulator
-        auto store_out_split = [&](int d_mem, uint32_t col0, uint16_t* base16, float mul) {
-          float* dst = reinterpret_cast<float*>(base16) +
+        auto store_out_split = [&](int d_mem, uint32_t col0, void* base, float mul) {
+          float* dst = static_cast<float*>(base) +
                        (static_cast<size_t>(head) * n_stat + (g_row < n_stat ? g_row : 0)) * d_mem + half * 32;
 #pragma unroll
           for (int ch = 0; ch < 2; ++ch) {
@@ -615,12 +630,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
           }
         };
         const float mul0 = MODE == FO_ONE ? inv_l : p.scale;
+        void* out0 = MODE == FO_ONE ? p.o : (MODE == FO_BQ ? p.dq : p.dk);
+        const int d_out0 = MODE == FO_ONE ? p.d_v : p.d;
         if constexpr (SPLIT) {
-          store_out_split(p.d_out0, 0, p.out0, mul0);
-          if (C::NOUT == 2) store_out_split(p.d_out1, C::OUT0_COLS, p.out1, 1.f);
+          store_out_split(d_out0, 0, out0, mul0);
+          if (C::NOUT == 2) store_out_split(p.d_v, C::OUT0_COLS, p.dv, 1.f);
         } else {
-          store_out(std::integral_constant<int, (C::OUT0_COLS ? C::OUT0_COLS : 64)>{}, p.d_out0, 0, p.out0, mul0);
-          if constexpr (C::NOUT == 2) store_out(std::integral_constant<int, DV>{}, p.d_out1, C::OUT0_COLS, p.out1, 1.f);
+          store_out(std::integral_constant<int, (C::OUT0_COLS ? C::OUT0_COLS : 64)>{}, d_out0, 0, out0, mul0);
+          if constexpr (C::NOUT == 2) store_out(std::integral_constant<int, DV>{}, p.d_v, C::OUT0_COLS, p.dv, 1.f);
         }
       }
     }
@@ -634,54 +651,56 @@ __global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
+  if (threadIdx.x == 0 && fault) atomicOr(status, fault);
 }
 
-template <int MODE, int DQK, int DV, bool F16, bool SPLIT = false>
-int fo_launch(const FhobProblem& p, FoParams& tp, cudaStream_t s) {
-  using C = FoCfg<MODE, DQK, DV>;
-  const void* q_side[2] = {p.q, p.d_o};
-  const void* k_side[2] = {p.k, p.v};
+template <int MODE, int DQK, int DV, bool F16, bool SPLIT>
+__global__ void __launch_bounds__(NTHREADS, 1) fo_kernel(const __grid_constant__ FoParams p) {
+  fo_body<MODE, DQK, DV, F16, SPLIT>(p, blockIdx.x);
+}
+
+// Both halves of the first backward in one launch (neither needs the other).
+template <int DQK, int DV, bool F16, bool SPLIT>
+__global__ void __launch_bounds__(NTHREADS, 1) fo_backward_kernel(const __grid_constant__ FoParams p) {
+  const int block = blockIdx.x;
+  if (block < p.q_blocks) fo_body<FO_BQ, DQK, DV, F16, SPLIT>(p, block);
+  else fo_body<FO_BK, DQK, DV, F16, SPLIT>(p, block - p.q_blocks);
+}
+
+template <bool F16, bool SPLIT>
+int fo_fill(const FhobProblem& p, FoParams& tp, bool need_v, bool need_do) {
+  memset(&tp, 0, sizeof(tp));
+  const void* mats[kFoMaps] = {p.q, p.d_o, p.k, p.v};
+  const int ids[kFoMaps] = {kTenQ, kTenDO, kTenK, kTenV};
   if (SPLIT) {
     // the bf16 hi/lo copies the caller of this function left in the workspace
     SplitBuffers sb = split_buffers(p);
-    q_side[0] = sb.q; q_side[1] = sb.d_o;
-    k_side[0] = sb.k; k_side[1] = sb.v;
+    mats[kFoQ] = sb.q; mats[kFoDO] = sb.d_o; mats[kFoK] = sb.k; mats[kFoV] = sb.v;
   }
-  // head dims below the tile widths: the boxes reach past the end of a row and are zero-filled there
-  const int d_mem[2] = {SPLIT ? 128 : p.d, SPLIT ? 128 : head_dim_v(p)};
-  // where each input lives: the caller's layout, or contiguous (always so for the split copies)
-  const int q_ids[2] = {kTenQ, kTenDO}, k_ids[2] = {kTenK, kTenV};
-  auto view = [&](int id, int n_rows, int d) {
-    return SPLIT ? contiguous_view(p.bh, n_rows, d) : tensor_view(p, id, n_rows, d);
-  };
-  int st = FHOB_OK;
-  if (MODE != FO_BK) {
-    for (int i = 0; i < C::NSTAT && st == FHOB_OK; ++i)
-      st = make_map(&tp.stat[i], q_side[i], view(q_ids[i], p.n_q, d_mem[i]), p.n_q, d_mem[i], BM, F16);
-    for (int i = 0; i < C::NSTRM && st == FHOB_OK; ++i)
-      st = make_map(&tp.strm[i], k_side[i], view(k_ids[i], p.n_k, d_mem[i]), p.n_k, d_mem[i], C::BN, F16);
-  } else {
-    for (int i = 0; i < C::NSTAT && st == FHOB_OK; ++i)
-      st = make_map(&tp.stat[i], k_side[i], view(k_ids[i], p.n_k, d_mem[i]), p.n_k, d_mem[i], BM, F16);
-    for (int i = 0; i < C::NSTRM && st == FHOB_OK; ++i)
-      st = make_map(&tp.strm[i], q_side[i], view(q_ids[i], p.n_q, d_mem[i]), p.n_q, d_mem[i], C::BN, F16);
+  for (int i = 0; i < kFoMaps; ++i) {
+    if ((i == kFoV && !need_v) || (i == kFoDO && !need_do)) continue;
+    const int n = i < kFoK ? p.n_q : p.n_k;
+    // head dims below the tile widths: the boxes reach past the end of a row and are zero-filled there
+    const int d = SPLIT ? 128 : (i == kFoDO || i == kFoV ? head_dim_v(p) : p.d);
+    // where each input lives: the caller's layout, or contiguous (always so for the split copies)
+    const int st = make_map(&tp.map[i], mats[i], SPLIT ? contiguous_view(p.bh, n, d) : tensor_view(p, ids[i], n, d), n, d, F16);
+    if (st != FHOB_OK) return st;
   }
-  if (st != FHOB_OK) return st;
   tp.heads = (!SPLIT && p.layout) ? p.layout->heads : p.bh;
-  tp.d_out0 = MODE == FO_ONE ? head_dim_v(p) : p.d;   // columns in memory of O | dQ | dK
-  tp.d_out1 = head_dim_v(p);                          // dV
+  tp.d = p.d;
+  tp.d_v = head_dim_v(p);
   tp.n_q = p.n_q; tp.n_k = p.n_k; tp.causal = p.causal; tp.window = p.window; tp.scale = p.scale;
-  const int n_stat = MODE == FO_BK ? p.n_k : p.n_q;
-  tp.tiles_per_head = (n_stat + BM - 1) / BM;
-  constexpr auto kernel = fo_kernel<MODE, DQK, DV, F16, SPLIT>;
-  {
-    const int st_attr = allow_smem(kernel, C::SMEM_BYTES);
-    if (st_attr != FHOB_OK) return st_attr;
-  }
-  const long long blocks = static_cast<long long>(tp.tiles_per_head) * p.bh;
+  tp.tiles_q = (p.n_q + BM - 1) / BM;
+  tp.tiles_k = (p.n_k + BM - 1) / BM;
+  return FHOB_OK;
+}
+
+template <class K>
+int fo_launch(K kernel, const FoParams& tp, long long blocks, int smem, cudaStream_t s) {
   if (blocks > 0x7fffffffLL) return FHOB_ERR_SHAPE;
-  kernel<<<static_cast<unsigned>(blocks), NTHREADS, C::SMEM_BYTES, s>>>(tp);
-  FHOB_CUDA_OK(cudaGetLastError());
+  const int st = allow_smem(kernel, smem);
+  if (st != FHOB_OK) return st;
+  FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(blocks), NTHREADS, smem, s, tp));
   return FHOB_OK;
 }
 
@@ -701,28 +720,32 @@ int check_device() {
 template <int DQK, int DV, bool F16, bool SPLIT = false>
 int forward_impl(const FhobProblem& p, void* o_out, float* lse_out, int* status, cudaStream_t s) {
   FoParams tp;
-  memset(&tp, 0, sizeof(tp));
+  const int st = fo_fill<F16, SPLIT>(p, tp, o_out != nullptr, false);
+  if (st != FHOB_OK) return st;
   tp.status = status;
   tp.lse_out = lse_out;
-  tp.out0 = static_cast<uint16_t*>(o_out);
+  tp.o = o_out;
+  const long long blocks = static_cast<long long>(tp.tiles_q) * p.bh;
   // no O wanted: the scores alone, reduced to the logsumexp (no tile of the second head dim is touched)
-  return o_out ? fo_launch<FO_ONE, DQK, DV, F16, SPLIT>(p, tp, s) : fo_launch<FO_LSE, DQK, DQK, F16, SPLIT>(p, tp, s);
+  if (!o_out) return fo_launch(fo_kernel<FO_LSE, DQK, DQK, F16, SPLIT>, tp, blocks, FoCfg<FO_LSE, DQK, DQK>::SMEM_BYTES, s);
+  return fo_launch(fo_kernel<FO_ONE, DQK, DV, F16, SPLIT>, tp, blocks, FoCfg<FO_ONE, DQK, DV>::SMEM_BYTES, s);
 }
 
 template <int DQK, int DV, bool F16, bool SPLIT = false>
 int backward_impl(const FhobProblem& p, void* dq, void* dk, void* dv, cudaStream_t s) {
   RowVectors rv = row_vectors(p);
   FoParams tp;
-  memset(&tp, 0, sizeof(tp));
+  const int st = fo_fill<F16, SPLIT>(p, tp, true, true);
+  if (st != FHOB_OK) return st;
   tp.status = rv.status;
   tp.nlc = rv.nlc;
   tp.k1 = rv.k1;
-  tp.out0 = static_cast<uint16_t*>(dq);
-  int st = fo_launch<FO_BQ, DQK, DV, F16, SPLIT>(p, tp, s);
-  if (st != FHOB_OK) return st;
-  tp.out0 = static_cast<uint16_t*>(dk);
-  tp.out1 = static_cast<uint16_t*>(dv);
-  return fo_launch<FO_BK, DQK, DV, F16, SPLIT>(p, tp, s);
+  tp.dq = dq; tp.dk = dk; tp.dv = dv;
+  const long long q_blocks = static_cast<long long>(tp.tiles_q) * p.bh, k_blocks = static_cast<long long>(tp.tiles_k) * p.bh;
+  if (q_blocks > 0x7fffffffLL) return FHOB_ERR_SHAPE;
+  tp.q_blocks = static_cast<int>(q_blocks);
+  constexpr int kSmemQ = FoCfg<FO_BQ, DQK, DV>::SMEM_BYTES, kSmemK = FoCfg<FO_BK, DQK, DV>::SMEM_BYTES;
+  return fo_launch(fo_backward_kernel<DQK, DV, F16, SPLIT>, tp, q_blocks + k_blocks, kSmemQ > kSmemK ? kSmemQ : kSmemK, s);
 }
 
 // One warp waits on an mbarrier nothing ever arrives on: exercises the give-up branch of wait_bar.

@@ -105,19 +105,27 @@ struct Cfg {
   static_assert(PASS <= 2 || BN == 64, "passes 3 and 4 are written for 64-row streamed tiles");
 };
 
+enum { kMapQ = 0, kMapDDQ, kMapDO, kMapK, kMapDDK, kMapV, kMapDDV, kMaps };
+
 struct TcParams {
-  CUtensorMap stat[4];
-  CUtensorMap strm[4];
-  const float* nlc;  // -L*log2(e)
-  const float* k1;   // -D
-  float* ndd;        // -dd           (written by pass 1)
-  float* k23;        // -D*dd - b     (written by pass 2)
-  uint16_t* out0;  // 16-bit elements: bf16 or f16
-  uint16_t* out1;
+  CUtensorMap map[kMaps];
+  float* nlc;         // -L*log2(e)        (written by the sweep or the pre-pass)
+  float* k1;          // -D                (the same)
+  float* ndd;         // -dd               (written by pass 1 or the sweep)
+  float* k23;         // -D*dd - b         (written by pass 2 or the sweep)
+  const void* o;      // the sweep: D = rowsum(dO * O) comes from these two, read in place
+  const void* d_o;
+  const float* lse;
+  View vo, vdo;
+  long long lse_head, lse_batch;
+  void *dq2, *ddo, *dk2, *dv2;
   int* status;
-  int n_q, n_k, causal, window, tiles_per_head;
-  int heads;            // heads per batch entry of the input tensor maps (4-D: columns, rows, head, batch)
-  int d_out0, d_out1;   // columns of the two results in memory (<= the tile widths DQK, DV; see launch)
+  int n_q, n_k, causal, window;
+  int tiles_q, tiles_k;   // 128-row tiles of a head
+  int q_blocks;           // passes 3 and 4 in one launch: the first q_blocks CTAs are pass 3
+  int heads;              // heads per batch entry of the input tensor maps (4-D: columns, rows, head, batch)
+  int d, d_v;             // columns in memory (<= the tile widths DQK, DV; see fill_params)
+  int first_live;         // first query with a visible key (causal, n_k < n_q)
   float scale;
 };
 
@@ -385,8 +393,33 @@ __device__ __forceinline__ void ew_half_b(uint32_t acc_b, uint32_t dst_ds, uint3
   }
 }
 
-template <int PASS, int DQK, int DV, int BN, int FUSED = 0, bool F16 = false, bool SPLIT = false>
-__global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_constant__ TcParams p) {
+// D = sum_d dO * O over columns [c0, c0 + N) of one row (T = storage type), 16 bytes per load.
+template <class T, int N>
+__device__ __forceinline__ float row_dot(const void* o, const void* d_o, int c0, int d) {
+  constexpr int V = 16 / sizeof(T);
+  uint4 a[N / V], b[N / V];
+#pragma unroll
+  for (int i = 0; i < N / V; ++i) {
+    a[i] = b[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (c0 + V * i < d) {   // rows are whole 16-byte pieces
+      a[i] = *reinterpret_cast<const uint4*>(static_cast<const T*>(o) + c0 + V * i);
+      b[i] = *reinterpret_cast<const uint4*>(static_cast<const T*>(d_o) + c0 + V * i);
+    }
+  }
+  float acc = 0.f;
+#pragma unroll
+  for (int i = 0; i < N / V; ++i) {
+    const T* ea = reinterpret_cast<const T*>(&a[i]);
+    const T* eb = reinterpret_cast<const T*>(&b[i]);
+#pragma unroll
+    for (int e = 0; e < V; ++e) acc = fmaf(static_cast<float>(ea[e]), static_cast<float>(eb[e]), acc);
+  }
+  return acc;
+}
+
+// One pass over one 128-row tile of one head; `block` numbers the (head, tile) pairs of the pass.
+template <int PASS, int DQK, int DV, int BN, int FUSED, bool F16, bool SPLIT>
+__device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
   static_assert(FUSED == 0 || PASS == 2, "only pass 2 has a fused form");
   static_assert(!SPLIT || (DQK == 128 && DV == 128 && !F16), "split fp32 operands are [hi(64) | lo(64)] bf16 rows");
   using C = Cfg<PASS, DQK, DV, BN>;
@@ -399,10 +432,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
   Bars* bars = reinterpret_cast<Bars*>(strm_tiles + C::NSLOT * C::SLOT_BYTES);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int head = blockIdx.x / p.tiles_per_head;
-  const int tile_in_head = blockIdx.x - head * p.tiles_per_head;
+  const int tiles_per_head = kQStat ? p.tiles_q : p.tiles_k;
+  const int head = block / tiles_per_head;
+  const int tile_in_head = block - head * tiles_per_head;
   // causal: longest tiles first (late queries in passes 1-3, early keys in pass 4)
-  const int tile = kQStat ? p.tiles_per_head - 1 - tile_in_head : tile_in_head;
+  const int tile = kQStat ? tiles_per_head - 1 - tile_in_head : tile_in_head;
   const int m0 = tile * BM;
   const int n_stat = kQStat ? p.n_q : p.n_k;
   const int n_strm = kQStat ? p.n_k : p.n_q;
@@ -412,9 +446,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
   visible_tiles(kQStat, m0, BM, BN, n_strm, off, p.causal, p.window, t_begin, t_end);
   const int n_iter = t_end - t_begin;
 
+  auto stat_map = [&](int i) { return &p.map[kQStat ? kMapQ + i : kMapK + i]; };   // Q, ddQ, dO | K, ddK, V, ddV
+  auto strm_map = [&](int i) { return &p.map[kQStat ? kMapK + i : kMapQ + i]; };
+
   // ---- set-up
+  int fault = 0;   // thread 0: what to report at the end
   if (threadIdx.x == 0) {
-    if (smem_u32(smem) & 1023u) atomicOr(p.status, FHOB_ERR_SMEM_ALIGN);
+    if (smem_u32(smem) & 1023u) fault |= FHOB_ERR_SMEM_ALIGN;
     mbar_init(&bars->stat_full, 1);
     for (int i = 0; i < 4; ++i) {
       mbar_init(&bars->strm_full[i], 1);
@@ -439,8 +477,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
     tmem_relinquish();
   }
   if (warp == TMA_WARP && lane == 0) {
-    for (int i = 0; i < C::NSTAT; ++i) prefetch_tensormap(&p.stat[i]);
-    for (int i = 0; i < C::NSTRM; ++i) prefetch_tensormap(&p.strm[i]);
+    for (int i = 0; i < C::NSTAT; ++i) prefetch_tensormap(stat_map(i));
+    for (int i = 0; i < C::NSTRM; ++i) prefetch_tensormap(strm_map(i));
   }
   tc_fence_before();
   __syncthreads();
@@ -450,18 +488,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
   // the allocator is reported through the status word.
   constexpr uint32_t tmem_base = 0;
   if (threadIdx.x == 0 && *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base) != 0)
-    atomicOr(p.status, FHOB_ERR_TMEM_BASE);
+    fault |= FHOB_ERR_TMEM_BASE;
+  // Everything up to here overlaps the end of the kernel in front; from here on memory is touched.
+  pdl_wait();
+  if (threadIdx.x == 0) {
+    pdl_launch_dependents();
+    if (FUSED && block == 0) *p.status = 0;   // every operator call starts clean
+  }
 
   if (warp == TMA_WARP) {
     // ================================================= TMA producer
     if (n_iter > 0 && elect_one()) {
       const int head_b = head / p.heads, head_h = head - head_b * p.heads;   // batch entry and head within it
+      if (PASS == 4) fence_proxy_async_global();   // the row vectors the bulk copies read were written by a kernel in front
       mbar_arrive_expect_tx(&bars->stat_full, C::STAT_BYTES);
 #pragma unroll
-      for (int i = 0; i < C::NSTAT; ++i)
-        for (int bx = 0; bx < C::tile_d(i) / 64; ++bx)
-          tma_load_4d(stat_tiles + C::stat_off(i) + bx * (BM * 128), &p.stat[i], &bars->stat_full, bx * 64, m0,
-                      head_h, head_b);
+      for (int i = 0; i < C::NSTAT; ++i) {
+        if (i < 2) load_tile<BM, DQK, BM * 128>(stat_tiles + C::stat_off(i), stat_map(i), &bars->stat_full, m0, head_h, head_b);
+        else load_tile<BM, DV, BM * 128>(stat_tiles + C::stat_off(i), stat_map(i), &bars->stat_full, m0, head_h, head_b);
+      }
       int issued = 0;
       for (int it = 0; it < n_iter; ++it) {
         const int slot = it % C::NSLOT;
@@ -470,10 +515,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
         uint8_t* dst = strm_tiles + slot * C::SLOT_BYTES;
         const int n0 = (t_begin + it) * BN;
 #pragma unroll
-        for (int i = 0; i < C::NSTRM; ++i)
-          for (int bx = 0; bx < C::tile_d(i) / 64; ++bx)
-            tma_load_4d(dst + C::strm_base(i) + bx * C::strm_box(i), &p.strm[i], &bars->strm_full[slot], bx * 64,
-                        n0, head_h, head_b);
+        for (int i = 0; i < C::NSTRM; ++i) {
+          uint8_t* at = dst + C::strm_base(i);
+          if (i < 2) load_tile<BN, DQK, C::strm_box(0)>(at, strm_map(i), &bars->strm_full[slot], n0, head_h, head_b);
+          else load_tile<BN, DV, C::strm_box(2)>(at, strm_map(i), &bars->strm_full[slot], n0, head_h, head_b);
+        }
         if (PASS == 4) {
           const size_t vo = static_cast<size_t>(head) * row_stride(p.n_q) + n0;
           uint8_t* sv = dst + C::STRM_BYTES;
@@ -672,11 +718,27 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
     c.scale = p.scale;
     c.sl2 = p.scale * kLog2e;
     c.r_nlc = c.r_k1 = c.r_ndd = c.r_k23 = 0.f;
-    if (kQStat && g_row < p.n_q) {
+    float d_part = 0.f;   // the sweep: this thread's half of D = rowsum(dO * O)
+    if (FUSED) {
+      // A query the causal mask leaves without any visible key contributes nothing (every P of its
+      // row is masked to zero): its saved L (-inf) and O (0 or NaN) are not looked at.
+      if (g_row < p.n_q && g_row >= p.first_live) {
+        const int hb = head / p.vo.heads, hh = head - hb * p.vo.heads;
+        c.r_nlc = -p.lse[hb * p.lse_batch + hh * p.lse_head + g_row] * kLog2e;
+        if (FUSED == 1) {
+          using T = typename std::conditional<SPLIT, float, typename std::conditional<F16, __half, __nv_bfloat16>::type>::type;
+          constexpr int W = SPLIT ? 32 : DV / 2;
+          d_part = row_dot<T, W>(static_cast<const T*>(p.o) + hb * p.vo.batch + hh * p.vo.head + g_row * p.vo.row,
+                                 static_cast<const T*>(p.d_o) + hb * p.vdo.batch + hh * p.vdo.head + g_row * p.vdo.row,
+                                 half * W, p.d_v);
+        }
+      }
+      if (half == 0 && g_row < p.n_q) p.nlc[vec_head + g_row] = c.r_nlc;
+    } else if (kQStat && g_row < p.n_q) {
       c.r_nlc = p.nlc[vec_head + g_row];
       if (PASS >= 2) {
-        if (FUSED != 2) c.r_k1 = p.k1[vec_head + g_row];
-        if (FUSED == 0) c.r_ndd = p.ndd[vec_head + g_row];
+        c.r_k1 = p.k1[vec_head + g_row];
+        c.r_ndd = p.ndd[vec_head + g_row];
       }
       if (PASS >= 3) c.r_k23 = p.k23[vec_head + g_row];
     }
@@ -769,20 +831,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
       if (half == 1) bars->red[row] = rb;
       asm volatile("bar.sync 1, 256;" ::: "memory");
       if (half == 0) rb += bars->red[row];
-      float d_row = -c.r_k1;
-      if (FUSED == 2) {
-        // D = sum P dP (the caller passed no O): it is also what passes 3 and 4 read as k1 = -D
-        d_row = racc[3].x + racc[3].y;
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (half == 1) bars->red[row] = d_row;
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (half == 0) d_row += bars->red[row];
-      }
+      // D = rowsum(dO * O), or sum P dP when the caller passed no O
+      float d_row = FUSED == 2 ? racc[3].x + racc[3].y : d_part;
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (half == 1) bars->red[row] = d_row;
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (half == 0) d_row += bars->red[row];
       if (half == 0 && ok && g_row < p.n_q) {
         const float dd = c.scale * r1;
         p.ndd[vec_head + g_row] = -dd;
         p.k23[vec_head + g_row] = d_row * dd - rb;  // -D*dd - b = D*dd - (sum P X + scale * sum dP P A2)
-        if (FUSED == 2) const_cast<float*>(p.k1)[vec_head + g_row] = -d_row;
+        p.k1[vec_head + g_row] = -d_row;
       }
     } else if (PASS <= 2) {
       if (half == 1) bars->red[row] = rowacc.x + rowacc.y;
@@ -796,9 +855,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
       if (n_iter > 0) ok = ok && __all_sync(0xffffffffu, wait_bar(&bars->out_full, 0, bars, p.status));
       tc_fence_after();
       if (ok) {
-        auto store_out = [&](auto width, int d_mem, uint32_t col0, uint16_t* base, float mul) {
+        auto store_out = [&](auto width, int d_mem, uint32_t col0, void* base, float mul) {
           constexpr int DO = decltype(width)::value;   // columns of the accumulator; d_mem <= DO of them exist in memory
-          uint16_t* dst = base + (static_cast<size_t>(head) * n_stat + (g_row < n_stat ? g_row : 0)) * d_mem + half * (DO / 2);
+          uint16_t* dst = static_cast<uint16_t*>(base) + (static_cast<size_t>(head) * n_stat + (g_row < n_stat ? g_row : 0)) * d_mem + half * (DO / 2);
 #pragma unroll
           for (int ch = 0; ch < DO / 32; ++ch) {
             uint32_t v[16];
@@ -822,8 +881,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
           }
         };
         // split operands: a result has 64 fp32 columns, the sum of the two 64-column halves of its accumulator
-        auto store_out_split = [&](int d_mem, uint32_t col0, uint16_t* base16, float mul) {
-          float* dst = reinterpret_cast<float*>(base16) +
+        auto store_out_split = [&](int d_mem, uint32_t col0, void* base, float mul) {
+          float* dst = static_cast<float*>(base) +
                        (static_cast<size_t>(head) * n_stat + (g_row < n_stat ? g_row : 0)) * d_mem + half * 32;
 #pragma unroll
           for (int ch = 0; ch < 2; ++ch) {
@@ -849,12 +908,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
           }
         };
         // dS and dS2 were stored without the factor `scale`: it is applied to dQ2 | dK2 here
+        void *out0 = kQStat ? p.dq2 : p.dk2, *out1 = kQStat ? p.ddo : p.dv2;
         if constexpr (SPLIT) {
-          store_out_split(p.d_out0, 0, p.out0, c.scale);
-          store_out_split(p.d_out1, C::OUT0_COLS, p.out1, 1.f);
+          store_out_split(p.d, 0, out0, c.scale);
+          store_out_split(p.d_v, C::OUT0_COLS, out1, 1.f);
         } else {
-          store_out(std::integral_constant<int, DQK>{}, p.d_out0, 0, p.out0, c.scale);
-          store_out(std::integral_constant<int, DV>{}, p.d_out1, C::OUT0_COLS, p.out1, 1.f);
+          store_out(std::integral_constant<int, DQK>{}, p.d, 0, out0, c.scale);
+          store_out(std::integral_constant<int, DV>{}, p.d_v, C::OUT0_COLS, out1, 1.f);
         }
       }
     }
@@ -868,6 +928,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_const
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
+  if (threadIdx.x == 0 && fault) atomicOr(p.status, fault);
+}
+
+template <int PASS, int DQK, int DV, int BN, int FUSED, bool F16, bool SPLIT>
+__global__ void __launch_bounds__(NTHREADS, 1) tc_pass_kernel(const __grid_constant__ TcParams p) {
+  tc_pass_body<PASS, DQK, DV, BN, FUSED, F16, SPLIT>(p, blockIdx.x);
+}
+
+// Passes 3 and 4 in one launch: they only need the sweep, not each other, so pass 4's CTAs fill the
+// SMs that run out of pass-3 work (and a small problem runs both side by side).
+template <int DQK, int DV, bool F16, bool SPLIT>
+__global__ void __launch_bounds__(NTHREADS, 1) tc_pass34_kernel(const __grid_constant__ TcParams p) {
+  const int block = blockIdx.x;
+  if (block < p.q_blocks) tc_pass_body<3, DQK, DV, 64, 0, F16, SPLIT>(p, block);
+  else tc_pass_body<4, DQK, DV, 64, 0, F16, SPLIT>(p, block - p.q_blocks);
 }
 
 // ------------------------------------------------------------------ host side
@@ -883,6 +958,8 @@ struct SplitJobs {
   View view[7];
 };
 __global__ void split_rows_kernel(const __grid_constant__ SplitJobs jobs) {
+  pdl_wait();
+  if (threadIdx.x == 0) pdl_launch_dependents();
   const int t = blockIdx.y;
   const long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= jobs.pairs[t]) return;
@@ -900,75 +977,97 @@ __global__ void split_rows_kernel(const __grid_constant__ SplitJobs jobs) {
   dst[row * 64 + 32 + c2] = lo;
 }
 
-template <int PASS, int DQK, int DV, int BN, int FUSED = 0, bool F16 = false, bool SPLIT = false>
-int launch(const FhobProblem& p, cudaStream_t s) {
-  using C = Cfg<PASS, DQK, DV, BN>;
-  constexpr auto kernel = tc_pass_kernel<PASS, DQK, DV, BN, FUSED, F16, SPLIT>;
+int first_live_query(const FhobProblem& p) {
+  // bottom-right aligned causal mask: query i sees key 0 only if i + n_k - n_q >= 0
+  return (p.causal && p.n_q > p.n_k) ? p.n_q - p.n_k : 0;
+}
+
+template <bool F16, bool SPLIT>
+int fill_params(const FhobProblem& p, TcParams& tp) {
   RowVectors rv = row_vectors(p);
-  TcParams tp;
-  memset(&tp, 0, sizeof(tp));
-  const void* q_side[3] = {p.q, p.ddq, p.d_o};
-  const void* k_side[4] = {p.k, p.ddk, p.v, p.ddv};
+  const void* mats[kMaps] = {p.q, p.ddq, p.d_o, p.k, p.ddk, p.v, p.ddv};
+  const int ids[kMaps] = {kTenQ, kTenDDQ, kTenDO, kTenK, kTenDDK, kTenV, kTenDDV};
   if (SPLIT) {
     // the kernels read the bf16 hi/lo copies the preparation step left behind the row vectors
     SplitBuffers sb = split_buffers(p);
-    q_side[0] = sb.q; q_side[1] = sb.ddq; q_side[2] = sb.d_o;
-    k_side[0] = sb.k; k_side[1] = sb.ddk; k_side[2] = sb.v; k_side[3] = sb.ddv;
+    mats[0] = sb.q; mats[1] = sb.ddq; mats[2] = sb.d_o;
+    mats[3] = sb.k; mats[4] = sb.ddk; mats[5] = sb.v; mats[6] = sb.ddv;
   }
-  // A head dim below the tile width (any multiple of 8 up to 128) needs nothing but the right
-  // tensor map: the 64-column boxes reach past the end of a row, the TMA unit fills those columns
-  // with zeros, zeros add nothing to a contraction, and the epilogue stores only the columns that exist.
-  const int d_mem[2] = {SPLIT ? 128 : p.d, SPLIT ? 128 : head_dim_v(p)};   // columns in memory of the two tile kinds
-  // where each input lives: the caller's layout, or contiguous (always so for the split copies)
-  const int q_ids[3] = {kTenQ, kTenDDQ, kTenDO}, k_ids[4] = {kTenK, kTenDDK, kTenV, kTenDDV};
-  auto view = [&](int id, int n_rows, int d) {
-    return SPLIT ? contiguous_view(p.bh, n_rows, d) : tensor_view(p, id, n_rows, d);
-  };
-  int st = FHOB_OK;
-  if (PASS != 4) {
-    for (int i = 0; i < C::NSTAT && st == FHOB_OK; ++i)
-      st = make_map(&tp.stat[i], q_side[i], view(q_ids[i], p.n_q, d_mem[i < 2 ? 0 : 1]), p.n_q, d_mem[i < 2 ? 0 : 1], BM, F16);
-    for (int i = 0; i < C::NSTRM && st == FHOB_OK; ++i)
-      st = make_map(&tp.strm[i], k_side[i], view(k_ids[i], p.n_k, d_mem[i < 2 ? 0 : 1]), p.n_k, d_mem[i < 2 ? 0 : 1], BN, F16);
-  } else {
-    for (int i = 0; i < C::NSTAT && st == FHOB_OK; ++i)
-      st = make_map(&tp.stat[i], k_side[i], view(k_ids[i], p.n_k, d_mem[i < 2 ? 0 : 1]), p.n_k, d_mem[i < 2 ? 0 : 1], BM, F16);
-    for (int i = 0; i < C::NSTRM && st == FHOB_OK; ++i)
-      st = make_map(&tp.strm[i], q_side[i], view(q_ids[i], p.n_q, d_mem[i < 2 ? 0 : 1]), p.n_q, d_mem[i < 2 ? 0 : 1], BN, F16);
+  const int dv = head_dim_v(p);
+  for (int i = 0; i < kMaps; ++i) {
+    const int n = i < kMapK ? p.n_q : p.n_k;
+    // A head dim below the tile width (any multiple of 8 up to 128) needs nothing but the right
+    // tensor map: the 64-column boxes reach past the end of a row, the TMA unit fills those columns
+    // with zeros, zeros add nothing to a contraction, and the epilogue stores only the columns that exist.
+    const int d = SPLIT ? 128 : (i == kMapDO || i >= kMapV ? dv : p.d);
+    // where each input lives: the caller's layout, or contiguous (always so for the split copies)
+    const int st = make_map(&tp.map[i], mats[i], SPLIT ? contiguous_view(p.bh, n, d) : tensor_view(p, ids[i], n, d), n, d, F16);
+    if (st != FHOB_OK) return st;
   }
-  if (st != FHOB_OK) return st;
-  tp.heads = (!SPLIT && p.layout) ? p.layout->heads : p.bh;
-  tp.d_out0 = p.d;               // columns of the results in memory (split operands: up to 64 fp32 columns)
-  tp.d_out1 = head_dim_v(p);
   tp.nlc = rv.nlc; tp.k1 = rv.k1; tp.ndd = rv.ndd; tp.k23 = rv.k23;
-  tp.out0 = static_cast<uint16_t*>(PASS == 3 ? p.dq2 : p.dk2);
-  tp.out1 = static_cast<uint16_t*>(PASS == 3 ? p.ddo : p.dv2);
+  tp.o = p.o; tp.d_o = p.d_o; tp.lse = p.lse;
+  tp.vo = tensor_view(p, kTenO, p.n_q, dv);
+  tp.vdo = tensor_view(p, kTenDO, p.n_q, dv);
+  tp.lse_head = p.layout ? p.layout->lse_head : p.n_q;
+  tp.lse_batch = p.layout ? p.layout->lse_batch : static_cast<long long>(p.bh) * p.n_q;
+  tp.dq2 = p.dq2; tp.ddo = p.ddo; tp.dk2 = p.dk2; tp.dv2 = p.dv2;
   tp.status = rv.status;
   tp.n_q = p.n_q; tp.n_k = p.n_k; tp.causal = p.causal; tp.window = p.window; tp.scale = p.scale;
-  const int n_stat = PASS == 4 ? p.n_k : p.n_q;
-  tp.tiles_per_head = (n_stat + BM - 1) / BM;
-  {
-    const int st_attr = allow_smem(kernel, C::SMEM_BYTES);
-    if (st_attr != FHOB_OK) return st_attr;
-  }
-  const long long blocks = static_cast<long long>(tp.tiles_per_head) * p.bh;
-  if (blocks > 0x7fffffffLL) return FHOB_ERR_SHAPE;
-  kernel<<<static_cast<unsigned>(blocks), NTHREADS, C::SMEM_BYTES, s>>>(tp);
-  FHOB_CUDA_OK(cudaGetLastError());
+  tp.tiles_q = (p.n_q + BM - 1) / BM;
+  tp.tiles_k = (p.n_k + BM - 1) / BM;
+  tp.q_blocks = 0;
+  tp.heads = (!SPLIT && p.layout) ? p.layout->heads : p.bh;
+  tp.d = p.d;
+  tp.d_v = dv;
+  tp.first_live = first_live_query(p);
   return FHOB_OK;
 }
 
+template <class K>
+int launch(K kernel, const TcParams& tp, long long blocks, int smem, cudaStream_t s) {
+  if (blocks > 0x7fffffffLL) return FHOB_ERR_SHAPE;
+  const int st = allow_smem(kernel, smem);
+  if (st != FHOB_OK) return st;
+  FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(blocks), NTHREADS, smem, s, tp));
+  return FHOB_OK;
+}
+
+template <int PASS, int DQK, int DV, int BN, int FUSED, bool F16, bool SPLIT>
+int launch_pass(const FhobProblem& p, const TcParams& tp, cudaStream_t s) {
+  return launch(tc_pass_kernel<PASS, DQK, DV, BN, FUSED, F16, SPLIT>, tp, static_cast<long long>(tp.tiles_q) * p.bh,
+                Cfg<PASS, DQK, DV, BN>::SMEM_BYTES, s);
+}
+
+template <int DQK, int DV, bool F16, bool SPLIT>
+int launch_34(const FhobProblem& p, TcParams& tp, bool pass3, bool pass4, cudaStream_t s) {
+  constexpr int kSmem3 = Cfg<3, DQK, DV, 64>::SMEM_BYTES, kSmem4 = Cfg<4, DQK, DV, 64>::SMEM_BYTES;
+  const long long q_blocks = pass3 ? static_cast<long long>(tp.tiles_q) * p.bh : 0;
+  const long long k_blocks = pass4 ? static_cast<long long>(tp.tiles_k) * p.bh : 0;
+  if (q_blocks > 0x7fffffffLL) return FHOB_ERR_SHAPE;
+  tp.q_blocks = static_cast<int>(q_blocks);
+  return launch(tc_pass34_kernel<DQK, DV, F16, SPLIT>, tp, q_blocks + k_blocks, kSmem3 > kSmem4 ? kSmem3 : kSmem4, s);
+}
+
+// `pass`: 1, 2, 3, 4 alone, 12 = passes 1 and 2 in one sweep, kWholeOperator = the sweep, then passes 3 and 4
+constexpr int kWholeOperator = 1234;
 template <int DQK, int DV, bool F16, bool SPLIT = false>
 int dispatch(int pass, const FhobProblem& p, cudaStream_t s) {
+  TcParams tp;
+  int st = fill_params<F16, SPLIT>(p, tp);
+  if (st != FHOB_OK) return st;
   switch (pass) {
     // pass 1 streams 128-row tiles (the stacked [K ; ddK] operand reaches N = 256), the others 64;
     // it touches no tile of the second head dim
-    case 1: return launch<1, DQK, DQK, 128, 0, F16, SPLIT>(p, s);
-    case 2: return launch<2, DQK, DV, 64, 0, F16, SPLIT>(p, s);
-    case 12: return launch<2, DQK, DV, 64, 1, F16, SPLIT>(p, s);  // passes 1 and 2 in one sweep
-    case 13: return launch<2, DQK, DV, 64, 2, F16, SPLIT>(p, s);  // the same, also producing D = sum P dP (no O given)
-    case 3: return launch<3, DQK, DV, 64, 0, F16, SPLIT>(p, s);
-    case 4: return launch<4, DQK, DV, 64, 0, F16, SPLIT>(p, s);
+    case 1: return launch_pass<1, DQK, DQK, 128, 0, F16, SPLIT>(p, tp, s);
+    case 2: return launch_pass<2, DQK, DV, 64, 0, F16, SPLIT>(p, tp, s);
+    case 3: return launch_34<DQK, DV, F16, SPLIT>(p, tp, true, false, s);
+    case 4: return launch_34<DQK, DV, F16, SPLIT>(p, tp, false, true, s);
+    case 12:
+    case kWholeOperator:
+      // without O the sweep also produces D = sum P dP
+      st = p.o ? launch_pass<2, DQK, DV, 64, 1, F16, SPLIT>(p, tp, s) : launch_pass<2, DQK, DV, 64, 2, F16, SPLIT>(p, tp, s);
+      if (st != FHOB_OK || pass == 12) return st;
+      return launch_34<DQK, DV, F16, SPLIT>(p, tp, true, true, s);
   }
   return FHOB_ERR_ARG;
 }
@@ -1042,8 +1141,7 @@ int tc_split_inputs(const FhobProblem& p, cudaStream_t s, int which) {
   }
   const long blocks = (most + 255) / 256;
   if (blocks > 0x7fffffffL) return FHOB_ERR_SHAPE;
-  split_rows_kernel<<<dim3(static_cast<unsigned>(blocks), count), 256, 0, s>>>(jobs);
-  FHOB_CUDA_OK(cudaGetLastError());
+  FHOB_CUDA_OK(launch_pdl(split_rows_kernel, dim3(static_cast<unsigned>(blocks), count), 256, 0, s, jobs));
   return FHOB_OK;
 }
 
@@ -1053,6 +1151,14 @@ int tc_pass(int pass, const FhobProblem& p, cudaStream_t s) {
   if (st != FHOB_OK) return st;
   if (p.dtype == FHOB_F32) return dispatch<128, 128, false, true>(pass, p, s);
   return p.dtype == FHOB_F16 ? dispatch_dims<true>(pass, p, s) : dispatch_dims<false>(pass, p, s);
+}
+
+int tc_operator(const FhobProblem& p, cudaStream_t s) {
+  if (p.dtype == FHOB_F32) {
+    const int st = tc_split_inputs(p, s);
+    if (st != FHOB_OK) return st;
+  }
+  return tc_pass(kWholeOperator, p, s);
 }
 
 }  // namespace fhob
