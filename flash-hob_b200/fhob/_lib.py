@@ -87,6 +87,16 @@ def load() -> C.CDLL:
     return lib
 
 
+def native():
+    """The native host path (csrc/host_binding.cpp).  Missing is an error, as for the library itself."""
+    load()
+    try:
+        from . import _native
+    except ImportError as e:
+        raise RuntimeError(f"fhob._native cannot be imported ({e}): build it with `python flash-hob_b200/build.py`") from e
+    return _native
+
+
 def check(status: int, what: str) -> None:
     if status == 0:
         return

@@ -31,6 +31,29 @@ def _workspace(device: torch.device, stream: int, nbytes: int) -> torch.Tensor:
     return ws
 
 
+_native_module = None
+
+
+def _native():
+    """The native host path.  Its functions take well-formed calls on CUDA tensors and return None for
+    any other; the Python code below then makes the copies that such a call needs or raises its error."""
+    global _native_module
+    if _native_module is None:
+        module = _lib.native()
+        module.use_workspaces(_workspaces)
+        _native_module = module
+    return _native_module
+
+
+def _check_status(device: torch.device, what: str) -> None:
+    """Synchronises the current stream and raises if the last native call on it set its status word."""
+    stream = torch.cuda.current_stream(device).cuda_stream
+    p = _lib.FhobProblem()
+    p.workspace = _workspaces[(device.index, stream)].data_ptr()
+    with torch.cuda.device(device):
+        _lib.check(_lib.load().fhob_read_status(C.byref(p), C.c_void_p(stream)), f"{what} (device status)")
+
+
 def _fold(t: torch.Tensor, name: str) -> torch.Tensor:
     if t.dim() == 4:
         t = t.reshape(t.shape[0] * t.shape[1], t.shape[2], t.shape[3])
@@ -280,6 +303,12 @@ def flash_bwdbwd(Q, K, V, O, dO, ddQ, ddK, ddV, L, scale, *, is_causal: bool = F
     memory, and the four results come back as pinned host tensors (or in
     ``out``, four host tensors, preferably pinned) after a stream synchronise.
     """
+    if Q.is_cuda and out is None and workspace is None:
+        got = _native().bwdbwd(Q, K, V, O, dO, ddQ, ddK, ddV, L, scale, is_causal, sliding_window, impl)
+        if got is not None:
+            if check:
+                _check_status(Q.device, "fhob_bwdbwd")
+            return got
     if Q.numel() == 0 or K.numel() == 0 or V.numel() == 0:
         return _empty_problem(Q, K, V, dO, out)
     if Q.device.type == "cuda":
@@ -434,6 +463,12 @@ def attention_forward(Q, K, V, scale=None, *, is_causal: bool = False, sliding_w
     ``check`` synchronises and raises if a bounded device wait ran out.
     Queries that see no key (causal with N_K < N_Q) get ``O = 0``, ``L = -inf``.
     """
+    if Q.is_cuda:
+        got = _native().forward(Q, K, V, scale, is_causal, sliding_window, impl, need_o)
+        if got is not None:
+            if check:
+                _check_status(Q.device, "fhob_forward")
+            return got
     shape_q = Q.shape
     if Q.device.type != "cuda" or str(Q.dtype) not in _lib.DTYPES:
         raise ValueError("attention_forward needs CUDA bfloat16/float16/float32 tensors")
