@@ -108,21 +108,90 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, 
       tma_load_4d(dst + bx * BOX + by * (BOX_ROWS * 128), map, bar, bx * 64, y + by * BOX_ROWS, head, batch);
 }
 
+// ---- split streamed axis: a cluster of `split` CTAs shares the streamed tiles of one stationary tile
+// and adds up its results through distributed shared memory, in rank order (so bits do not vary).
+
+// Streamed tiles of part `part` of `split` of the range [begin, end).
+__device__ __forceinline__ void split_range(int part, int split, int& begin, int& end) {
+  const int n = end - begin, b = begin;
+  begin = b + static_cast<int>(static_cast<long long>(n) * part / split);
+  end = b + static_cast<int>(static_cast<long long>(n) * (part + 1) / split);
+}
+
+// This thread's W fp32 accumulator columns (TMEM addresses taddr..) of its row -> staging area.
+template <int W>
+__device__ __forceinline__ void stage_row(float* dst, uint32_t taddr, bool any) {
+#pragma unroll
+  for (int c = 0; c < W; c += 16) {
+    uint32_t v[16];
+    if (any) {
+      tmem_ld16(taddr + c, v);
+      tmem_wait_ld();
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < 16; j += 4)
+      *reinterpret_cast<uint4*>(dst + c + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+  }
+}
+
+// Adds the staged columns [c0, c0 + W) of all parts for this CTA's share of the rows, times `mul`, and stores
+// them to `base` (n_rows x d_mem per head).  `stage` = shared address of the staging area (row pitch
+// `pitch` floats), `rank0` = cluster rank of part 0, `tid` of 256 threads.
+template <int W, bool F32, bool F16>
+__device__ __forceinline__ void reduce_store(uint32_t stage, int pitch, int c0, int rank0, int part, int split, int tid, void* base,
+                                             int head, int m0, int n_rows, int d_mem, float mul) {
+  constexpr int V = F32 ? 4 : 8;
+  const int rows = (BM + split - 1) / split;
+  for (int i = tid; i < rows * (W / V); i += EW_THREADS) {
+    const int r = part * rows + i / (W / V), c = (i % (W / V)) * V;
+    if (r >= BM || m0 + r >= n_rows || c >= d_mem) continue;   // rows are whole 16-byte pieces
+    float4 a[V / 4];
+#pragma unroll
+    for (int h = 0; h < V / 4; ++h) a[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t at = stage + (r * pitch + c0 + c) * 4;
+    for (int s = 0; s < split; ++s) {
+      const uint32_t from = cluster_map(at, rank0 + s);
+#pragma unroll
+      for (int h = 0; h < V / 4; ++h) {
+        const float4 x = cluster_ld4(from + 16 * h);
+        a[h].x += x.x; a[h].y += x.y; a[h].z += x.z; a[h].w += x.w;
+      }
+    }
+    const size_t off = (static_cast<size_t>(head) * n_rows + m0 + r) * d_mem + c;
+    if constexpr (F32) {
+      *reinterpret_cast<float4*>(static_cast<float*>(base) + off) = make_float4(a[0].x * mul, a[0].y * mul, a[0].z * mul, a[0].w * mul);
+    } else {
+      *reinterpret_cast<uint4*>(static_cast<uint16_t*>(base) + off) =
+          make_uint4(pack16<F16>(a[0].x * mul, a[0].y * mul), pack16<F16>(a[0].z * mul, a[0].w * mul),
+                     pack16<F16>(a[V / 4 - 1].x * mul, a[V / 4 - 1].y * mul), pack16<F16>(a[V / 4 - 1].z * mul, a[V / 4 - 1].w * mul));
+    }
+  }
+}
+
 // ------------------------------------------------------------------ host side
 // Launches with programmatic stream serialization: the kernel's CTAs may start while the kernel in
 // front of it drains (it says pdl_launch_dependents), and wait in pdl_wait before they touch memory.
 template <class... P, class... A>
-cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, int cluster, cudaStream_t s, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (cluster > 1) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
@@ -228,6 +297,94 @@ int allow_smem(K kernel, int bytes) {
   }
   if (e) e->devices |= bit;
   return FHOB_OK;
+}
+
+// How many CTAs share the streamed tiles of an item (a head's 128-row tile), for one or two kinds of
+// item that need not wait for each other.
+struct SplitWork {
+  int items, tiles;   // items of this kind, streamed tiles of the longest one
+};
+struct SplitChoice {
+  int a, b;
+  bool together;   // one launch for both kinds (clusters are of one size in a launch)
+};
+constexpr int kMaxSplit = 8;   // the portable cluster size
+
+// CTAs the device runs at once in clusters of `c` of a kernel that has an SM to itself: clusters do not
+// straddle GPCs, so some SMs stay idle (a B200 with 148 SMs: 132 in clusters of 4 or 6, 120 in clusters
+// of 8).  Asked once per device and host thread.
+template <class K>
+int cluster_slots(K kernel, int smem, int c) {
+  constexpr int kDevices = 64;
+  static thread_local int table[kDevices][kMaxSplit + 1] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices || c < 1 || c > kMaxSplit) return 0;
+  int& slots = table[dev][c];
+  if (slots == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = c;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(c * 64);
+    cfg.blockDim = dim3(NTHREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    slots = n > 0 ? n * c : -1;   // -1: not available
+  }
+  return slots > 0 ? slots : 0;
+}
+
+// A head whose sequences both have 4096 rows or more is never split: jobs of that size are cut over
+// GPUs by heads, and a head's bits must not depend on which heads it is launched with (the number of
+// parts is a number of partial sums).
+bool may_split(int n_q, int n_k) { return n_q < 4096 || n_k < 4096; }
+
+// Splitting pays while the items leave SMs idle.  Times are in streamed tiles: a CTA takes about kFixed
+// tiles' time besides its own (launch, prologue, first loads, epilogue: 6 to 9 us against 1 to 1.7 us a
+// tile), kCluster more in a cluster (its CTAs start together and meet twice), and a second launch costs
+// kLaunch.  Measured with 16 heads, 100 queries, 6000 keys (16 items of 94 tiles, 752 of 2): sweep
+// 102 -> 29 us; passes 3 and 4 205 us in one unsplit launch.
+template <class K>
+SplitChoice choose_split(K kernel, int smem, const SplitWork& wa, const SplitWork& wb) {
+  constexpr float kFixed = 5.f, kCluster = 1.f, kLaunch = 1.f;
+  SplitChoice best = {1, 1, true};
+  const int sms = cluster_slots(kernel, smem, 1);
+  auto fills = [&](const SplitWork& w) { return w.items == 0 || w.items >= sms; };
+  if (fills(wa) && fills(wb)) return best;
+  auto item_time = [&](const SplitWork& w, int split, int cluster) {
+    return w.items == 0 ? 0.f : (w.tiles + split - 1) / split + kFixed + (cluster > 1 ? kCluster : 0.f);
+  };
+  auto wave_time = [&](int sa, int sb, int cluster, const SplitWork& a, const SplitWork& b) {
+    const float slots = static_cast<float>(cluster_slots(kernel, smem, cluster));
+    if (slots == 0.f) return 1e30f;
+    const float ta = item_time(a, sa, cluster), tb = item_time(b, sb, cluster), longest = ta > tb ? ta : tb;
+    const float ctas = static_cast<float>(a.items) * sa + static_cast<float>(b.items) * sb;
+    // one wave takes as long as its longest CTA; more CTAs fill the slots as they come free
+    return ctas <= slots ? longest : (a.items * sa * ta + b.items * sb * tb) / slots + 0.5f * longest;
+  };
+  const SplitWork none = {0, 0};
+  float best_time = wave_time(1, 1, 1, wa, wb);
+  for (int sa = 1; sa <= kMaxSplit && (sa == 1 || sa <= wa.tiles); ++sa)
+    for (int sb = 1; sb <= kMaxSplit && (sb == 1 || sb <= wb.tiles); ++sb) {
+      if ((sa > 1 && wa.items == 0) || (sb > 1 && wb.items == 0)) continue;
+      const int most = sa > sb ? sa : sb, least = sa > sb ? sb : sa;
+      if (most % least == 0) {
+        const float t = wave_time(sa, sb, most, wa, wb);
+        if (t < best_time) { best_time = t; best = {sa, sb, true}; }
+      }
+      if (wa.items && wb.items) {
+        const float t = wave_time(sa, 1, sa, wa, none) + wave_time(1, sb, sb, none, wb) + kLaunch;
+        if (t < best_time) { best_time = t; best = {sa, sb, false}; }
+      }
+    }
+  return best;
 }
 
 }  // namespace

@@ -700,7 +700,7 @@ int fo_launch(K kernel, const FoParams& tp, long long blocks, int smem, cudaStre
   if (blocks > 0x7fffffffLL) return FHOB_ERR_SHAPE;
   const int st = allow_smem(kernel, smem);
   if (st != FHOB_OK) return st;
-  FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(blocks), NTHREADS, smem, s, tp));
+  FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(blocks), NTHREADS, smem, 1, s, tp));
   return FHOB_OK;
 }
 

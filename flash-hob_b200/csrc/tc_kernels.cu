@@ -123,6 +123,9 @@ struct TcParams {
   int n_q, n_k, causal, window;
   int tiles_q, tiles_k;   // 128-row tiles of a head
   int q_blocks;           // passes 3 and 4 in one launch: the first q_blocks CTAs are pass 3
+  int items_q, items_k;   // (head, tile) pairs of the query-tiled and key-tiled passes
+  int split_q, split_k;   // CTAs that share the streamed tiles of one such pair
+  int cluster;            // CTAs of a cluster (a multiple of both)
   int heads;              // heads per batch entry of the input tensor maps (4-D: columns, rows, head, batch)
   int d, d_v;             // columns in memory (<= the tile widths DQK, DV; see fill_params)
   int first_live;         // first query with a visible key (causal, n_k < n_q)
@@ -417,7 +420,9 @@ __device__ __forceinline__ float row_dot(const void* o, const void* d_o, int c0,
   return acc;
 }
 
-// One pass over one 128-row tile of one head; `block` numbers the (head, tile) pairs of the pass.
+// One pass over one 128-row tile of one head; `block` numbers the (head, tile, part) triples of the pass.
+// With few tiles the streamed axis is split over the CTAs of a cluster (see choose_split); each computes its
+// part's sums and the cluster adds them up.
 template <int PASS, int DQK, int DV, int BN, int FUSED, bool F16, bool SPLIT>
 __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
   static_assert(FUSED == 0 || PASS == 2, "only pass 2 has a fused form");
@@ -426,6 +431,8 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
   constexpr bool kQStat = PASS != 4;
   constexpr bool kDeep = C::DEEP_FITS && !SPLIT;
   constexpr bool kEarly = early_s(PASS) && !kDeep;
+  constexpr int kPitch = (SPLIT ? 128 : DQK + DV) + 4;   // floats per row of the staging area (split streamed axis)
+  static_assert(PASS <= 2 || BM * kPitch * 4 <= C::STAT_BYTES + C::NSLOT * C::SLOT_BYTES, "staging area");
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* stat_tiles = smem;
   uint8_t* strm_tiles = smem + C::STAT_BYTES;
@@ -433,8 +440,16 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_per_head = kQStat ? p.tiles_q : p.tiles_k;
-  const int head = block / tiles_per_head;
-  const int tile_in_head = block - head * tiles_per_head;
+  const int split = kQStat ? p.split_q : p.split_k;
+  int item = block, part = 0;
+  if (split > 1) {
+    item = block / split;
+    part = block - item * split;
+  }
+  const bool live = item < (kQStat ? p.items_q : p.items_k);   // the grid is padded to whole clusters
+  if (!live) item = 0;
+  const int head = item / tiles_per_head;
+  const int tile_in_head = item - head * tiles_per_head;
   // causal: longest tiles first (late queries in passes 1-3, early keys in pass 4)
   const int tile = kQStat ? tiles_per_head - 1 - tile_in_head : tile_in_head;
   const int m0 = tile * BM;
@@ -444,7 +459,8 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
 
   int t_begin, t_end;
   visible_tiles(kQStat, m0, BM, BN, n_strm, off, p.causal, p.window, t_begin, t_end);
-  const int n_iter = t_end - t_begin;
+  if (split > 1) split_range(part, split, t_begin, t_end);
+  const int n_iter = live ? t_end - t_begin : 0;
 
   auto stat_map = [&](int i) { return &p.map[kQStat ? kMapQ + i : kMapK + i]; };   // Q, ddQ, dO | K, ddK, V, ddV
   auto strm_map = [&](int i) { return &p.map[kQStat ? kMapK + i : kMapQ + i]; };
@@ -725,7 +741,7 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
       if (g_row < p.n_q && g_row >= p.first_live) {
         const int hb = head / p.vo.heads, hh = head - hb * p.vo.heads;
         c.r_nlc = -p.lse[hb * p.lse_batch + hh * p.lse_head + g_row] * kLog2e;
-        if (FUSED == 1) {
+        if (FUSED == 1 && part == 0) {
           using T = typename std::conditional<SPLIT, float, typename std::conditional<F16, __half, __nv_bfloat16>::type>::type;
           constexpr int W = SPLIT ? 32 : DV / 2;
           d_part = row_dot<T, W>(static_cast<const T*>(p.o) + hb * p.vo.batch + hh * p.vo.head + g_row * p.vo.row,
@@ -733,7 +749,7 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
                                  half * W, p.d_v);
         }
       }
-      if (half == 0 && g_row < p.n_q) p.nlc[vec_head + g_row] = c.r_nlc;
+      if (half == 0 && part == 0 && g_row < p.n_q) p.nlc[vec_head + g_row] = c.r_nlc;
     } else if (kQStat && g_row < p.n_q) {
       c.r_nlc = p.nlc[vec_head + g_row];
       if (PASS >= 2) {
@@ -837,7 +853,15 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
       if (half == 1) bars->red[row] = d_row;
       asm volatile("bar.sync 1, 256;" ::: "memory");
       if (half == 0) d_row += bars->red[row];
-      if (half == 0 && ok && g_row < p.n_q) {
+      if (split > 1) {
+        // this part's sums; the stationary tiles are no longer read
+        float* sums = reinterpret_cast<float*>(stat_tiles);
+        if (half == 0) {
+          sums[row] = r1;
+          sums[BM + row] = rb;
+          sums[2 * BM + row] = d_row;
+        }
+      } else if (half == 0 && ok && g_row < p.n_q) {
         const float dd = c.scale * r1;
         p.ndd[vec_head + g_row] = -dd;
         p.k23[vec_head + g_row] = d_row * dd - rb;  // -D*dd - b = D*dd - (sum P X + scale * sum dP P A2)
@@ -854,7 +878,36 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
     } else {
       if (n_iter > 0) ok = ok && __all_sync(0xffffffffu, wait_bar(&bars->out_full, 0, bars, p.status));
       tc_fence_after();
-      if (ok) {
+      if (split > 1) {
+        float* dst = reinterpret_cast<float*>(smem) + row * kPitch;   // every tile has been read: out_full follows the last product
+        const uint32_t acc = tmem_base + lane_base;
+        if constexpr (SPLIT) {
+          // a result is the sum of the two 64-column halves of its accumulator
+#pragma unroll
+          for (int o = 0; o < 2; ++o) {
+            uint32_t a[16], b[16];
+#pragma unroll
+            for (int ch = 0; ch < 32; ch += 16) {
+              if (n_iter > 0) {
+                tmem_ld16(acc + o * 128 + half * 32 + ch, a);
+                tmem_ld16(acc + o * 128 + 64 + half * 32 + ch, b);
+                tmem_wait_ld();
+              } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) a[j] = b[j] = 0u;
+              }
+#pragma unroll
+              for (int j = 0; j < 16; j += 4)
+                *reinterpret_cast<float4*>(dst + o * 64 + half * 32 + ch + j) =
+                    make_float4(__uint_as_float(a[j]) + __uint_as_float(b[j]), __uint_as_float(a[j + 1]) + __uint_as_float(b[j + 1]),
+                                __uint_as_float(a[j + 2]) + __uint_as_float(b[j + 2]), __uint_as_float(a[j + 3]) + __uint_as_float(b[j + 3]));
+            }
+          }
+        } else {
+          stage_row<DQK / 2>(dst + half * (DQK / 2), acc + half * (DQK / 2), n_iter > 0);
+          stage_row<DV / 2>(dst + DQK + half * (DV / 2), acc + C::OUT0_COLS + half * (DV / 2), n_iter > 0);
+        }
+      } else if (ok) {
         auto store_out = [&](auto width, int d_mem, uint32_t col0, void* base, float mul) {
           constexpr int DO = decltype(width)::value;   // columns of the accumulator; d_mem <= DO of them exist in memory
           uint16_t* dst = static_cast<uint16_t*>(base) + (static_cast<size_t>(head) * n_stat + (g_row < n_stat ? g_row : 0)) * d_mem + half * (DO / 2);
@@ -918,6 +971,38 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
         }
       }
     }
+  }
+
+  // ---- split streamed axis: add up the parts
+  if ((FUSED || PASS >= 3) && p.cluster > 1) {
+    __syncwarp();
+    cluster_sync();
+    const int tid = threadIdx.x - EW_WARP0 * 32, rank0 = static_cast<int>(cluster_rank()) - part;
+    if (split > 1 && live && tid >= 0) {
+      if constexpr (FUSED != 0) {
+        const int g_row = m0 + tid;
+        if (part == 0 && tid < BM && g_row < p.n_q) {
+          float r1 = 0.f, rb = 0.f, d_row = 0.f;
+          for (int i = 0; i < split; ++i) {
+            const uint32_t from = cluster_map(smem_u32(stat_tiles) + tid * 4, rank0 + i);
+            r1 += cluster_ld(from);
+            rb += cluster_ld(from + BM * 4);
+            d_row += cluster_ld(from + 2 * BM * 4);
+          }
+          const size_t at = static_cast<size_t>(head) * row_stride(p.n_q) + g_row;
+          const float dd = p.scale * r1;
+          p.ndd[at] = -dd;
+          p.k23[at] = d_row * dd - rb;
+          p.k1[at] = -d_row;
+        }
+      } else {
+        void *out0 = kQStat ? p.dq2 : p.dk2, *out1 = kQStat ? p.ddo : p.dv2;
+        constexpr int W0 = SPLIT ? 64 : DQK, W1 = SPLIT ? 64 : DV;
+        reduce_store<W0, SPLIT, F16>(smem_u32(smem), kPitch, 0, rank0, part, split, tid, out0, head, m0, n_stat, p.d, p.scale);
+        reduce_store<W1, SPLIT, F16>(smem_u32(smem), kPitch, W0, rank0, part, split, tid, out1, head, m0, n_stat, p.d_v, 1.f);
+      }
+    }
+    cluster_sync();   // the others are done with this CTA's shared memory
   }
 
   // ---- teardown
@@ -984,6 +1069,8 @@ int first_live_query(const FhobProblem& p) {
 
 template <bool F16, bool SPLIT>
 int fill_params(const FhobProblem& p, TcParams& tp) {
+  const long long most_items = static_cast<long long>((p.n_q > p.n_k ? p.n_q : p.n_k) + BM - 1) / BM * p.bh;
+  if (most_items > 0x3fffffffLL) return FHOB_ERR_SHAPE;   // both passes together stay below 2^31 CTAs
   RowVectors rv = row_vectors(p);
   const void* mats[kMaps] = {p.q, p.ddq, p.d_o, p.k, p.ddk, p.v, p.ddv};
   const int ids[kMaps] = {kTenQ, kTenDDQ, kTenDO, kTenK, kTenDDK, kTenV, kTenDDV};
@@ -1016,6 +1103,9 @@ int fill_params(const FhobProblem& p, TcParams& tp) {
   tp.tiles_q = (p.n_q + BM - 1) / BM;
   tp.tiles_k = (p.n_k + BM - 1) / BM;
   tp.q_blocks = 0;
+  tp.items_q = tp.tiles_q * p.bh;   // at most 2^31 - 1: checked by the caller
+  tp.items_k = tp.tiles_k * p.bh;
+  tp.split_q = tp.split_k = tp.cluster = 1;
   tp.heads = (!SPLIT && p.layout) ? p.layout->heads : p.bh;
   tp.d = p.d;
   tp.d_v = dv;
@@ -1025,27 +1115,48 @@ int fill_params(const FhobProblem& p, TcParams& tp) {
 
 template <class K>
 int launch(K kernel, const TcParams& tp, long long blocks, int smem, cudaStream_t s) {
-  if (blocks > 0x7fffffffLL) return FHOB_ERR_SHAPE;
   const int st = allow_smem(kernel, smem);
   if (st != FHOB_OK) return st;
-  FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(blocks), NTHREADS, smem, s, tp));
+  FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(blocks), NTHREADS, smem, tp.cluster, s, tp));
   return FHOB_OK;
 }
 
 template <int PASS, int DQK, int DV, int BN, int FUSED, bool F16, bool SPLIT>
-int launch_pass(const FhobProblem& p, const TcParams& tp, cudaStream_t s) {
-  return launch(tc_pass_kernel<PASS, DQK, DV, BN, FUSED, F16, SPLIT>, tp, static_cast<long long>(tp.tiles_q) * p.bh,
-                Cfg<PASS, DQK, DV, BN>::SMEM_BYTES, s);
+int launch_pass(TcParams& tp, cudaStream_t s) {
+  constexpr auto kernel = tc_pass_kernel<PASS, DQK, DV, BN, FUSED, F16, SPLIT>;
+  constexpr int kSmem = Cfg<PASS, DQK, DV, BN>::SMEM_BYTES;
+  if (FUSED && may_split(tp.n_q, tp.n_k)) {
+    const int st = allow_smem(kernel, kSmem);
+    if (st != FHOB_OK) return st;
+    tp.split_q = tp.cluster = choose_split(kernel, kSmem, SplitWork{tp.items_q, (tp.n_k + BN - 1) / BN}, SplitWork{0, 0}).a;
+  }
+  return launch(kernel, tp, static_cast<long long>(tp.items_q) * tp.split_q, kSmem, s);
 }
 
+// Passes 3 and 4, or one of them.
 template <int DQK, int DV, bool F16, bool SPLIT>
-int launch_34(const FhobProblem& p, TcParams& tp, bool pass3, bool pass4, cudaStream_t s) {
+int launch_34(TcParams& tp, bool pass3, bool pass4, cudaStream_t s) {
+  constexpr auto kernel = tc_pass34_kernel<DQK, DV, F16, SPLIT>;
   constexpr int kSmem3 = Cfg<3, DQK, DV, 64>::SMEM_BYTES, kSmem4 = Cfg<4, DQK, DV, 64>::SMEM_BYTES;
-  const long long q_blocks = pass3 ? static_cast<long long>(tp.tiles_q) * p.bh : 0;
-  const long long k_blocks = pass4 ? static_cast<long long>(tp.tiles_k) * p.bh : 0;
-  if (q_blocks > 0x7fffffffLL) return FHOB_ERR_SHAPE;
-  tp.q_blocks = static_cast<int>(q_blocks);
-  return launch(tc_pass34_kernel<DQK, DV, F16, SPLIT>, tp, q_blocks + k_blocks, kSmem3 > kSmem4 ? kSmem3 : kSmem4, s);
+  constexpr int kSmem = kSmem3 > kSmem4 ? kSmem3 : kSmem4;
+  const SplitWork w3 = {pass3 ? tp.items_q : 0, (tp.n_k + 63) / 64}, w4 = {pass4 ? tp.items_k : 0, (tp.n_q + 63) / 64};
+  SplitChoice c = {1, 1, true};
+  if (may_split(tp.n_q, tp.n_k)) {
+    const int st = allow_smem(kernel, kSmem);
+    if (st != FHOB_OK) return st;
+    c = choose_split(kernel, kSmem, w3, w4);
+  }
+  auto go = [&](int items3, int items4, int cluster) {
+    // whole clusters for either pass, so that the parts of an item are neighbours in one cluster
+    auto padded = [&](long long n) { return (n + cluster - 1) / cluster * cluster; };
+    tp.split_q = c.a; tp.split_k = c.b;
+    tp.cluster = cluster;
+    tp.q_blocks = static_cast<int>(padded(static_cast<long long>(items3) * c.a));
+    return launch(kernel, tp, tp.q_blocks + padded(static_cast<long long>(items4) * c.b), kSmem, s);
+  };
+  if (c.together) return go(w3.items, w4.items, c.a > c.b ? c.a : c.b);
+  const int st = go(w3.items, 0, c.a);
+  return st != FHOB_OK ? st : go(0, w4.items, c.b);
 }
 
 // `pass`: 1, 2, 3, 4 alone, 12 = passes 1 and 2 in one sweep, kWholeOperator = the sweep, then passes 3 and 4
@@ -1058,16 +1169,16 @@ int dispatch(int pass, const FhobProblem& p, cudaStream_t s) {
   switch (pass) {
     // pass 1 streams 128-row tiles (the stacked [K ; ddK] operand reaches N = 256), the others 64;
     // it touches no tile of the second head dim
-    case 1: return launch_pass<1, DQK, DQK, 128, 0, F16, SPLIT>(p, tp, s);
-    case 2: return launch_pass<2, DQK, DV, 64, 0, F16, SPLIT>(p, tp, s);
-    case 3: return launch_34<DQK, DV, F16, SPLIT>(p, tp, true, false, s);
-    case 4: return launch_34<DQK, DV, F16, SPLIT>(p, tp, false, true, s);
+    case 1: return launch_pass<1, DQK, DQK, 128, 0, F16, SPLIT>(tp, s);
+    case 2: return launch_pass<2, DQK, DV, 64, 0, F16, SPLIT>(tp, s);
+    case 3: return launch_34<DQK, DV, F16, SPLIT>(tp, true, false, s);
+    case 4: return launch_34<DQK, DV, F16, SPLIT>(tp, false, true, s);
     case 12:
     case kWholeOperator:
       // without O the sweep also produces D = sum P dP
-      st = p.o ? launch_pass<2, DQK, DV, 64, 1, F16, SPLIT>(p, tp, s) : launch_pass<2, DQK, DV, 64, 2, F16, SPLIT>(p, tp, s);
+      st = p.o ? launch_pass<2, DQK, DV, 64, 1, F16, SPLIT>(tp, s) : launch_pass<2, DQK, DV, 64, 2, F16, SPLIT>(tp, s);
       if (st != FHOB_OK || pass == 12) return st;
-      return launch_34<DQK, DV, F16, SPLIT>(p, tp, true, true, s);
+      return launch_34<DQK, DV, F16, SPLIT>(tp, true, true, s);
   }
   return FHOB_ERR_ARG;
 }
@@ -1141,7 +1252,7 @@ int tc_split_inputs(const FhobProblem& p, cudaStream_t s, int which) {
   }
   const long blocks = (most + 255) / 256;
   if (blocks > 0x7fffffffL) return FHOB_ERR_SHAPE;
-  FHOB_CUDA_OK(launch_pdl(split_rows_kernel, dim3(static_cast<unsigned>(blocks), count), 256, 0, s, jobs));
+  FHOB_CUDA_OK(launch_pdl(split_rows_kernel, dim3(static_cast<unsigned>(blocks), count), 256, 0, 1, s, jobs));
   return FHOB_OK;
 }
 
