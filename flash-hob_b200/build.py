@@ -22,7 +22,7 @@ OBJ = HERE / "build"
 OUT = HERE / "fhob" / "libfhob.so"
 NATIVE = HERE / "fhob" / "_native.so"          # host path of the Python package, against torch's C++ API
 NATIVE_SOURCE = "host_binding.cpp"
-SOURCES = ["fhob_api.cu", "simt_kernels.cu", "tc_kernels.cu", "tc_first_order.cu", "static_scratch.cu"]
+SOURCES = ["fhob_api.cu", "simt_kernels.cu", "tc_kernels.cu", "tc_forward.cu", "tc_backward.cu", "static_scratch.cu"]
 HEADERS = ["fhob_common.cuh", "sm100_ptx.cuh", "tc_common.cuh", "../../include/fhob.h"]
 FLAGS = ["-Xcompiler", "-fPIC", "-O3", "-std=c++17", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a"]
 

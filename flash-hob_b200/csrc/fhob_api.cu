@@ -6,7 +6,7 @@
 #include <cstring>
 #include <mutex>
 
-#include "fhob_common.cuh"
+#include "tc_common.cuh"
 
 namespace fhob {
 
@@ -32,6 +32,8 @@ __global__ void prepass_kernel(const T* __restrict__ o, const T* __restrict__ d_
                                float* __restrict__ nlc, float* __restrict__ k1, int* status, unsigned blocks_per_head, int d,
                                int n_q, int first_live_query, View vo, View vdo, long long lse_head,
                                long long lse_batch, int lanes) {
+  ptx::pdl_wait();
+  if (threadIdx.x == 0) ptx::pdl_launch_dependents();
   if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
   // blocks do not straddle heads: head and row come from 32-bit arithmetic that is uniform per block
   const int groups = blockDim.x / lanes;
@@ -251,20 +253,12 @@ static int run_prepass(const FhobProblem* p, void* stream, bool for_operator = t
   const View vo = tensor_view(*p, kTenO, p->n_q, dv_), vdo = tensor_view(*p, kTenDO, p->n_q, dv_);
   const long long lse_head = p->layout ? p->layout->lse_head : p->n_q;
   const long long lse_batch = p->layout ? p->layout->lse_batch : static_cast<long long>(p->bh) * p->n_q;
-  if (p->dtype == FHOB_BF16) {
-    prepass_kernel<__nv_bfloat16><<<grid, threads, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(p->o), static_cast<const __nv_bfloat16*>(p->d_o), p->lse, rv.nlc, rv.k1,
-        rv.status, blocks_per_head, dv_, p->n_q, first_live, vo, vdo, lse_head, lse_batch, lanes);
-  } else if (p->dtype == FHOB_F16) {
-    prepass_kernel<__half><<<grid, threads, 0, s>>>(static_cast<const __half*>(p->o),
-                                                       static_cast<const __half*>(p->d_o), p->lse, rv.nlc, rv.k1,
-                                                       rv.status, blocks_per_head, dv_, p->n_q, first_live, vo, vdo, lse_head, lse_batch, lanes);
-  } else {
-    prepass_kernel<float><<<grid, threads, 0, s>>>(static_cast<const float*>(p->o),
-                                                      static_cast<const float*>(p->d_o), p->lse, rv.nlc, rv.k1,
-                                                      rv.status, blocks_per_head, dv_, p->n_q, first_live, vo, vdo, lse_head, lse_batch, lanes);
-  }
-  FHOB_CUDA_OK(cudaGetLastError());
+  auto go = [&](auto type) {
+    using T = decltype(type);
+    return launch_pdl(prepass_kernel<T>, grid, threads, 0, 1, s, static_cast<const T*>(p->o), static_cast<const T*>(p->d_o), p->lse,
+                      rv.nlc, rv.k1, rv.status, blocks_per_head, dv_, p->n_q, first_live, vo, vdo, lse_head, lse_batch, lanes);
+  };
+  FHOB_CUDA_OK(p->dtype == FHOB_BF16 ? go(__nv_bfloat16{}) : (p->dtype == FHOB_F16 ? go(__half{}) : go(float{})));
   return FHOB_OK;
 }
 

@@ -179,7 +179,7 @@ int tc_split_inputs(const FhobProblem& p, cudaStream_t s, int which = kSplitAll)
 int tc_pass(int pass, const FhobProblem& p, cudaStream_t s);
 int tc_operator(const FhobProblem& p, cudaStream_t s);   // the whole double backward
 
-// tensor-core forward (O, L) and first backward (dQ, dK, dV): tc_first_order.cu
+// tensor-core forward (O, L): tc_forward.cu, and first backward (dQ, dK, dV): tc_backward.cu
 bool tc_first_order_supported(const FhobProblem& p);
 int tc_forward(const FhobProblem& p, void* o_out, float* lse_out, int* status, cudaStream_t s);
 int tc_backward(const FhobProblem& p, void* dq, void* dk, void* dv, cudaStream_t s);

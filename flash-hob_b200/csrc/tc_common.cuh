@@ -56,6 +56,17 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, B* b, i
   }
 }
 
+// Bounded wait for something already in flight (a load to land, products to finish) before the CTA exits.
+__device__ __forceinline__ void wait_landed(uint64_t* bar, uint32_t parity, int* status) {
+  const long long start = clock64();
+  while (!mbar_try_wait(bar, parity)) {
+    if (clock64() - start > kTimeoutCycles) {
+      atomicOr(status, FHOB_ERR_TIMEOUT);
+      break;
+    }
+  }
+}
+
 // Descriptor words of 128-byte-swizzled bf16 tiles (rows of 64 elements, 8-row groups 1024 B apart).
 constexpr uint32_t kDescHi = umma_desc_hi_sw128(1024);
 
@@ -106,6 +117,29 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, 
 #pragma unroll
     for (int by = 0; by < ROWS / BOX_ROWS; ++by)
       tma_load_4d(dst + bx * BOX + by * (BOX_ROWS * 128), map, bar, bx * 64, y + by * BOX_ROWS, head, batch);
+}
+
+// 2^x for two numbers on the FMA and ALU pipes, to relieve the special-function units (16 a clock and SM)
+// where they are what a kernel waits for.  x = n + f with n the nearest integer, |f| <= 1/2; 2^f is the
+// degree-5 polynomial with the smallest relative error there (Remez exchange, 7.5e-8; 2.1e-7 evaluated in
+// fp32, as ex2.approx: 2^-22), and n is added to the exponent field.  x <= 127; below -126 the result
+// is about 2^-126 or less, never a larger number.
+__device__ __forceinline__ float2 exp2_fma(float2 x) {
+  constexpr float kMagic = 12582912.f;   // 1.5 * 2^23: adding it leaves the nearest integer in the low bits
+  x.x = fmaxf(x.x, -126.f);
+  x.y = fmaxf(x.y, -126.f);
+  const float2 r = __fadd2_rn(x, make_float2(kMagic, kMagic));
+  const float2 n = __fadd2_rn(r, make_float2(-kMagic, -kMagic));
+  const float2 f = __ffma2_rn(n, make_float2(-1.f, -1.f), x);
+  auto c = [](float v) { return make_float2(v, v); };
+  float2 y = __ffma2_rn(c(0.0013276472f), f, c(0.009675541f));
+  y = __ffma2_rn(y, f, c(0.05550713f));
+  y = __ffma2_rn(y, f, c(0.2402212f));
+  y = __ffma2_rn(y, f, c(0.69314694f));
+  y = __ffma2_rn(y, f, c(1.0000001f));
+  y.x = __uint_as_float(__float_as_uint(y.x) + (__float_as_uint(r.x) << 23));
+  y.y = __uint_as_float(__float_as_uint(y.y) + (__float_as_uint(r.y) << 23));
+  return y;
 }
 
 // ---- split streamed axis: a cluster of `split` CTAs shares the streamed tiles of one stationary tile
@@ -172,6 +206,19 @@ __device__ __forceinline__ void reduce_store(uint32_t stage, int pitch, int c0, 
 }
 
 // ------------------------------------------------------------------ host side
+int check_device() {
+  static thread_local int checked_dev = -1;
+  int dev = 0;
+  FHOB_CUDA_OK(cudaGetDevice(&dev));
+  if (dev != checked_dev) {
+    int major = 0;
+    FHOB_CUDA_OK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
+    if (major != 10) return FHOB_ERR_ARCH;
+    checked_dev = dev;
+  }
+  return FHOB_OK;
+}
+
 // Launches with programmatic stream serialization: the kernel's CTAs may start while the kernel in
 // front of it drains (it says pdl_launch_dependents), and wait in pdl_wait before they touch memory.
 template <class... P, class... A>

@@ -550,13 +550,7 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
       wait_bar(&bars->stat_full, 0, bars, p.status);
       for (int it = issued > C::NSLOT ? issued - C::NSLOT : 0; it < issued; ++it) {
         const int slot = it % C::NSLOT;
-        const long long start = clock64();
-        while (!mbar_try_wait(&bars->strm_full[slot], (it / C::NSLOT) & 1)) {
-          if (clock64() - start > kTimeoutCycles) {
-            atomicOr(p.status, FHOB_ERR_TIMEOUT);
-            break;
-          }
-        }
+        wait_landed(&bars->strm_full[slot], (it / C::NSLOT) & 1, p.status);
       }
     }
   } else if (warp == MMA_WARP || warp == MMA_WARP2) {
@@ -717,10 +711,7 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
       } else {
         // abort path: no tcgen05.mma may still be reading shared memory or TMEM at exit
         commit(&bars->teardown[chain]);
-        const long long start = clock64();
-        while (!mbar_try_wait(&bars->teardown[chain], 0)) {
-          if (clock64() - start > kTimeoutCycles) break;
-        }
+        wait_landed(&bars->teardown[chain], 0, p.status);
       }
     }
   } else if (warp >= EW_WARP0) {
@@ -1191,19 +1182,6 @@ int dispatch_dims(int pass, const FhobProblem& p, cudaStream_t s) {
   return dv <= 64 ? dispatch<128, 64, F16>(pass, p, s) : dispatch<128, 128, F16>(pass, p, s);
 }
 
-int check_arch() {
-  static thread_local int checked_dev = -1;
-  int dev = 0;
-  FHOB_CUDA_OK(cudaGetDevice(&dev));
-  if (dev != checked_dev) {
-    int major = 0;
-    FHOB_CUDA_OK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
-    if (major != 10) return FHOB_ERR_ARCH;
-    checked_dev = dev;
-  }
-  return FHOB_OK;
-}
-
 }  // namespace
 
 bool tc_supported(const FhobProblem& p) {
@@ -1258,7 +1236,7 @@ int tc_split_inputs(const FhobProblem& p, cudaStream_t s, int which) {
 
 int tc_pass(int pass, const FhobProblem& p, cudaStream_t s) {
   if (!tc_supported(p)) return FHOB_ERR_SHAPE;
-  int st = check_arch();
+  int st = check_device();
   if (st != FHOB_OK) return st;
   if (p.dtype == FHOB_F32) return dispatch<128, 128, false, true>(pass, p, s);
   return p.dtype == FHOB_F16 ? dispatch_dims<true>(pass, p, s) : dispatch_dims<false>(pass, p, s);
