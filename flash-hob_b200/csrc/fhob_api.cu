@@ -275,8 +275,7 @@ int fhob_pass12(const FhobProblem* p, void* stream) {
   if (st != FHOB_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (use_tc(*p)) return tc_pass(12, *p, s);
-  st = simt_pass(1, *p, s);
-  return st != FHOB_OK ? st : simt_pass(2, *p, s);
+  return simt_pass(12, *p, s);
 }
 int fhob_pass3(const FhobProblem* p, void* stream) { return run_pass(3, p, stream); }
 int fhob_pass4(const FhobProblem* p, void* stream) { return run_pass(4, p, stream); }
@@ -290,11 +289,8 @@ int fhob_bwdbwd(const FhobProblem* p, void* stream) {
   if (use_tc(*p)) return tc_operator(*p, s);
   st = run_prepass(p, stream);
   if (st != FHOB_OK) return st;
-  for (int pass = 1; pass <= 4; ++pass) {
-    st = simt_pass(pass, *p, s);
-    if (st != FHOB_OK) return st;
-  }
-  return FHOB_OK;
+  st = simt_pass(12, *p, s);
+  return st != FHOB_OK ? st : simt_pass(34, *p, s);
 }
 
 int fhob_row_stats(const FhobProblem* p, float* d_out, float* dd_out, float* b_out, void* stream) {

@@ -1,27 +1,25 @@
 // CUDA-core (FFMA) kernels of the double-backward attention operator.
 //
-// They serve fp32 problems, where bf16 tensor-core products could not reach a
-// 1e-4 relative error, and any bf16 problem the caller forces onto them.  The
-// algorithm is the same four recomputation passes as the tensor-core kernels
-// (reference: fhog/triton_bwdbwd.py:178-313 for the query-tiled passes 1-3,
-// :321-535 for the key-tiled pass 4): a CTA keeps TM "stationary" rows in
-// shared memory, streams TN rows of the other side per step, rebuilds the four
-// score-shaped tiles S, A2, dP, X from fp32 dot products, applies the
-// elementwise formulas of fhob_common.cuh and either reduces along the row
-// (passes 1, 2) or feeds the resulting tiles into the output products
-// (passes 3, 4).  Arbitrary n_q, n_k and head dims <= 128 are handled by bounds
-// checks; pairs outside the matrix or hidden by the causal mask contribute zero.
+// They serve fp32 problems with a head dim above 64, and any problem the caller
+// forces onto them.  The algorithm is that of the tensor-core kernels
+// (reference: fhog/triton_bwdbwd.py:178-313 for the query-tiled passes, :321-535
+// for the key-tiled one): a CTA keeps "stationary" rows in shared memory, streams
+// rows of the other side, rebuilds the score-shaped tiles S, A2, dP, X from fp32
+// dot products, applies the elementwise formulas of fhob_common.cuh and either
+// reduces along the row (the sweep) or feeds the resulting tiles into the output
+// products (passes 3, 4).  Arbitrary n_q, n_k and head dims <= 128 are handled by
+// bounds checks; pairs outside the matrix or hidden by the mask contribute zero.
 // Two head dims: Q, K, ddQ, ddK, dQ2, dK2 have `d` columns, V, ddV, dO, O, ddO, dV2
-// have `dv` (jax_refs/flash_impl.py:381-389 has d_in != d_out); shared-memory
-// tiles all use the row pitch of the larger one.
+// have `dv` (jax_refs/flash_impl.py:381-389 has d_in != d_out).
 #include "fhob_common.cuh"
 
 namespace fhob {
 namespace {
 
+constexpr int NT = 256;       // threads per CTA
+// the forward: 8 warps, warp w owns rows 4w..4w+3, lane = column
 constexpr int TM = 32;        // stationary rows per CTA
 constexpr int TN = 32;        // streamed rows per step
-constexpr int NT = 256;       // threads per CTA: 8 warps, warp w owns rows 4w..4w+3, lane = column
 constexpr int RPW = TM / 8;   // rows per warp
 constexpr int DCH = 4;        // output columns per thread and row: lane + 32*m, m < DCH  (d <= 128)
 
@@ -91,214 +89,380 @@ __device__ __forceinline__ float warp_max(float x) {
   return x;
 }
 
-// PASS 1..3: stationary = query tile, streamed = key tiles.
-// PASS 4:    stationary = key tile,   streamed = query tiles.
-template <typename T, int PASS>
-__global__ void __launch_bounds__(NT) simt_pass_kernel(const SimtParams p) {
-  extern __shared__ float smem[];
-  const int d = p.d, dv = p.dv;
-  const int ld = (d > dv ? d : dv) + 1;
-  constexpr bool kQStationary = PASS != 4;
-  float* stat[4];
-  float* strm[4];
-  for (int i = 0; i < 4; ++i) stat[i] = smem + i * TM * ld;
-  for (int i = 0; i < 4; ++i) strm[i] = smem + (4 * TM + i * TN) * ld;
-  float* sacc = smem + (4 * TM + 4 * TN) * ld;     // [4][TM][TN+1]: S, A2, dP, X
-  float* ptile = sacc + 4 * TM * (TN + 1);          // [4][TM][TN+1]: P-type tiles
-  float* svec = ptile + 4 * TM * (TN + 1);          // [4][TN]: row vectors of streamed queries (pass 4)
-  constexpr int LT = TN + 1;
+// ---- the operator's passes and the first backward
+//
+// What bounds them is the FMA pipe (128 a clock and SM) and, close behind, shared-memory reads: a
+// 16-byte read by a warp takes up to four clocks of the SM's one read port, so a thread has to make about
+// 16 multiply-adds of every float4 it reads.  A CTA owns OM = 64 stationary rows and streams ON = 32;
+// two groups of four warps take one half of the work of each phase:
+//
+//   scores    group 0: S, A2 (4 x 4 of the 64 x 32 tile a thread, 12 FMA per float4 read)
+//             group 1: dP, X                                     (10.7)
+//   elements  group 0: P, t, ddP;  then group 1: dS, dS2          (tiles pass through shared memory)
+//   outputs   group 0: dQ2 | dK2,  group 1: ddO | dV2             (8 x 8 of 64 x 128 a thread, 16)
+//
+// Warps w and w + 4 share a scheduler, so the pipe stays busy while the groups' shares differ.  Products
+// are packed fp32 pairs (fma.f32x2): over even and odd elements of the contraction in the scores,
+// over neighbouring columns in the outputs; a packed FMA takes one issue slot for two.
+// Row statistics come from one sweep (MODE 2).  With D known, centred sums need neither dd nor a second pass:
+//   dd = scale sum P A2,   k23 = -D dd - b = -sum P (X + (dP - D) scale A2).
+// Passes 3 and 4 share a launch, as do the two halves of the first backward.
+//
+// fp32, 8 heads, N = 1024, D = 128, the operator: 4884 -> 1316 us
+// (one 4 x 1 strip of scores a thread, four passes in launches of their own, before).
+constexpr int OM = 64;
+constexpr int ON = 32;
+constexpr int OP = 128 + 4;    // row pitch of the operand tiles: 8 neighbouring rows lie in different banks
+constexpr int PP = OM + 4;     // row pitch of the tiles of P and its derivatives, stored [streamed][stationary]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * TM;
-  const int bh = blockIdx.y + blockIdx.z * kMaxGridY;   // see head_grid
-  if (bh >= p.bh) return;
+// MODE 2 = sweep, 3, 4 = passes 3 and 4 (dQ2, ddO | dK2, dV2), 5, 6 = first backward (dQ | dK, dV)
+template <int MODE>
+struct Tiles {
+  static constexpr bool kQStat = MODE != 4 && MODE != 6;
+  static constexpr bool kFirst = MODE >= 5;                    // first backward: S and dP alone
+  static constexpr bool kBoth2 = MODE == 2 || MODE == 3;       // X = dO . ddV^T reads a streamed tile of its own
+  // tiles: 0 = Q | K, 1 = ddQ | ddK, 2 = dO | V (streamed: V | dO), 3 = ddV
+  static constexpr int NSTAT = kFirst ? 2 : (MODE == 4 ? 4 : 3);
+  static constexpr int NSTRM = kFirst ? 2 : (MODE == 4 ? 3 : 4);
+  static constexpr int NP = MODE == 3 ? 4 : (MODE == 4 ? 3 : 2);
+  static constexpr int SMEM_BYTES = 4 * (NSTAT * OM * OP + NSTRM * ON * OP + NP * ON * PP + 4 * ON);
+  static_assert(SMEM_BYTES <= 232448, "shared memory");
+};
+
+__device__ __forceinline__ void cp_async16(float* dst, const void* src, bool live) {
+  const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+
+// Rows [row0, row0 + rows) of a head's (n, d) matrix -> [rows][OP] fp32, zero beyond n.  Rows are whole
+// 16-byte pieces and the base is 16-byte aligned (checked by the entry points).  fp32 arrives asynchronously.
+template <typename T>
+__device__ __forceinline__ void load_rows(float* tile, const void* src, size_t head_off, int row0, int rows, int n, int d) {
+  constexpr int V = 16 / sizeof(T);
+  const int pieces = d / V;
+  const T* base = static_cast<const T*>(src) + head_off;
+  for (int idx = threadIdx.x; idx < rows * pieces; idx += NT) {
+    const int r = idx / pieces, c = (idx - r * pieces) * V;
+    const bool live = row0 + r < n;
+    const T* from = base + static_cast<size_t>(live ? row0 + r : 0) * d + c;
+    float* to = tile + r * OP + c;
+    if constexpr (V == 4) {
+      cp_async16(to, from, live);
+    } else {
+      uint4 w = make_uint4(0u, 0u, 0u, 0u);
+      if (live) w = *reinterpret_cast<const uint4*>(from);
+      const T* e = reinterpret_cast<const T*>(&w);
+      *reinterpret_cast<float4*>(to) = make_float4(static_cast<float>(e[0]), static_cast<float>(e[1]), static_cast<float>(e[2]), static_cast<float>(e[3]));
+      *reinterpret_cast<float4*>(to + 4) = make_float4(static_cast<float>(e[4]), static_cast<float>(e[5]), static_cast<float>(e[6]), static_cast<float>(e[7]));
+    }
+  }
+}
+__device__ __forceinline__ void loads_landed() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
+
+// acc[i][j] += a_i . b_j over four elements, even and odd ones apart
+__device__ __forceinline__ void dot4(float2& acc, const float4& a, const float4& b) {
+  acc = __ffma2_rn(lo2(a), lo2(b), acc);
+  acc = __ffma2_rn(hi2(a), hi2(b), acc);
+}
+
+// out (8 rows x 8 columns: 4 at col, 4 at col + 64) += at[c][rows] . b[c][cols] over the ON streamed rows,
+// for one or two such products.  WIDE: the second four columns exist.
+template <bool TWO, bool WIDE>
+__device__ __forceinline__ void outer(float2 (&out)[8][4], const float* a0, const float* b0, const float* a1, const float* b1) {
+#pragma unroll 4
+  for (int c = 0; c < ON; ++c) {
+#pragma unroll
+    for (int t = 0; t < (TWO ? 2 : 1); ++t) {
+      const float* a = (t ? a1 : a0) + c * PP;
+      const float* b = (t ? b1 : b0) + c * OP;
+      const float4 al = ld4(a), ah = ld4(a + 4), bl = ld4(b);
+      float4 bh = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (WIDE) bh = ld4(b + 64);
+      const float r[8] = {al.x, al.y, al.z, al.w, ah.x, ah.y, ah.z, ah.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float2 rr = make_float2(r[i], r[i]);
+        out[i][0] = __ffma2_rn(rr, lo2(bl), out[i][0]);
+        out[i][1] = __ffma2_rn(rr, hi2(bl), out[i][1]);
+        if (WIDE) {
+          out[i][2] = __ffma2_rn(rr, lo2(bh), out[i][2]);
+          out[i][3] = __ffma2_rn(rr, hi2(bh), out[i][3]);
+        }
+      }
+    }
+  }
+}
+
+// Four neighbouring columns of a result row.
+template <typename T>
+__device__ __forceinline__ void store4(void* base, size_t at, const float2& a, const float2& b, float mul) {
+  if constexpr (sizeof(T) == 4) {
+    *reinterpret_cast<float4*>(static_cast<float*>(base) + at) = make_float4(a.x * mul, a.y * mul, b.x * mul, b.y * mul);
+  } else {
+    T w[4] = {static_cast<T>(a.x * mul), static_cast<T>(a.y * mul), static_cast<T>(b.x * mul), static_cast<T>(b.y * mul)};
+    *reinterpret_cast<uint2*>(static_cast<T*>(base) + at) = *reinterpret_cast<const uint2*>(w);
+  }
+}
+
+template <typename T, int MODE>
+__device__ __forceinline__ void simt_body(const SimtParams& p, int item) {
+  using C = Tiles<MODE>;
+  constexpr bool kQStat = C::kQStat, kFirst = C::kFirst;
+  extern __shared__ float smem[];
+  // first backward: tiles 0 and 2 only, stored one after the other
+  float* stat[4] = {smem, smem + OM * OP, smem + (kFirst ? 1 : 2) * OM * OP, smem + 3 * OM * OP};
+  float* strm0 = smem + C::NSTAT * OM * OP;
+  float* strm[4] = {strm0, strm0 + ON * OP, strm0 + (kFirst ? 1 : 2) * ON * OP, strm0 + 3 * ON * OP};
+  float* pt0 = strm0 + C::NSTRM * ON * OP;
+  float* svec = pt0 + C::NP * ON * PP;   // key-tiled: nlc, ndd, k1, k23 of the streamed queries
+  // tiles of P and its derivatives.  t and (unless it is an operand itself) P wait where dS and dS2 go.
+  float* pt[4] = {pt0, pt0 + ON * PP, pt0 + 2 * ON * PP, pt0 + 3 * ON * PP};
+  float* const p_tile = MODE == 3 ? pt[3] : pt[1];
+
+  const int d = p.d, dv = p.dv;
+  const int group = threadIdx.x >> 7, tid = threadIdx.x & 127;
+  const int ty = tid >> 3, tx = tid & 7;     // scores: rows 4 ty + i, streamed rows tx + 8 j
+  const int ry = tid >> 4, cx = tid & 15;    // outputs: rows 8 ry + i, columns 4 cx.. and 64 + 4 cx..
+  const int tile_no = item / p.bh, bh = item - tile_no * p.bh;   // causal: the longest tiles of all heads first
+  const int tiles = ((kQStat ? p.n_q : p.n_k) + OM - 1) / OM;
+  const int m0 = (kQStat ? tiles - 1 - tile_no : tile_no) * OM;
   const size_t qoff = static_cast<size_t>(bh) * p.n_q * d, qoff_v = static_cast<size_t>(bh) * p.n_q * dv;
   const size_t koff = static_cast<size_t>(bh) * p.n_k * d, koff_v = static_cast<size_t>(bh) * p.n_k * dv;
-  const size_t voff = static_cast<size_t>(bh) * row_stride(p.n_q);  // row-vector offset
-  const int causal_off = p.n_k - p.n_q;
-  const int n_stat = kQStationary ? p.n_q : p.n_k;
-  const int n_strm = kQStationary ? p.n_k : p.n_q;
+  const size_t voff = static_cast<size_t>(bh) * row_stride(p.n_q);
+  const int off = p.n_k - p.n_q;
+  const int n_stat = kQStat ? p.n_q : p.n_k, n_strm = kQStat ? p.n_k : p.n_q;
 
-  if (kQStationary) {
-    load_tile<T>(stat[0], ld, p.q, qoff, m0, TM, p.n_q, d);
-    load_tile<T>(stat[1], ld, p.ddq, qoff, m0, TM, p.n_q, d);
-    if (PASS >= 2) load_tile<T>(stat[2], ld, p.d_o, qoff_v, m0, TM, p.n_q, dv);
-  } else {
-    load_tile<T>(stat[0], ld, p.k, koff, m0, TM, p.n_k, d);
-    load_tile<T>(stat[1], ld, p.ddk, koff, m0, TM, p.n_k, d);
-    load_tile<T>(stat[2], ld, p.v, koff_v, m0, TM, p.n_k, dv);
-    load_tile<T>(stat[3], ld, p.ddv, koff_v, m0, TM, p.n_k, dv);
-  }
+  // operands of the (q/k, v) head dims on either side
+  const void *q_in[4] = {p.q, p.ddq, p.d_o, nullptr}, *k_in[4] = {p.k, p.ddk, p.v, p.ddv};
+  auto load_side = [&](float* const (&dst)[4], bool q_side, int row0, int rows) {
+    const int n = q_side ? p.n_q : p.n_k;
+    const size_t o = q_side ? qoff : koff, o_v = q_side ? qoff_v : koff_v;
+    const void* const* in = q_side ? q_in : k_in;
+    load_rows<T>(dst[0], in[0], o, row0, rows, n, d);
+    if (!kFirst) load_rows<T>(dst[1], in[1], o, row0, rows, n, d);
+    load_rows<T>(dst[2], in[2], o_v, row0, rows, n, dv);
+    if (!kFirst && !q_side) load_rows<T>(dst[3], in[3], o_v, row0, rows, n, dv);
+  };
+  load_side(stat, kQStat, m0, OM);
 
-  // per-row constants of the stationary queries (passes 1-3)
-  float r_nlc[RPW], r_k1[RPW], r_nds[RPW], r_ndd[RPW], r_nbs[RPW], rowacc[RPW];
+  float r_nlc[4], r_ndd[4], r_k1[4], r_k23[4];   // constants of the thread's stationary queries
 #pragma unroll
-  for (int i = 0; i < RPW; ++i) {
-    int qi = m0 + warp * RPW + i;
-    bool ok = kQStationary && qi < p.n_q;
+  for (int i = 0; i < 4; ++i) {
+    const int qi = m0 + 4 * ty + i;
+    const bool ok = kQStat && qi < p.n_q;
     r_nlc[i] = ok ? p.nlc[voff + qi] : 0.f;
-    const float k1 = ok && PASS >= 2 ? p.k1[voff + qi] : 0.f;
-    r_k1[i] = k1;
-    r_nds[i] = k1 * p.scale;                                                    // -D*scale
-    r_ndd[i] = ok && PASS >= 2 ? p.ndd[voff + qi] : 0.f;
-    r_nbs[i] = ok && PASS >= 3 ? (p.k23[voff + qi] + k1 * r_ndd[i]) * p.scale : 0.f;  // -b*scale
-    rowacc[i] = 0.f;
+    r_k1[i] = ok ? p.k1[voff + qi] : 0.f;
+    r_ndd[i] = ok && MODE == 3 ? p.ndd[voff + qi] : 0.f;
+    r_k23[i] = ok && MODE == 3 ? p.k23[voff + qi] : 0.f;
   }
-  float out0[RPW][DCH], out1[RPW][DCH];
+  float rowacc[4] = {0.f, 0.f, 0.f, 0.f};   // sweep
+  float2 out[8][4];
 #pragma unroll
-  for (int i = 0; i < RPW; ++i)
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int m = 0; m < DCH; ++m) out0[i][m] = out1[i][m] = 0.f;
+    for (int j = 0; j < 4; ++j) out[i][j] = make_float2(0.f, 0.f);
 
-  // streamed range
   int t_begin, t_end;
-  visible_tiles(kQStationary, m0, TM, TN, n_strm, causal_off, p.causal, p.window, t_begin, t_end);
+  visible_tiles(kQStat, m0, OM, ON, n_strm, off, p.causal, p.window, t_begin, t_end);
   const float sl2 = p.scale * kLog2e;
 
   for (int t = t_begin; t < t_end; ++t) {
-    const int n0 = t * TN;
-    __syncthreads();  // previous step finished with strm/ptile
-    if (kQStationary) {
-      load_tile<T>(strm[0], ld, p.k, koff, n0, TN, p.n_k, d);
-      load_tile<T>(strm[1], ld, p.ddk, koff, n0, TN, p.n_k, d);
-      if (PASS >= 2) {
-        load_tile<T>(strm[2], ld, p.v, koff_v, n0, TN, p.n_k, dv);
-        load_tile<T>(strm[3], ld, p.ddv, koff_v, n0, TN, p.n_k, dv);
-      }
-    } else {
-      load_tile<T>(strm[0], ld, p.q, qoff, n0, TN, p.n_q, d);
-      load_tile<T>(strm[1], ld, p.ddq, qoff, n0, TN, p.n_q, d);
-      load_tile<T>(strm[2], ld, p.d_o, qoff_v, n0, TN, p.n_q, dv);
-      if (threadIdx.x < TN) {
-        int qi = n0 + threadIdx.x;
-        bool ok = qi < p.n_q;
-        svec[0 * TN + threadIdx.x] = ok ? p.nlc[voff + qi] : 0.f;
-        const float k1 = ok ? p.k1[voff + qi] : 0.f, ndd = ok ? p.ndd[voff + qi] : 0.f;
-        svec[1 * TN + threadIdx.x] = k1 * p.scale;
-        svec[2 * TN + threadIdx.x] = ndd;
-        svec[3 * TN + threadIdx.x] = ok ? (p.k23[voff + qi] + k1 * ndd) * p.scale : 0.f;
+    const int n0 = t * ON;
+    __syncthreads();   // the previous step has read its tiles
+    load_side(strm, !kQStat, n0, ON);
+    if (!kQStat && threadIdx.x < ON) {
+      const int qi = n0 + threadIdx.x;
+      const bool ok = qi < p.n_q;
+      svec[threadIdx.x] = ok ? p.nlc[voff + qi] : 0.f;
+      svec[2 * ON + threadIdx.x] = ok ? p.k1[voff + qi] : 0.f;
+      if (!kFirst) {
+        svec[ON + threadIdx.x] = ok ? p.ndd[voff + qi] : 0.f;
+        svec[3 * ON + threadIdx.x] = ok ? p.k23[voff + qi] : 0.f;
       }
     }
+    loads_landed();
     __syncthreads();
 
-    // score-shaped tiles: rows = stationary, columns = streamed; this thread: RPW rows x column `lane`
-    float s[RPW], a2[RPW], dp[RPW], x[RPW];
-#pragma unroll
-    for (int i = 0; i < RPW; ++i) s[i] = a2[i] = dp[i] = x[i] = 0.f;
-    for (int e = 0; e < d; ++e) {   // contractions over the q/k head dim
-      float c0 = strm[0][lane * ld + e], c1 = strm[1][lane * ld + e];
-#pragma unroll
-      for (int i = 0; i < RPW; ++i) {
-        int r = warp * RPW + i;
-        float a0 = stat[0][r * ld + e], a1 = stat[1][r * ld + e];
-        s[i] = fmaf(a0, c0, s[i]);
-        a2[i] = fmaf(a1, c0, fmaf(a0, c1, a2[i]));
-      }
+    // does any pair of this tile need masking?  (uniform over the CTA)
+    bool masked = n0 + ON > n_strm;
+    if (p.causal) {
+      if (kQStat) masked = masked || n0 + ON - 1 > m0 + off || (p.window > 0 && m0 + OM - 1 + off - n0 >= p.window);
+      else masked = masked || n0 + off < m0 + OM - 1 || (p.window > 0 && n0 + ON - 1 + off - m0 >= p.window);
     }
-    if (PASS >= 2) {
-      for (int e = 0; e < dv; ++e) {   // contractions over the v head dim
-        float c2 = strm[2][lane * ld + e];
-        float c3 = kQStationary ? strm[3][lane * ld + e] : 0.f;
-#pragma unroll
-        for (int i = 0; i < RPW; ++i) {
-          int r = warp * RPW + i;
-          float a2v = stat[2][r * ld + e];
-          dp[i] = fmaf(a2v, c2, dp[i]);
-          if (kQStationary) x[i] = fmaf(a2v, c3, x[i]);
-          else x[i] = fmaf(stat[3][r * ld + e], c2, x[i]);
-        }
-      }
-    }
+    auto allowed = [&](int i, int j) {
+      if (!masked) return true;
+      const int r = m0 + 4 * ty + i, c = n0 + tx + 8 * j;
+      return c < n_strm && pair_visible(kQStat ? r : c, kQStat ? c : r, off, p.causal, p.window);
+    };
 
-    // elementwise
+    float2 u0[4][4], u1[4][4];   // group 0: S, A2; group 1: dP, X
 #pragma unroll
-    for (int i = 0; i < RPW; ++i) {
-      int r = warp * RPW + i;
-      int qi = kQStationary ? m0 + r : n0 + lane;
-      int kj = kQStationary ? n0 + lane : m0 + r;
-      bool allowed = qi < p.n_q && kj < p.n_k && pair_visible(qi, kj, causal_off, p.causal, p.window);
-      float nlc, nds, ndd, nbs;
-      if (kQStationary) { nlc = r_nlc[i]; nds = r_nds[i]; ndd = r_ndd[i]; nbs = r_nbs[i]; }
-      else { nlc = svec[lane]; nds = svec[TN + lane]; ndd = svec[2 * TN + lane]; nbs = svec[3 * TN + lane]; }
-      float pr = allowed ? exp2f(fmaf(s[i], sl2, nlc)) : 0.f;
-      if (PASS == 1) {
-        rowacc[i] = fmaf(pr, a2[i], rowacc[i]);
-      } else {
-        float tt = fmaf(a2[i], p.scale, ndd);
-        float u = fmaf(dp[i], tt, x[i]);
-        u = fmaf(nds, a2[i], u);
-        if (PASS == 2) {
-          rowacc[i] = fmaf(pr, u, rowacc[i]);
-        } else {
-          ptile[(0 * TM + r) * LT + lane] = pr * fmaf(dp[i], p.scale, nds);  // dS
-          ptile[(1 * TM + r) * LT + lane] = pr * fmaf(u, p.scale, nbs);      // dS2
-          ptile[(2 * TM + r) * LT + lane] = pr * tt;                          // ddP
-          ptile[(3 * TM + r) * LT + lane] = pr;                               // P
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) u0[i][j] = u1[i][j] = make_float2(0.f, 0.f);
+    if (group == 0) {
+      const float *sa = stat[0] + 4 * ty * OP, *sb = stat[1] + 4 * ty * OP, *ca = strm[0] + tx * OP, *cb = strm[1] + tx * OP;
+#pragma unroll 2
+      for (int e = 0; e < d; e += 4) {
+        float4 k[4], kk[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          k[j] = ld4(ca + 8 * j * OP + e);
+          if (!kFirst) kk[j] = ld4(cb + 8 * j * OP + e);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 q = ld4(sa + i * OP + e);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dot4(u0[i][j], q, k[j]);
+          if (!kFirst) {
+            const float4 qq = ld4(sb + i * OP + e);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              dot4(u1[i][j], q, kk[j]);
+              dot4(u1[i][j], qq, k[j]);
+            }
+          }
         }
       }
-    }
-
-    if (PASS >= 3) {
-      __syncwarp();  // a warp only reads the ptile rows it wrote itself
-      // PASS 3: out0 = dQ2 += dS ddK + dS2 K ;  out1 = ddO += ddP V + P ddV
-      // PASS 4: out0 = dK2 += dS ddQ + dS2 Q ;  out1 = dV2 += ddP dO
-      const float* b_ds = kQStationary ? strm[1] : strm[1];   // ddK | ddQ
-      const float* b_ds2 = kQStationary ? strm[0] : strm[0];  // K   | Q
-      const float* b_ddp = kQStationary ? strm[2] : strm[2];  // V   | dO
-      for (int c = 0; c < TN; ++c) {
-        float bds[DCH], bds2[DCH], bddp[DCH], bp[DCH];
 #pragma unroll
-        for (int m = 0; m < DCH; ++m) {
-          int col = lane + 32 * m;
-          bool in = col < d, in_v = col < dv;
-          bds[m] = in ? b_ds[c * ld + col] : 0.f;
-          bds2[m] = in ? b_ds2[c * ld + col] : 0.f;
-          bddp[m] = in_v ? b_ddp[c * ld + col] : 0.f;
-          bp[m] = (in_v && kQStationary) ? strm[3][c * ld + col] : 0.f;
+      for (int j = 0; j < 4; ++j) {
+        const int c = tx + 8 * j;
+        float pr[4], tt[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const bool ok = allowed(i, j);
+          const float s = u0[i][j].x + u0[i][j].y, a2 = u1[i][j].x + u1[i][j].y;
+          pr[i] = ok ? exp2f(fmaf(s, sl2, kQStat ? r_nlc[i] : svec[c])) : 0.f;
+          if (MODE == 2) {
+            tt[i] = ok ? a2 * p.scale : 0.f;
+            rowacc[i] = fmaf(pr[i], tt[i], rowacc[i]);
+          } else if (!kFirst) {
+            tt[i] = ok ? fmaf(a2, p.scale, kQStat ? r_ndd[i] : svec[ON + c]) : 0.f;
+          }
+        }
+        const int at = c * PP + 4 * ty;
+        *reinterpret_cast<float4*>(p_tile + at) = make_float4(pr[0], pr[1], pr[2], pr[3]);
+        if (!kFirst) *reinterpret_cast<float4*>(pt[0] + at) = make_float4(tt[0], tt[1], tt[2], tt[3]);
+        if (MODE == 3 || MODE == 4)
+          *reinterpret_cast<float4*>(pt[2] + at) = make_float4(pr[0] * tt[0], pr[1] * tt[1], pr[2] * tt[2], pr[3] * tt[3]);
+      }
+    } else {
+      const float *sa = stat[2] + 4 * ty * OP, *sb = stat[3] + 4 * ty * OP, *ca = strm[2] + tx * OP, *cb = strm[3] + tx * OP;
+#pragma unroll 2
+      for (int e = 0; e < dv; e += 4) {
+        float4 v[4], vv[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          v[j] = ld4(ca + 8 * j * OP + e);
+          if (C::kBoth2) vv[j] = ld4(cb + 8 * j * OP + e);
         }
 #pragma unroll
-        for (int i = 0; i < RPW; ++i) {
-          int r = warp * RPW + i;
-          float vds = ptile[(0 * TM + r) * LT + c], vds2 = ptile[(1 * TM + r) * LT + c];
-          float vddp = ptile[(2 * TM + r) * LT + c], vp = ptile[(3 * TM + r) * LT + c];
+        for (int i = 0; i < 4; ++i) {
+          const float4 g = ld4(sa + i * OP + e);
 #pragma unroll
-          for (int m = 0; m < DCH; ++m) {
-            out0[i][m] = fmaf(vds, bds[m], fmaf(vds2, bds2[m], out0[i][m]));
-            out1[i][m] = fmaf(vddp, bddp[m], out1[i][m]);
-            if (kQStationary) out1[i][m] = fmaf(vp, bp[m], out1[i][m]);
+          for (int j = 0; j < 4; ++j) {
+            dot4(u0[i][j], g, v[j]);
+            if (C::kBoth2) dot4(u1[i][j], g, vv[j]);
+          }
+          if (MODE == 4) {
+            const float4 gg = ld4(sb + i * OP + e);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dot4(u1[i][j], gg, v[j]);
           }
         }
       }
     }
+    __syncthreads();   // P and t are there
+    if (group == 1) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int c = tx + 8 * j, at = c * PP + 4 * ty;
+        const float4 p4 = ld4(p_tile + at);
+        float4 t4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!kFirst) t4 = ld4(pt[0] + at);
+        const float pr[4] = {p4.x, p4.y, p4.z, p4.w}, tt[4] = {t4.x, t4.y, t4.z, t4.w};
+        float ds[4], ds2[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const bool ok = allowed(i, j);
+          const float dpp = u0[i][j].x + u0[i][j].y + (kQStat ? r_k1[i] : svec[2 * ON + c]);
+          const float x = u1[i][j].x + u1[i][j].y;
+          if (MODE == 2) {
+            if (ok) rowacc[i] = fmaf(pr[i], fmaf(dpp, tt[i], x), rowacc[i]);
+          } else {
+            ds[i] = ok ? pr[i] * dpp : 0.f;
+            if (!kFirst) ds2[i] = ok ? pr[i] * fmaf(dpp, tt[i], x + (kQStat ? r_k23[i] : svec[3 * ON + c])) : 0.f;
+          }
+        }
+        if (MODE != 2) *reinterpret_cast<float4*>(pt[0] + at) = make_float4(ds[0], ds[1], ds[2], ds[3]);
+        if (MODE == 3 || MODE == 4) *reinterpret_cast<float4*>(pt[1] + at) = make_float4(ds2[0], ds2[1], ds2[2], ds2[3]);
+      }
+    }
+    if constexpr (MODE == 3 || MODE == 4) {
+      __syncthreads();   // dS and dS2 are there
+      const int ro = 8 * ry, co = 4 * cx;
+      if (group == 0) {   // dS . ddK | ddQ + dS2 . K | Q
+        if (d > 64) outer<true, true>(out, pt[0] + ro, strm[1] + co, pt[1] + ro, strm[0] + co);
+        else outer<true, false>(out, pt[0] + ro, strm[1] + co, pt[1] + ro, strm[0] + co);
+      } else {            // ddP . V | dO (+ P . ddV)
+        if (dv > 64) outer<MODE == 3, true>(out, pt[2] + ro, strm[2] + co, pt[3] + ro, strm[3] + co);
+        else outer<MODE == 3, false>(out, pt[2] + ro, strm[2] + co, pt[3] + ro, strm[3] + co);
+      }
+    } else if constexpr (kFirst) {
+      __syncthreads();
+      const int ro = 8 * ry, co = 4 * cx;
+      if constexpr (MODE == 5) {   // dS . K, 64 columns a group
+        if (64 * group < d) outer<false, false>(out, pt[0] + ro, strm[0] + 64 * group + co, nullptr, nullptr);
+      } else if (group == 0) {     // dS . Q
+        if (d > 64) outer<false, true>(out, pt[0] + ro, strm[0] + co, nullptr, nullptr);
+        else outer<false, false>(out, pt[0] + ro, strm[0] + co, nullptr, nullptr);
+      } else {                     // P . dO
+        if (dv > 64) outer<false, true>(out, pt[1] + ro, strm[2] + co, nullptr, nullptr);
+        else outer<false, false>(out, pt[1] + ro, strm[2] + co, nullptr, nullptr);
+      }
+    }
   }
 
+  loads_landed();   // a tile without visible pairs has not waited yet
+
   // results
-  if (PASS <= 2) {
+  if (MODE == 2) {
 #pragma unroll
-    for (int i = 0; i < RPW; ++i) {
-      float tot = warp_sum(rowacc[i]);
-      int qi = m0 + warp * RPW + i;
-      if (lane == 0 && qi < p.n_q) {
-        if (PASS == 1) p.ndd[voff + qi] = -p.scale * tot;          // -dd, dd = scale * sum P A2
-        else p.k23[voff + qi] = -r_k1[i] * r_ndd[i] - tot;          // -D*dd - b, b = sum P dP2
-      }
+    for (int i = 0; i < 4; ++i) {
+      float tot = rowacc[i];
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+      const int qi = m0 + 4 * ty + i;
+      if (tx == 0 && qi < p.n_q) (group == 0 ? p.ndd : p.k23)[voff + qi] = -tot;
     }
   } else {
-    void* o0 = kQStationary ? p.dq2 : p.dk2;
-    void* o1 = kQStationary ? p.ddo : p.dv2;
-    size_t off = kQStationary ? qoff : koff, off_v = kQStationary ? qoff_v : koff_v;
+    const bool first = group == 0 || MODE == 5;
+    void* base = first ? (MODE == 3 || MODE == 5 ? p.dq2 : p.dk2) : (MODE == 3 ? p.ddo : p.dv2);
+    const int cols = first ? d : dv, col = 4 * cx + (MODE == 5 ? 64 * group : 0);
+    const size_t head = first ? (kQStat ? qoff : koff) : (kQStat ? qoff_v : koff_v);
+    const float mul = first ? p.scale : 1.f;   // dS and dS2 carry no factor `scale`
 #pragma unroll
-    for (int i = 0; i < RPW; ++i) {
-      int gr = m0 + warp * RPW + i;
-      if (gr >= n_stat) continue;
-#pragma unroll
-      for (int m = 0; m < DCH; ++m) {
-        int col = lane + 32 * m;
-        if (col < d) st_elem<T>(o0, off + static_cast<size_t>(gr) * d + col, out0[i][m]);
-        if (col < dv) st_elem<T>(o1, off_v + static_cast<size_t>(gr) * dv + col, out1[i][m]);
-      }
+    for (int i = 0; i < 8; ++i) {
+      const int r = m0 + 8 * ry + i;
+      if (r >= n_stat) continue;
+      const size_t at = head + static_cast<size_t>(r) * cols + col;
+      if (col < cols) store4<T>(base, at, out[i][0], out[i][1], mul);
+      if (MODE != 5 && col + 64 < cols) store4<T>(base, at + 64, out[i][2], out[i][3], mul);
     }
   }
+}
+
+// MODE_Q on the first q_blocks CTAs, MODE_K (if not 0) on the others
+template <typename T, int MODE_Q, int MODE_K>
+__global__ void __launch_bounds__(NT, 1) simt_pass_kernel(const __grid_constant__ SimtParams p, int q_blocks) {
+  const int block = blockIdx.x;
+  if (block < q_blocks) simt_body<T, MODE_Q>(p, block);
+  else if constexpr (MODE_K != 0) simt_body<T, MODE_K>(p, block - q_blocks);
 }
 
 // O(N)-memory forward: online softmax over key tiles.
@@ -389,135 +553,9 @@ __global__ void __launch_bounds__(NT) simt_forward_kernel(const SimtParams p, vo
   }
 }
 
-// First backward (dQ | dK, dV) of attention from the saved forward results, O(N) memory.
-// KSIDE = false: a CTA owns TM queries and streams keys:   dQ = scale * (P (dP - D)) K.
-// KSIDE = true:  a CTA owns TM keys and streams queries:   dV = P^T dO,  dK = scale * (P (dP - D))^T Q.
-// Reads nlc = -L*log2(e) and k1 = -D from the workspace (written by the pre-pass).
-template <typename T, bool KSIDE>
-__global__ void __launch_bounds__(NT) simt_backward_kernel(const SimtParams p, void* out0, void* out1) {
-  extern __shared__ float smem[];
-  const int d = p.d, dv = p.dv, ld = (d > dv ? d : dv) + 1;
-  float* stat0 = smem;                       // Q | K
-  float* stat1 = stat0 + TM * ld;            // dO | V
-  float* strm0 = stat1 + TM * ld;            // K | Q
-  float* strm1 = strm0 + TN * ld;            // V | dO
-  float* pt = strm1 + TN * ld;               // [2][TM][TN+1]: P and dS tiles
-  float* svec = pt + 2 * TM * (TN + 1);      // [2][TN]: nlc, k1 of streamed queries (KSIDE)
-  constexpr int LT = TN + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * TM, bh = blockIdx.y + blockIdx.z * kMaxGridY;   // see head_grid
-  if (bh >= p.bh) return;
-  const size_t qoff = static_cast<size_t>(bh) * p.n_q * d, qoff_v = static_cast<size_t>(bh) * p.n_q * dv;
-  const size_t koff = static_cast<size_t>(bh) * p.n_k * d, koff_v = static_cast<size_t>(bh) * p.n_k * dv;
-  const size_t voff = static_cast<size_t>(bh) * row_stride(p.n_q);
-  const int causal_off = p.n_k - p.n_q;
-  const int n_stat = KSIDE ? p.n_k : p.n_q, n_strm = KSIDE ? p.n_q : p.n_k;
-  if (KSIDE) {
-    load_tile<T>(stat0, ld, p.k, koff, m0, TM, p.n_k, d);
-    load_tile<T>(stat1, ld, p.v, koff_v, m0, TM, p.n_k, dv);
-  } else {
-    load_tile<T>(stat0, ld, p.q, qoff, m0, TM, p.n_q, d);
-    load_tile<T>(stat1, ld, p.d_o, qoff_v, m0, TM, p.n_q, dv);
-  }
-  float r_nlc[RPW], r_k1[RPW];
-#pragma unroll
-  for (int i = 0; i < RPW; ++i) {
-    const int qi = m0 + warp * RPW + i;
-    const bool ok = !KSIDE && qi < p.n_q;
-    r_nlc[i] = ok ? p.nlc[voff + qi] : 0.f;
-    r_k1[i] = ok ? p.k1[voff + qi] : 0.f;
-  }
-  float acc0[RPW][DCH], acc1[RPW][DCH];
-#pragma unroll
-  for (int i = 0; i < RPW; ++i)
-#pragma unroll
-    for (int m = 0; m < DCH; ++m) acc0[i][m] = acc1[i][m] = 0.f;
-  int t_begin, t_end;
-  visible_tiles(!KSIDE, m0, TM, TN, n_strm, causal_off, p.causal, p.window, t_begin, t_end);
-  const float sl2 = p.scale * kLog2e;
-  for (int t = t_begin; t < t_end; ++t) {
-    const int n0 = t * TN;
-    __syncthreads();
-    if (KSIDE) {
-      load_tile<T>(strm0, ld, p.q, qoff, n0, TN, p.n_q, d);
-      load_tile<T>(strm1, ld, p.d_o, qoff_v, n0, TN, p.n_q, dv);
-      if (threadIdx.x < TN) {
-        const int qi = n0 + threadIdx.x;
-        svec[threadIdx.x] = qi < p.n_q ? p.nlc[voff + qi] : 0.f;
-        svec[TN + threadIdx.x] = qi < p.n_q ? p.k1[voff + qi] : 0.f;
-      }
-    } else {
-      load_tile<T>(strm0, ld, p.k, koff, n0, TN, p.n_k, d);
-      load_tile<T>(strm1, ld, p.v, koff_v, n0, TN, p.n_k, dv);
-    }
-    __syncthreads();
-    float s[RPW], dp[RPW];
-#pragma unroll
-    for (int i = 0; i < RPW; ++i) s[i] = dp[i] = 0.f;
-    for (int e = 0; e < d; ++e) {
-      const float c0 = strm0[lane * ld + e];
-#pragma unroll
-      for (int i = 0; i < RPW; ++i) s[i] = fmaf(stat0[(warp * RPW + i) * ld + e], c0, s[i]);
-    }
-    for (int e = 0; e < dv; ++e) {
-      const float c1 = strm1[lane * ld + e];
-#pragma unroll
-      for (int i = 0; i < RPW; ++i) dp[i] = fmaf(stat1[(warp * RPW + i) * ld + e], c1, dp[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < RPW; ++i) {
-      const int r = warp * RPW + i;
-      const int qi = KSIDE ? n0 + lane : m0 + r, kj = KSIDE ? m0 + r : n0 + lane;
-      const bool allowed = qi < p.n_q && kj < p.n_k && pair_visible(qi, kj, causal_off, p.causal, p.window);
-      const float nlc = KSIDE ? svec[lane] : r_nlc[i], k1 = KSIDE ? svec[TN + lane] : r_k1[i];
-      const float pr = allowed ? exp2f(fmaf(s[i], sl2, nlc)) : 0.f;
-      pt[(0 * TM + r) * LT + lane] = pr;
-      pt[(1 * TM + r) * LT + lane] = allowed ? pr * (dp[i] + k1) * p.scale : 0.f;  // dS
-    }
-    __syncwarp();
-    for (int c = 0; c < TN; ++c) {
-      float b0[DCH], b1[DCH];
-#pragma unroll
-      for (int m = 0; m < DCH; ++m) {
-        const int col = lane + 32 * m;
-        b0[m] = col < d ? strm0[c * ld + col] : 0.f;    // K | Q
-        b1[m] = col < dv ? strm1[c * ld + col] : 0.f;   // V | dO
-      }
-#pragma unroll
-      for (int i = 0; i < RPW; ++i) {
-        const int r = warp * RPW + i;
-        const float vp = pt[(0 * TM + r) * LT + c], vds = pt[(1 * TM + r) * LT + c];
-#pragma unroll
-        for (int m = 0; m < DCH; ++m) {
-          acc0[i][m] = fmaf(vds, b0[m], acc0[i][m]);              // dQ += dS K   | dK += dS^T Q
-          if (KSIDE) acc1[i][m] = fmaf(vp, b1[m], acc1[i][m]);    //              | dV += P^T dO
-        }
-      }
-    }
-  }
-  const size_t off = KSIDE ? koff : qoff;
-#pragma unroll
-  for (int i = 0; i < RPW; ++i) {
-    const int gr = m0 + warp * RPW + i;
-    if (gr >= n_stat) continue;
-#pragma unroll
-    for (int m = 0; m < DCH; ++m) {
-      const int col = lane + 32 * m;
-      if (col < d) st_elem<T>(out0, off + static_cast<size_t>(gr) * d + col, acc0[i][m]);
-      if (KSIDE && col < dv) st_elem<T>(out1, koff_v + static_cast<size_t>(gr) * dv + col, acc1[i][m]);
-    }
-  }
-}
-
-
 int pitch(const FhobProblem& p) {  // row pitch of the shared-memory tiles: the larger head dim + 1
   const int dv = head_dim_v(p);
   return (p.d > dv ? p.d : dv) + 1;
-}
-
-size_t pass_smem_bytes(const FhobProblem& p) {
-  size_t ld = pitch(p);
-  return sizeof(float) * ((4 * TM + 4 * TN) * ld + 8 * TM * (TN + 1) + 4 * TN);
 }
 
 SimtParams make_params(const FhobProblem& p) {
@@ -530,42 +568,39 @@ SimtParams make_params(const FhobProblem& p) {
   return s;
 }
 
-template <typename T, int PASS>
-int launch_pass(const FhobProblem& p, cudaStream_t st) {
-  size_t smem = pass_smem_bytes(p);
-  FHOB_CUDA_OK(cudaFuncSetAttribute(simt_pass_kernel<T, PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(smem)));
-  int n_stat = PASS == 4 ? p.n_k : p.n_q;
-  dim3 grid = head_grid((n_stat + TM - 1) / TM, p.bh);
-  simt_pass_kernel<T, PASS><<<grid, NT, smem, st>>>(make_params(p));
+template <typename T, int MODE_Q, int MODE_K>
+int launch_modes(const SimtParams& p, bool q_side, bool k_side, cudaStream_t st) {
+  constexpr auto kernel = simt_pass_kernel<T, MODE_Q, MODE_K>;
+  constexpr int kQ = Tiles<MODE_Q>::SMEM_BYTES, kK = Tiles<MODE_K ? MODE_K : MODE_Q>::SMEM_BYTES, kSmem = kQ > kK ? kQ : kK;
+  FHOB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  const long long items_q = q_side ? static_cast<long long>((p.n_q + OM - 1) / OM) * p.bh : 0;
+  const long long items_k = k_side ? static_cast<long long>((p.n_k + OM - 1) / OM) * p.bh : 0;
+  if (items_q + items_k > 0x7fffffffLL) return FHOB_ERR_SHAPE;
+  kernel<<<static_cast<unsigned>(items_q + items_k), NT, kSmem, st>>>(p, static_cast<int>(items_q));
   FHOB_CUDA_OK(cudaGetLastError());
   return FHOB_OK;
 }
 
+// `pass` as in the entry points; passes 1 and 2 are one sweep, whichever is asked for
 template <typename T>
 int dispatch_pass(int pass, const FhobProblem& p, cudaStream_t st) {
+  const SimtParams s = make_params(p);
   switch (pass) {
-    case 1: return launch_pass<T, 1>(p, st);
-    case 2: return launch_pass<T, 2>(p, st);
-    case 3: return launch_pass<T, 3>(p, st);
-    case 4: return launch_pass<T, 4>(p, st);
+    case 1:
+    case 2:
+    case 12: return launch_modes<T, 2, 0>(s, true, false, st);
+    case 3: return launch_modes<T, 3, 4>(s, true, false, st);
+    case 4: return launch_modes<T, 3, 4>(s, false, true, st);
+    case 34: return launch_modes<T, 3, 4>(s, true, true, st);
   }
   return FHOB_ERR_ARG;
 }
 
 template <typename T>
 int launch_backward(const FhobProblem& p, void* dq, void* dk, void* dv, cudaStream_t st) {
-  const size_t smem = sizeof(float) * ((2 * TM + 2 * TN) * pitch(p) + 2 * TM * (TN + 1) + 2 * TN);
   SimtParams s = make_params(p);
-  FHOB_CUDA_OK(cudaFuncSetAttribute(simt_backward_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(smem)));
-  FHOB_CUDA_OK(cudaFuncSetAttribute(simt_backward_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(smem)));
-  simt_backward_kernel<T, false><<<head_grid((p.n_q + TM - 1) / TM, p.bh), NT, smem, st>>>(s, dq, nullptr);
-  FHOB_CUDA_OK(cudaGetLastError());
-  simt_backward_kernel<T, true><<<head_grid((p.n_k + TM - 1) / TM, p.bh), NT, smem, st>>>(s, dk, dv);
-  FHOB_CUDA_OK(cudaGetLastError());
-  return FHOB_OK;
+  s.dq2 = dq; s.dk2 = dk; s.dv2 = dv;
+  return launch_modes<T, 5, 6>(s, true, true, st);
 }
 
 }  // namespace

@@ -1,0 +1,68 @@
+"""CUDA-core operator and first backward at the edges of their 64 x 32 tiles and 64-column halves."""
+from __future__ import annotations
+
+import math
+
+import pytest
+import torch
+
+from oracle import attn_oracle as O
+
+# n_q, n_k, d, d_v, causal, window
+EDGES = [(1, 1, 4, 4, False, None), (64, 32, 64, 68, False, None), (65, 33, 68, 64, False, None), (63, 31, 128, 4, False, None),
+         (64, 128, 60, 128, True, None), (97, 161, 124, 128, True, None), (130, 130, 128, 128, True, 33), (96, 200, 72, 80, True, 64),
+         (64, 1500, 128, 128, False, None), (700, 40, 96, 96, False, None)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bh", (1, 3))
+@pytest.mark.parametrize("nq,nk,d,dv,causal,window", EDGES)
+def test_edges_match_oracle(bh, nq, nk, d, dv, causal, window):
+    import fhob
+    g = torch.Generator().manual_seed(nq * 7 + nk)
+    mk = lambda n, e: torch.randn(bh, n, e, generator=g)
+    x = dict(q=mk(nq, d), k=mk(nk, d), v=mk(nk, dv), do=mk(nq, dv), ddq=mk(nq, d), ddk=mk(nk, d), ddv=mk(nk, dv))
+    x64 = {n: t.double() for n, t in x.items()}
+    w = math.inf if window is None else window
+    scale = d ** -0.5
+    ref2 = O.bwdbwd_closed_form(*x64.values(), scale, causal, sliding_window_length=w)
+    ref1 = O.attn_bwd(x64["q"], x64["k"], x64["v"], x64["do"], scale, causal, sliding_window_length=w)
+    dev = {n: t.cuda() for n, t in x.items()}
+    kw = dict(is_causal=causal, sliding_window=window, impl="simt")
+    o, lse = fhob.attention_forward(dev["q"], dev["k"], dev["v"], scale, **kw)
+    args = (dev["q"], dev["k"], dev["v"], o, dev["do"], dev["ddq"], dev["ddk"], dev["ddv"], lse, scale)
+    got2 = fhob.flash_bwdbwd(*args, **kw)
+    got1 = fhob.attention_backward(*args[:5], lse, scale, **kw)
+    # chains of n + 2 d fp32 multiply-adds, 2^-24 each, as a random walk: sqrt(1756) * 2^-24 = 2.5e-6 of a
+    # typical entry; the differences dP - D and X + k23 lose at most three bits of that (1 key: exact zeros)
+    for n, a, r in zip(("dq", "dk", "dv", "dq2", "dk2", "dv2", "ddo"), got1 + got2, tuple(ref1) + tuple(ref2)):
+        err = float((a.double().cpu() - r).abs().max()) / max(float(r.abs().max()), 0.1)
+        assert err < 2e-5, (n, err)
+    again = fhob.flash_bwdbwd(*args, **kw)
+    assert all(torch.equal(a, b) for a, b in zip(got2, again))   # one order of sums
+
+
+@pytest.mark.gpu
+def test_single_passes_give_the_operator():
+    """The four passes one by one, over the same workspace, leave the results of the whole operator."""
+    import ctypes as C
+    import fhob
+    from fhob import _lib
+    lib = _lib.load()
+    bh, nq, nk, d = 2, 70, 100, 96
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v, do, ddq, ddk, ddv = (torch.randn(bh, n, d, generator=g, device="cuda") for n in (nq, nk, nk, nq, nq, nk, nk))
+    o, lse = fhob.attention_forward(q, k, v, 0.1)
+    ref = fhob.flash_bwdbwd(q, k, v, o, do, ddq, ddk, ddv, lse, 0.1)
+    out = [torch.full_like(t, float("nan")) for t in (q, k, v, do)]
+    p = _lib.FhobProblem()
+    p.bh, p.n_q, p.n_k, p.d, p.dtype, p.scale = bh, nq, nk, d, _lib.FHOB_F32, 0.1
+    for n, t in zip(("q", "k", "v", "o", "d_o", "lse", "ddq", "ddk", "ddv", "dq2", "dk2", "dv2", "ddo"),
+                    (q, k, v, o, do, lse, ddq, ddk, ddv, *out)):
+        setattr(p, n, t.data_ptr())
+    ws = torch.zeros(lib.fhob_workspace_bytes(bh, nq), dtype=torch.uint8, device="cuda")
+    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for f in (lib.fhob_prepass, lib.fhob_pass1, lib.fhob_pass2, lib.fhob_pass3, lib.fhob_pass4):
+        assert f(C.byref(p), s) == 0
+    assert all(torch.equal(a, b) for a, b in zip(out, ref))
