@@ -11,7 +11,9 @@
 // bounds checks; pairs outside the matrix or hidden by the mask contribute zero.
 // Two head dims: Q, K, ddQ, ddK, dQ2, dK2 have `d` columns, V, ddV, dO, O, ddO, dV2
 // have `dv` (jax_refs/flash_impl.py:381-389 has d_in != d_out).
-#include "fhob_common.cuh"
+#include <type_traits>
+
+#include "tc_common.cuh"
 
 namespace fhob {
 namespace {
@@ -30,6 +32,10 @@ struct SimtParams {
   float *ndd, *k23;
   int bh, n_q, n_k, d, dv, causal, window;
   float scale;
+  int q_blocks;           // the first q_blocks CTAs are query-tiled, the others key-tiled
+  int items_q, items_k;   // (head, tile) pairs of either kind
+  int split_q, split_k;   // CTAs that share the streamed tiles of such a pair
+  int cluster;            // CTAs of a cluster (a multiple of both)
 };
 
 // Grid of (stationary tiles, heads): heads beyond what grid.y can index continue in grid.z.
@@ -209,7 +215,7 @@ __device__ __forceinline__ void store4(void* base, size_t at, const float2& a, c
 }
 
 template <typename T, int MODE>
-__device__ __forceinline__ void simt_body(const SimtParams& p, int item) {
+__device__ __forceinline__ void simt_body(const SimtParams& p, int block) {
   using C = Tiles<MODE>;
   constexpr bool kQStat = C::kQStat, kFirst = C::kFirst;
   extern __shared__ float smem[];
@@ -227,6 +233,12 @@ __device__ __forceinline__ void simt_body(const SimtParams& p, int item) {
   const int group = threadIdx.x >> 7, tid = threadIdx.x & 127;
   const int ty = tid >> 3, tx = tid & 7;     // scores: rows 4 ty + i, streamed rows tx + 8 j
   const int ry = tid >> 4, cx = tid & 15;    // outputs: rows 8 ry + i, columns 4 cx.. and 64 + 4 cx..
+  // with few items the streamed axis is split over the CTAs of a cluster
+  const int split = kQStat ? p.split_q : p.split_k;
+  int item = block / split;
+  const int begin_part = block - item * split;
+  const bool padding = item >= (kQStat ? p.items_q : p.items_k);   // the grid is padded to whole clusters
+  if (padding) item = 0;
   const int tile_no = item / p.bh, bh = item - tile_no * p.bh;   // causal: the longest tiles of all heads first
   const int tiles = ((kQStat ? p.n_q : p.n_k) + OM - 1) / OM;
   const int m0 = (kQStat ? tiles - 1 - tile_no : tile_no) * OM;
@@ -268,6 +280,8 @@ __device__ __forceinline__ void simt_body(const SimtParams& p, int item) {
 
   int t_begin, t_end;
   visible_tiles(kQStat, m0, OM, ON, n_strm, off, p.causal, p.window, t_begin, t_end);
+  if (split > 1) split_range(begin_part, split, t_begin, t_end);
+  if (padding) t_end = t_begin;
   const float sl2 = p.scale * kLog2e;
 
   for (int t = t_begin; t < t_end; ++t) {
@@ -430,7 +444,19 @@ __device__ __forceinline__ void simt_body(const SimtParams& p, int item) {
 
   loads_landed();   // a tile without visible pairs has not waited yet
 
-  // results
+  // Worked out again from the block number: kept in registers through the loop, these cost spills in it.
+  uint32_t block_again;
+  asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(block_again));
+  block_again -= kQStat ? 0 : p.q_blocks;
+  const bool live = block_again / split < static_cast<uint32_t>(kQStat ? p.items_q : p.items_k);
+  const int part = static_cast<int>(block_again % split);
+
+  // results; the parts of an item are staged in shared memory and added up in rank order
+  constexpr int kPitch = 256 + 4;   // floats per staged row: the two results
+  static_assert(4 * OM * kPitch <= C::SMEM_BYTES, "staging area");
+  if (split > 1) __syncthreads();   // every tile has been read
+  const bool first = group == 0 || MODE == 5;
+  void *base0 = MODE == 3 || MODE == 5 ? p.dq2 : p.dk2, *base1 = MODE == 3 ? p.ddo : p.dv2;
   if (MODE == 2) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -438,31 +464,59 @@ __device__ __forceinline__ void simt_body(const SimtParams& p, int item) {
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
       const int qi = m0 + 4 * ty + i;
-      if (tx == 0 && qi < p.n_q) (group == 0 ? p.ndd : p.k23)[voff + qi] = -tot;
+      if (tx != 0) continue;
+      if (split > 1) smem[group * OM + 4 * ty + i] = tot;
+      else if (live && qi < p.n_q) (group == 0 ? p.ndd : p.k23)[voff + qi] = -tot;
     }
   } else {
-    const bool first = group == 0 || MODE == 5;
-    void* base = first ? (MODE == 3 || MODE == 5 ? p.dq2 : p.dk2) : (MODE == 3 ? p.ddo : p.dv2);
     const int cols = first ? d : dv, col = 4 * cx + (MODE == 5 ? 64 * group : 0);
     const size_t head = first ? (kQStat ? qoff : koff) : (kQStat ? qoff_v : koff_v);
     const float mul = first ? p.scale : 1.f;   // dS and dS2 carry no factor `scale`
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
+      if (split > 1) {
+        const size_t at = (8 * ry + i) * kPitch + (first ? 0 : 128) + col;
+        store4<float>(smem, at, out[i][0], out[i][1], 1.f);
+        if (MODE != 5) store4<float>(smem, at + 64, out[i][2], out[i][3], 1.f);
+        continue;
+      }
       const int r = m0 + 8 * ry + i;
-      if (r >= n_stat) continue;
+      if (!live || r >= n_stat) continue;
       const size_t at = head + static_cast<size_t>(r) * cols + col;
-      if (col < cols) store4<T>(base, at, out[i][0], out[i][1], mul);
-      if (MODE != 5 && col + 64 < cols) store4<T>(base, at + 64, out[i][2], out[i][3], mul);
+      if (col < cols) store4<T>(first ? base0 : base1, at, out[i][0], out[i][1], mul);
+      if (MODE != 5 && col + 64 < cols) store4<T>(first ? base0 : base1, at + 64, out[i][2], out[i][3], mul);
     }
+  }
+  if (p.cluster > 1) {
+    cluster_sync();
+    const int rank0 = static_cast<int>(cluster_rank()) - part;
+    if (split > 1 && live) {
+      if constexpr (MODE == 2) {
+        const int row = threadIdx.x & (OM - 1), qi = m0 + row;
+        if (part == 0 && threadIdx.x < 2 * OM && qi < p.n_q) {
+          float tot = 0.f;
+          for (int i = 0; i < split; ++i) tot += cluster_ld(cluster_map(smem_u32(smem) + threadIdx.x * 4, rank0 + i));
+          (threadIdx.x < OM ? p.ndd : p.k23)[voff + qi] = -tot;
+        }
+      } else {
+        constexpr bool kF32 = sizeof(T) == 4, kF16 = std::is_same<T, __half>::value;
+        reduce_store<128, kF32, kF16, OM>(smem_u32(smem), kPitch, 0, rank0, part, split, threadIdx.x, base0, bh, m0, n_stat, d, p.scale);
+        if (MODE != 5)
+          reduce_store<128, kF32, kF16, OM>(smem_u32(smem), kPitch, 128, rank0, part, split, threadIdx.x, base1, bh, m0, n_stat, dv, 1.f);
+      }
+    }
+    cluster_sync();   // the others are done with this CTA's shared memory
   }
 }
 
 // MODE_Q on the first q_blocks CTAs, MODE_K (if not 0) on the others
 template <typename T, int MODE_Q, int MODE_K>
-__global__ void __launch_bounds__(NT, 1) simt_pass_kernel(const __grid_constant__ SimtParams p, int q_blocks) {
+__global__ void __launch_bounds__(NT, 1) simt_pass_kernel(const __grid_constant__ SimtParams p) {
+  pdl_wait();
+  if (threadIdx.x == 0) pdl_launch_dependents();
   const int block = blockIdx.x;
-  if (block < q_blocks) simt_body<T, MODE_Q>(p, block);
-  else if constexpr (MODE_K != 0) simt_body<T, MODE_K>(p, block - q_blocks);
+  if (block < p.q_blocks) simt_body<T, MODE_Q>(p, block);
+  else if constexpr (MODE_K != 0) simt_body<T, MODE_K>(p, block - p.q_blocks);
 }
 
 // O(N)-memory forward: online softmax over key tiles.
@@ -568,23 +622,50 @@ SimtParams make_params(const FhobProblem& p) {
   return s;
 }
 
+// Streamed tiles of `tile` rows that the longest item of `rows` stationary rows sees.
+inline int longest(int n, int tile, int rows, int window) {
+  const int all = (n + tile - 1) / tile;
+  const long long seen = window > 0 ? (static_cast<long long>(rows) + window - 2) / tile + 2 : all;
+  return seen < all ? static_cast<int>(seen) : all;
+}
+
+// In streamed tiles (fp32, D = 128: 12 us in passes 3 and 4): what a CTA takes besides its tiles is about one
+// tile's time, meeting in a cluster about half of one.  Operator, fp32, D = 128, us, one CTA an item ->
+// split: 1 head 64x3000 2434 -> 332, 1 causal head N=2000 1706 -> 723, 4 heads 200x5000 (d_v 64) 3435 -> 898.
+constexpr SplitCost kSimtCost = {1.f, 0.5f, 0.5f};
+
 template <typename T, int MODE_Q, int MODE_K>
-int launch_modes(const SimtParams& p, bool q_side, bool k_side, cudaStream_t st) {
+int launch_modes(SimtParams& p, bool q_side, bool k_side, cudaStream_t st) {
   constexpr auto kernel = simt_pass_kernel<T, MODE_Q, MODE_K>;
   constexpr int kQ = Tiles<MODE_Q>::SMEM_BYTES, kK = Tiles<MODE_K ? MODE_K : MODE_Q>::SMEM_BYTES, kSmem = kQ > kK ? kQ : kK;
-  FHOB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  const int ok = allow_smem(kernel, kSmem);
+  if (ok != FHOB_OK) return ok;
   const long long items_q = q_side ? static_cast<long long>((p.n_q + OM - 1) / OM) * p.bh : 0;
   const long long items_k = k_side ? static_cast<long long>((p.n_k + OM - 1) / OM) * p.bh : 0;
   if (items_q + items_k > 0x7fffffffLL) return FHOB_ERR_SHAPE;
-  kernel<<<static_cast<unsigned>(items_q + items_k), NT, kSmem, st>>>(p, static_cast<int>(items_q));
-  FHOB_CUDA_OK(cudaGetLastError());
-  return FHOB_OK;
+  const SplitWork wq = {static_cast<int>(items_q), longest(p.n_k, ON, OM, p.window)};
+  const SplitWork wk = {static_cast<int>(items_k), longest(p.n_q, ON, OM, p.window)};
+  SplitChoice c = {1, 1, true};
+  if (may_split(p.n_q, p.n_k)) c = choose_split(kernel, kSmem, wq, wk, NT, kSimtCost);
+  auto go = [&](int q, int k, int cluster) -> int {
+    auto padded = [&](long long n) { return (n + cluster - 1) / cluster * cluster; };   // whole clusters for either kind
+    p.items_q = q; p.items_k = k;
+    p.split_q = c.a; p.split_k = c.b;
+    p.cluster = cluster;
+    p.q_blocks = static_cast<int>(padded(static_cast<long long>(q) * c.a));
+    const long long blocks = p.q_blocks + padded(static_cast<long long>(k) * c.b);
+    FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(blocks), NT, kSmem, cluster, st, p));
+    return FHOB_OK;
+  };
+  if (c.together) return go(wq.items, wk.items, c.a > c.b ? c.a : c.b);
+  const int first = go(wq.items, 0, c.a);
+  return first != FHOB_OK ? first : go(0, wk.items, c.b);
 }
 
 // `pass` as in the entry points; passes 1 and 2 are one sweep, whichever is asked for
 template <typename T>
 int dispatch_pass(int pass, const FhobProblem& p, cudaStream_t st) {
-  const SimtParams s = make_params(p);
+  SimtParams s = make_params(p);
   switch (pass) {
     case 1:
     case 2:

@@ -173,15 +173,15 @@ __device__ __forceinline__ void stage_row(float* dst, uint32_t taddr, bool any) 
 
 // Adds the staged columns [c0, c0 + W) of all parts for this CTA's share of the rows, times `mul`, and stores
 // them to `base` (n_rows x d_mem per head).  `stage` = shared address of the staging area (row pitch
-// `pitch` floats), `rank0` = cluster rank of part 0, `tid` of 256 threads.
-template <int W, bool F32, bool F16>
+// `pitch` floats), `rank0` = cluster rank of part 0, `tid` of 256 threads; ROWS rows in all.
+template <int W, bool F32, bool F16, int ROWS = BM>
 __device__ __forceinline__ void reduce_store(uint32_t stage, int pitch, int c0, int rank0, int part, int split, int tid, void* base,
                                              int head, int m0, int n_rows, int d_mem, float mul) {
   constexpr int V = F32 ? 4 : 8;
-  const int rows = (BM + split - 1) / split;
+  const int rows = (ROWS + split - 1) / split;
   for (int i = tid; i < rows * (W / V); i += EW_THREADS) {
     const int r = part * rows + i / (W / V), c = (i % (W / V)) * V;
-    if (r >= BM || m0 + r >= n_rows || c >= d_mem) continue;   // rows are whole 16-byte pieces
+    if (r >= ROWS || m0 + r >= n_rows || c >= d_mem) continue;   // rows are whole 16-byte pieces
     float4 a[V / 4];
 #pragma unroll
     for (int h = 0; h < V / 4; ++h) a[h] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -361,7 +361,7 @@ constexpr int kMaxSplit = 8;   // the portable cluster size
 // straddle GPCs, so some SMs stay idle (a B200 with 148 SMs: 132 in clusters of 4 or 6, 120 in clusters
 // of 8).  Asked once per device and host thread.
 template <class K>
-int cluster_slots(K kernel, int smem, int c) {
+int cluster_slots(K kernel, int smem, int c, int threads = NTHREADS) {
   constexpr int kDevices = 64;
   static thread_local int table[kDevices][kMaxSplit + 1] = {};
   int dev = 0;
@@ -374,7 +374,7 @@ int cluster_slots(K kernel, int smem, int c) {
     attr.val.clusterDim.x = c;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.gridDim = dim3(c * 64);
-    cfg.blockDim = dim3(NTHREADS);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
@@ -393,23 +393,26 @@ int cluster_slots(K kernel, int smem, int c) {
 // parts is a number of partial sums).
 bool may_split(int n_q, int n_k) { return n_q < 4096 || n_k < 4096; }
 
-// Splitting pays while the items leave SMs idle.  Times are in streamed tiles: a CTA takes about kFixed
+// Splitting pays while the items leave SMs idle.  Times are in streamed tiles: a CTA takes about `fixed`
 // tiles' time besides its own (launch, prologue, first loads, epilogue: 6 to 9 us against 1 to 1.7 us a
-// tile), kCluster more in a cluster (its CTAs start together and meet twice), and a second launch costs
-// kLaunch.  Measured with 16 heads, 100 queries, 6000 keys (16 items of 94 tiles, 752 of 2): sweep
+// tile of the tensor-core kernels), `cluster` more in a cluster (its CTAs start together and meet twice), and
+// a second launch costs `launch`.  Measured with 16 heads, 100 queries, 6000 keys (16 items of 94 tiles, 752 of 2): sweep
 // 102 -> 29 us; passes 3 and 4 205 us in one unsplit launch.
+struct SplitCost {
+  float fixed = 5.f, cluster = 1.f, launch = 1.f;
+};
 template <class K>
-SplitChoice choose_split(K kernel, int smem, const SplitWork& wa, const SplitWork& wb) {
-  constexpr float kFixed = 5.f, kCluster = 1.f, kLaunch = 1.f;
+SplitChoice choose_split(K kernel, int smem, const SplitWork& wa, const SplitWork& wb, int threads = NTHREADS,
+                         const SplitCost& cost = SplitCost{}) {
   SplitChoice best = {1, 1, true};
-  const int sms = cluster_slots(kernel, smem, 1);
+  const int sms = cluster_slots(kernel, smem, 1, threads);
   auto fills = [&](const SplitWork& w) { return w.items == 0 || w.items >= sms; };
   if (fills(wa) && fills(wb)) return best;
   auto item_time = [&](const SplitWork& w, int split, int cluster) {
-    return w.items == 0 ? 0.f : (w.tiles + split - 1) / split + kFixed + (cluster > 1 ? kCluster : 0.f);
+    return w.items == 0 ? 0.f : (w.tiles + split - 1) / split + cost.fixed + (cluster > 1 ? cost.cluster : 0.f);
   };
   auto wave_time = [&](int sa, int sb, int cluster, const SplitWork& a, const SplitWork& b) {
-    const float slots = static_cast<float>(cluster_slots(kernel, smem, cluster));
+    const float slots = static_cast<float>(cluster_slots(kernel, smem, cluster, threads));
     if (slots == 0.f) return 1e30f;
     const float ta = item_time(a, sa, cluster), tb = item_time(b, sb, cluster), longest = ta > tb ? ta : tb;
     const float ctas = static_cast<float>(a.items) * sa + static_cast<float>(b.items) * sb;
@@ -427,7 +430,7 @@ SplitChoice choose_split(K kernel, int smem, const SplitWork& wa, const SplitWor
         if (t < best_time) { best_time = t; best = {sa, sb, true}; }
       }
       if (wa.items && wb.items) {
-        const float t = wave_time(sa, 1, sa, wa, none) + wave_time(1, sb, sb, none, wb) + kLaunch;
+        const float t = wave_time(sa, 1, sa, wa, none) + wave_time(1, sb, sb, none, wb) + cost.launch;
         if (t < best_time) { best_time = t; best = {sa, sb, false}; }
       }
     }
