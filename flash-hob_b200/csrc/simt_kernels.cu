@@ -19,11 +19,6 @@ namespace fhob {
 namespace {
 
 constexpr int NT = 256;       // threads per CTA
-// the forward: 8 warps, warp w owns rows 4w..4w+3, lane = column
-constexpr int TM = 32;        // stationary rows per CTA
-constexpr int TN = 32;        // streamed rows per step
-constexpr int RPW = TM / 8;   // rows per warp
-constexpr int DCH = 4;        // output columns per thread and row: lane + 32*m, m < DCH  (d <= 128)
 
 struct SimtParams {
   const void *q, *k, *v, *d_o, *ddq, *ddk, *ddv;
@@ -37,12 +32,6 @@ struct SimtParams {
   int split_q, split_k;   // CTAs that share the streamed tiles of such a pair
   int cluster;            // CTAs of a cluster (a multiple of both)
 };
-
-// Grid of (stationary tiles, heads): heads beyond what grid.y can index continue in grid.z.
-constexpr int kMaxGridY = 65535;
-inline dim3 head_grid(int tiles, int bh) {
-  return dim3(tiles, bh < kMaxGridY ? bh : kMaxGridY, (bh + kMaxGridY - 1) / kMaxGridY);
-}
 
 template <typename T>
 __device__ __forceinline__ float ld_elem(const void* p, size_t i);
@@ -71,17 +60,6 @@ __device__ __forceinline__ void st_elem<float>(void* p, size_t i, float v) {
 template <>
 __device__ __forceinline__ void st_elem<__nv_bfloat16>(void* p, size_t i, float v) {
   static_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(v);
-}
-
-// Loads rows [row0, row0+rows) of a (n, d) matrix into a [rows][ld] fp32 tile, zero beyond n.
-template <typename T>
-__device__ __forceinline__ void load_tile(float* tile, int ld, const void* src, size_t head_off,
-                                          int row0, int rows, int n, int d) {
-  for (int idx = threadIdx.x; idx < rows * d; idx += NT) {
-    int r = idx / d, c = idx - r * d;
-    int gr = row0 + r;
-    tile[r * ld + c] = gr < n ? ld_elem<T>(src, head_off + static_cast<size_t>(gr) * d + c) : 0.f;
-  }
 }
 
 __device__ __forceinline__ float warp_sum(float x) {
@@ -519,98 +497,207 @@ __global__ void __launch_bounds__(NT, 1) simt_pass_kernel(const __grid_constant_
   else if constexpr (MODE_K != 0) simt_body<T, MODE_K>(p, block - p.q_blocks);
 }
 
-// O(N)-memory forward: online softmax over key tiles.
+// O(N)-memory forward: online softmax.  A CTA owns OM = 64 queries and streams FN = 128 keys; a warp owns eight
+// rows of both the scores and the outputs, so a row's maximum and sum never leave the warp and P passes
+// through shared memory without a CTA barrier.  The warp's operand on the row side (Q, P) is the same
+// address for all lanes; of the other one (K, V) a thread reads one float4 per 32 multiply-adds.  K of the next
+// step arrives during P V, V during Q K^T.  Few items are split over clusters, as the operator's.
+// fp32, D = 128, us, before (32 queries a CTA, two to four FMAs per word read) -> now:
+// 8 heads N = 1024 405 -> 131, 32 causal heads N = 512 294 -> 91, 4 heads 200 x 5000 (d_v 64) 1260 -> 115.
+constexpr int FN = 128;
+constexpr int kForwardSmem = 4 * ((OM + 2 * FN) * OP + FN * PP);
+constexpr int kForwardPitch = 128 + 4;   // floats per staged row of a split problem: the outputs, maximum, sum
+
+// As load_rows for callers whose rows are not whole 16-byte pieces: element by element, zeros up to a multiple of four.
 template <typename T>
-__global__ void __launch_bounds__(NT) simt_forward_kernel(const SimtParams p, void* o_out, float* lse_out) {
-  extern __shared__ float smem[];
-  const int d = p.d, dv = p.dv, ld = (d > dv ? d : dv) + 1;
-  float* qs = smem;
-  float* ks = qs + TM * ld;
-  float* vs = ks + TN * ld;
-  float* ps = vs + TN * ld;  // [TM][TN+1]
-  constexpr int LT = TN + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * TM, bh = blockIdx.y + blockIdx.z * kMaxGridY;   // see head_grid
-  if (bh >= p.bh) return;
-  const size_t qoff = static_cast<size_t>(bh) * p.n_q * d, qoff_v = static_cast<size_t>(bh) * p.n_q * dv;
-  const size_t koff = static_cast<size_t>(bh) * p.n_k * d, koff_v = static_cast<size_t>(bh) * p.n_k * dv;
-  const int causal_off = p.n_k - p.n_q;
-  load_tile<T>(qs, ld, p.q, qoff, m0, TM, p.n_q, d);
-  float mrow[RPW], lrow[RPW], acc[RPW][DCH];
-#pragma unroll
-  for (int i = 0; i < RPW; ++i) {
-    mrow[i] = -INFINITY;
-    lrow[i] = 0.f;
-#pragma unroll
-    for (int m = 0; m < DCH; ++m) acc[i][m] = 0.f;
+__device__ __forceinline__ void load_rows_any(float* tile, const void* src, size_t head_off, int row0, int rows, int n, int d, bool vec) {
+  if (vec) {
+    load_rows<T>(tile, src, head_off, row0, rows, n, d);
+    return;
   }
-  int t_begin, t_end;
-  visible_tiles(true, m0, TM, TN, p.n_k, causal_off, p.causal, p.window, t_begin, t_end);
-  const float sl2 = p.scale * kLog2e;
-  for (int t = t_begin; t < t_end; ++t) {
-    const int n0 = t * TN;
-    __syncthreads();
-    load_tile<T>(ks, ld, p.k, koff, n0, TN, p.n_k, d);
-    if (o_out) load_tile<T>(vs, ld, p.v, koff_v, n0, TN, p.n_k, dv);
-    __syncthreads();
-    float s[RPW];
-#pragma unroll
-    for (int i = 0; i < RPW; ++i) s[i] = 0.f;
-    for (int e = 0; e < d; ++e) {
-      float c0 = ks[lane * ld + e];
-#pragma unroll
-      for (int i = 0; i < RPW; ++i) s[i] = fmaf(qs[(warp * RPW + i) * ld + e], c0, s[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < RPW; ++i) {
-      int r = warp * RPW + i, qi = m0 + r, kj = n0 + lane;
-      bool allowed = qi < p.n_q && kj < p.n_k && pair_visible(qi, kj, causal_off, p.causal, p.window);
-      float sv = allowed ? s[i] * sl2 : -INFINITY;  // log2 domain
-      float mnew = fmaxf(mrow[i], warp_max(sv));
-      float alpha = (mnew == -INFINITY) ? 1.f : exp2f(mrow[i] - mnew);
-      float pv = (mnew == -INFINITY) ? 0.f : exp2f(sv - mnew);
-      lrow[i] = lrow[i] * alpha + warp_sum(pv);
-      mrow[i] = mnew;
-      ps[r * LT + lane] = pv;
-#pragma unroll
-      for (int m = 0; m < DCH; ++m) acc[i][m] *= alpha;
-    }
-    __syncwarp();
-    for (int c = 0; c < TN; ++c) {
-      float bv[DCH];
-#pragma unroll
-      for (int m = 0; m < DCH; ++m) {
-        int col = lane + 32 * m;
-        bv[m] = (col < dv && o_out) ? vs[c * ld + col] : 0.f;
-      }
-#pragma unroll
-      for (int i = 0; i < RPW; ++i) {
-        float pv = ps[(warp * RPW + i) * LT + c];
-#pragma unroll
-        for (int m = 0; m < DCH; ++m) acc[i][m] = fmaf(pv, bv[m], acc[i][m]);
-      }
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < RPW; ++i) {
-    int qi = m0 + warp * RPW + i;
-    if (qi >= p.n_q) continue;
-    float inv = lrow[i] > 0.f ? 1.f / lrow[i] : 0.f;
-#pragma unroll
-    for (int m = 0; m < DCH; ++m) {
-      int col = lane + 32 * m;
-      if (col < dv && o_out) st_elem<T>(o_out, qoff_v + static_cast<size_t>(qi) * dv + col, acc[i][m] * inv);
-    }
-    if (lane == 0)
-      lse_out[static_cast<size_t>(bh) * p.n_q + qi] =
-          lrow[i] > 0.f ? (mrow[i] + log2f(lrow[i])) * 0.6931471805599453f : -INFINITY;
+  const int w = (d + 3) & ~3;
+  for (int idx = threadIdx.x; idx < rows * w; idx += NT) {
+    const int r = idx / w, c = idx - r * w;
+    const bool live = row0 + r < n && c < d;
+    tile[r * OP + c] = live ? ld_elem<T>(src, head_off + static_cast<size_t>(row0 + r) * d + c) : 0.f;
   }
 }
 
-int pitch(const FhobProblem& p) {  // row pitch of the shared-memory tiles: the larger head dim + 1
-  const int dv = head_dim_v(p);
-  return (p.d > dv ? p.d : dv) + 1;
+__device__ __forceinline__ void loads_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void loads_landed_but_last() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
+template <typename T>
+__global__ void __launch_bounds__(NT, 1) simt_forward_kernel(const __grid_constant__ SimtParams p, void* o_out, float* lse_out, bool vec) {
+  pdl_wait();
+  if (threadIdx.x == 0) pdl_launch_dependents();
+  extern __shared__ float smem[];
+  float *qs = smem, *ks = qs + OM * OP, *vs = ks + FN * OP, *ps = vs + FN * OP;   // ps: [key][query]
+  const int d = p.d, dv = p.dv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int split = p.split_q;
+  int item = blockIdx.x / split;
+  const int part = blockIdx.x - item * split;
+  const bool live = item < p.items_q;
+  if (!live) item = 0;
+  const int tile_no = item / p.bh, bh = item - tile_no * p.bh;   // causal: the longest tiles of all heads first
+  const int m0 = ((p.n_q + OM - 1) / OM - 1 - tile_no) * OM, row0 = m0 + 8 * warp;
+  const size_t qoff = static_cast<size_t>(bh) * p.n_q * d, ooff = static_cast<size_t>(bh) * p.n_q * dv;
+  const size_t koff = static_cast<size_t>(bh) * p.n_k * d, voff = static_cast<size_t>(bh) * p.n_k * dv;
+  const int off = p.n_k - p.n_q;
+  int t_begin, t_end;
+  visible_tiles(true, m0, OM, FN, p.n_k, off, p.causal, p.window, t_begin, t_end);
+  if (split > 1) split_range(part, split, t_begin, t_end);
+  if (!live) t_end = t_begin;
+  const float sl2 = p.scale * kLog2e;
+
+  float mrow[8], lrow[8];   // maximum (of the row) and sum (of this lane's columns), log2 domain
+  float2 acc[8][2];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    mrow[i] = -INFINITY;
+    lrow[i] = 0.f;
+    acc[i][0] = acc[i][1] = make_float2(0.f, 0.f);
+  }
+  load_rows_any<T>(qs, p.q, qoff, m0, OM, p.n_q, d, vec);
+  if (t_begin < t_end) load_rows_any<T>(ks, p.k, koff, t_begin * FN, FN, p.n_k, d, vec);
+  loads_commit();
+
+  for (int t = t_begin; t < t_end; ++t) {
+    const int n0 = t * FN;
+    if (o_out) load_rows_any<T>(vs, p.v, voff, n0, FN, p.n_k, dv, vec);
+    loads_commit();
+    loads_landed_but_last();
+    __syncthreads();   // Q, K
+
+    float2 s[8][4];   // rows 8 warp + i, keys lane + 32 j; even and odd elements of the contraction apart
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = make_float2(0.f, 0.f);
+    const float *qa = qs + 8 * warp * OP, *ka = ks + lane * OP;
+#pragma unroll 2
+    for (int e = 0; e < d; e += 4) {
+      float4 k[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) k[j] = ld4(ka + 32 * j * OP + e);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 q = ld4(qa + i * OP + e);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dot4(s[i][j], q, k[j]);
+      }
+    }
+    __syncthreads();   // K has been read
+    if (t + 1 < t_end) load_rows_any<T>(ks, p.k, koff, n0 + FN, FN, p.n_k, d, vec);
+    loads_commit();
+
+    const bool masked = n0 + FN > p.n_k || (p.causal && (n0 + FN - 1 > m0 + off || (p.window > 0 && m0 + OM - 1 + off - n0 >= p.window)));
+    float pr[4][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float sv[4], mx = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int c = n0 + lane + 32 * j;
+        const bool ok = !masked || (c < p.n_k && pair_visible(row0 + i, c, off, p.causal, p.window));
+        sv[j] = ok ? (s[i][j].x + s[i][j].y) * sl2 : -INFINITY;
+        mx = fmaxf(mx, sv[j]);
+      }
+      const float mnew = fmaxf(mrow[i], warp_max(mx));
+      const float alpha = mnew == -INFINITY ? 1.f : exp2f(mrow[i] - mnew);
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        pr[j][i] = mnew == -INFINITY ? 0.f : exp2f(sv[j] - mnew);
+        sum += pr[j][i];
+      }
+      lrow[i] = lrow[i] * alpha + sum;
+      mrow[i] = mnew;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) acc[i][h] = make_float2(acc[i][h].x * alpha, acc[i][h].y * alpha);
+    }
+    if (o_out) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float* to = ps + (lane + 32 * j) * PP + 8 * warp;
+        *reinterpret_cast<float4*>(to) = make_float4(pr[j][0], pr[j][1], pr[j][2], pr[j][3]);
+        *reinterpret_cast<float4*>(to + 4) = make_float4(pr[j][4], pr[j][5], pr[j][6], pr[j][7]);
+      }
+    }
+    loads_landed_but_last();
+    __syncthreads();   // V (and this warp's P)
+    if (o_out) {
+      const float *pa = ps + 8 * warp, *va = vs + 4 * lane;
+#pragma unroll 4
+      for (int c = 0; c < FN; ++c) {
+        const float4 al = ld4(pa + c * PP), ah = ld4(pa + c * PP + 4), v = ld4(va + c * OP);
+        const float r[8] = {al.x, al.y, al.z, al.w, ah.x, ah.y, ah.z, ah.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          acc[i][0] = __ffma2_rn(make_float2(r[i], r[i]), lo2(v), acc[i][0]);
+          acc[i][1] = __ffma2_rn(make_float2(r[i], r[i]), hi2(v), acc[i][1]);
+        }
+      }
+      __syncthreads();   // V has been read
+    }
+  }
+  loads_landed();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) lrow[i] = warp_sum(lrow[i]);
+
+  auto store = [&](int row, const float (&o)[4], float m, float l) {   // lane: columns 4 lane..
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+    if (o_out) {
+      const size_t at = ooff + static_cast<size_t>(row) * dv + 4 * lane;
+      if (vec) {
+        if (4 * lane < dv) store4<T>(o_out, at, make_float2(o[0], o[1]), make_float2(o[2], o[3]), inv);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (4 * lane + e < dv) st_elem<T>(o_out, at + e, o[e] * inv);
+      }
+    }
+    if (lane == 0)
+      lse_out[static_cast<size_t>(bh) * p.n_q + row] = l > 0.f ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
+  };
+  if (split <= 1) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float o[4] = {acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y};
+      if (live && row0 + i < p.n_q) store(row0 + i, o, mrow[i], lrow[i]);
+    }
+    return;   // launches without a split have no clusters
+  }
+  // the parts' rows are staged and put on a common maximum, in rank order
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    float* to = smem + (8 * warp + i) * kForwardPitch;
+    store4<float>(to, 4 * lane, acc[i][0], acc[i][1], 1.f);
+    if (lane == 0) {
+      to[128] = mrow[i];
+      to[129] = lrow[i];
+    }
+  }
+  cluster_sync();
+  if (live) {
+    const int rank0 = static_cast<int>(cluster_rank()) - part;
+    for (int r = part + split * warp; r < OM && m0 + r < p.n_q; r += split * 8) {
+      const uint32_t at = smem_u32(smem) + r * kForwardPitch * 4;
+      float m = -INFINITY, l = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
+      for (int i = 0; i < split; ++i) m = fmaxf(m, cluster_ld(cluster_map(at, rank0 + i) + 128 * 4));
+      for (int i = 0; i < split; ++i) {
+        const uint32_t from = cluster_map(at, rank0 + i);
+        const float mi = cluster_ld(from + 128 * 4), w = mi == -INFINITY ? 0.f : exp2f(mi - m);
+        const float4 x = cluster_ld4(from + 16 * lane);
+        l = fmaf(cluster_ld(from + 129 * 4), w, l);
+        o[0] = fmaf(x.x, w, o[0]); o[1] = fmaf(x.y, w, o[1]); o[2] = fmaf(x.z, w, o[2]); o[3] = fmaf(x.w, w, o[3]);
+      }
+      store(m0 + r, o, m, l);
+    }
+  }
+  cluster_sync();   // the others are done with this CTA's shared memory
 }
+
 
 SimtParams make_params(const FhobProblem& p) {
   RowVectors rv = row_vectors(p);
@@ -684,42 +771,46 @@ int launch_backward(const FhobProblem& p, void* dq, void* dk, void* dv, cudaStre
   return launch_modes<T, 5, 6>(s, true, true, st);
 }
 
+// The forward reads rows element by element if they are not whole, aligned 16-byte pieces.
+template <typename T>
+int launch_forward(const FhobProblem& p, void* o_out, float* lse_out, cudaStream_t st) {
+  constexpr auto kernel = simt_forward_kernel<T>;
+  const int ok = allow_smem(kernel, kForwardSmem);
+  if (ok != FHOB_OK) return ok;
+  SimtParams s = make_params(p);
+  auto whole = [](const void* x, int cols) { return ((reinterpret_cast<uintptr_t>(x) | (cols * sizeof(T))) & 15u) == 0; };
+  const bool vec = whole(p.q, s.d) && whole(p.k, s.d) && whole(p.v, s.dv) && whole(o_out, s.dv);
+  const long long items = static_cast<long long>((p.n_q + OM - 1) / OM) * p.bh;
+  if (items > 0x7fffffffLL) return FHOB_ERR_SHAPE;
+  s.items_q = static_cast<int>(items);
+  s.split_q = s.cluster = 1;
+  if (may_split(p.n_q, p.n_k))
+    s.split_q = s.cluster = choose_split(kernel, kForwardSmem, SplitWork{s.items_q, longest(p.n_k, FN, OM, p.window)}, SplitWork{0, 0}, NT, kSimtCost).a;
+  FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(items * s.split_q), NT, kForwardSmem, s.cluster, st, s, o_out, lse_out, vec));
+  return FHOB_OK;
+}
+
 }  // namespace
 
 int simt_backward(const FhobProblem& p, void* dq, void* dk, void* dv, cudaStream_t st) {
-  if (p.d > 32 * DCH || head_dim_v(p) > 32 * DCH) return FHOB_ERR_SHAPE;
+  if (p.d > 128 || head_dim_v(p) > 128) return FHOB_ERR_SHAPE;
   if (p.dtype == FHOB_F32) return launch_backward<float>(p, dq, dk, dv, st);
   if (p.dtype == FHOB_F16) return launch_backward<__half>(p, dq, dk, dv, st);
   return launch_backward<__nv_bfloat16>(p, dq, dk, dv, st);
 }
 
 int simt_pass(int pass, const FhobProblem& p, cudaStream_t st) {
-  if (p.d > 32 * DCH || head_dim_v(p) > 32 * DCH) return FHOB_ERR_SHAPE;
+  if (p.d > 128 || head_dim_v(p) > 128) return FHOB_ERR_SHAPE;
   if (p.dtype == FHOB_F32) return dispatch_pass<float>(pass, p, st);
   if (p.dtype == FHOB_F16) return dispatch_pass<__half>(pass, p, st);
   return dispatch_pass<__nv_bfloat16>(pass, p, st);
 }
 
 int simt_forward(const FhobProblem& p, void* o_out, float* lse_out, cudaStream_t st) {
-  if (p.d > 32 * DCH || head_dim_v(p) > 32 * DCH) return FHOB_ERR_SHAPE;
-  size_t smem = sizeof(float) * ((TM + 2 * TN) * pitch(p) + TM * (TN + 1));
-  dim3 grid = head_grid((p.n_q + TM - 1) / TM, p.bh);
-  SimtParams s = make_params(p);
-  if (p.dtype == FHOB_F32) {
-    FHOB_CUDA_OK(cudaFuncSetAttribute(simt_forward_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem)));
-    simt_forward_kernel<float><<<grid, NT, smem, st>>>(s, o_out, lse_out);
-  } else if (p.dtype == FHOB_F16) {
-    FHOB_CUDA_OK(cudaFuncSetAttribute(simt_forward_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem)));
-    simt_forward_kernel<__half><<<grid, NT, smem, st>>>(s, o_out, lse_out);
-  } else {
-    FHOB_CUDA_OK(cudaFuncSetAttribute(simt_forward_kernel<__nv_bfloat16>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    simt_forward_kernel<__nv_bfloat16><<<grid, NT, smem, st>>>(s, o_out, lse_out);
-  }
-  FHOB_CUDA_OK(cudaGetLastError());
-  return FHOB_OK;
+  if (p.d > 128 || head_dim_v(p) > 128) return FHOB_ERR_SHAPE;
+  if (p.dtype == FHOB_F32) return launch_forward<float>(p, o_out, lse_out, st);
+  if (p.dtype == FHOB_F16) return launch_forward<__half>(p, o_out, lse_out, st);
+  return launch_forward<__nv_bfloat16>(p, o_out, lse_out, st);
 }
 
 }  // namespace fhob

@@ -68,3 +68,38 @@ def test_single_passes_give_the_operator():
         assert f(C.byref(p), s) == 0
     for a, b in zip(out, ref):   # chains of 70 to 100 FMAs in another order: sqrt(100) * 2^-24 = 6e-7, on both sides, of the largest entry
         assert O.rel_err(a, b) < 2e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bh,nq,nk,d,dv,causal,window",
+                         [(1, 1, 1, 4, 128, False, None), (2, 64, 128, 128, 64, False, None), (3, 65, 129, 96, 4, True, None),
+                          (1, 200, 127, 128, 128, True, None), (2, 130, 300, 68, 72, True, 40), (1, 64, 4000, 128, 128, False, None),
+                          (5, 70, 3000, 128, 96, True, 900), (1, 33, 70, 5, 7, False, None), (2, 100, 600, 127, 2, True, None)])
+def test_forward_matches_oracle(bh, nq, nk, d, dv, causal, window):
+    """The forward at the edges of its 64 x 128 tiles, split keys, dead rows, and rows that are not whole 16-byte pieces (C ABI)."""
+    import ctypes as C
+    from fhob import _lib
+    lib = _lib.load()
+    g = torch.Generator().manual_seed(nq + nk)
+    q, k, v = torch.randn(bh, nq, d, generator=g), torch.randn(bh, nk, d, generator=g), torch.randn(bh, nk, dv, generator=g)
+    w = math.inf if window is None else window
+    scale = d ** -0.5
+    dead = max(0, nq - nk) if causal else 0
+    dev = [t.cuda() for t in (q, k, v)]
+    p = _lib.FhobProblem()
+    p.bh, p.n_q, p.n_k, p.d, p.d_v, p.dtype, p.scale = bh, nq, nk, d, dv, _lib.FHOB_F32, scale
+    p.causal, p.window, p.impl = int(causal), window or 0, _lib.IMPL["simt"]
+    p.q, p.k, p.v = (t.data_ptr() for t in dev)
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for need_o in (True, False):
+        o = torch.full((bh, nq, dv), float("nan"), device="cuda")
+        lse = torch.full((bh, nq), float("nan"), device="cuda")
+        assert lib.fhob_forward(C.byref(p), C.c_void_p(o.data_ptr() if need_o else None), C.c_void_p(lse.data_ptr()), stream) == 0
+        ql = q[:, dead:].double()
+        ref_l = O.attn_lse(ql, k.double(), scale, causal, w)
+        # sums of up to 4000 + 128 terms with 2^-24 each as a random walk (4e-6), doubled for the exponent of 2
+        assert float((lse[:, dead:].double().cpu() - ref_l).abs().max()) < 1e-5
+        assert (lse[:, :dead] == -math.inf).all()
+        if need_o:
+            assert O.rel_err(o[:, dead:], O.attn_fwd(ql, k.double(), v.double(), scale, causal, w)) < 1e-5
+            assert (o[:, :dead] == 0).all()
