@@ -185,7 +185,9 @@ int fhob_pass4(const FhobProblem* p, void* stream);
  *   b_i = sum_j P_ij (X_ij + dP_ij ddS_ij) - 2 D_i dd_i,
  * whose sums do not need dd_i while the tiles stream by, so S, P and ddS
  * are recomputed once instead of twice (5 contractions instead of 3 + 5).
- * The reference has no such stage.  (The CUDA-core path runs its two passes.)
+ * The reference has no such stage.  The CUDA-core path runs one sweep as
+ * well, with D known beforehand (fhob_prepass): fhob_pass1, fhob_pass2 and
+ * fhob_pass12 are that sweep there, and each leaves both dd and b.
  */
 int fhob_pass12(const FhobProblem* p, void* stream);
 
