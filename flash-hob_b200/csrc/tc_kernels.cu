@@ -898,7 +898,7 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
           stage_row<DQK / 2>(dst + half * (DQK / 2), acc + half * (DQK / 2), n_iter > 0);
           stage_row<DV / 2>(dst + DQK + half * (DV / 2), acc + C::OUT0_COLS + half * (DV / 2), n_iter > 0);
         }
-      } else if (ok) {
+      } else if (ok && live) {   // a CTA that only fills up a cluster has no tile to store
         auto store_out = [&](auto width, int d_mem, uint32_t col0, void* base, float mul) {
           constexpr int DO = decltype(width)::value;   // columns of the accumulator; d_mem <= DO of them exist in memory
           uint16_t* dst = static_cast<uint16_t*>(base) + (static_cast<size_t>(head) * n_stat + (g_row < n_stat ? g_row : 0)) * d_mem + half * (DO / 2);
