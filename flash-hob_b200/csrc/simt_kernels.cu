@@ -604,10 +604,11 @@ __global__ void __launch_bounds__(NT, 1) simt_forward_kernel(const __grid_consta
       }
       const float mnew = fmaxf(mrow[i], warp_max(mx));
       const float alpha = mnew == -INFINITY ? 1.f : exp2f(mrow[i] - mnew);
+      const float from = mnew == -INFINITY ? 0.f : mnew;   // no maximum yet: P = 0 for hidden keys, NaN for NaN scores
       float sum = 0.f;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        pr[j][i] = mnew == -INFINITY ? 0.f : exp2f(sv[j] - mnew);
+        pr[j][i] = exp2f(sv[j] - from);
         sum += pr[j][i];
       }
       lrow[i] = lrow[i] * alpha + sum;
@@ -645,7 +646,7 @@ __global__ void __launch_bounds__(NT, 1) simt_forward_kernel(const __grid_consta
   for (int i = 0; i < 8; ++i) lrow[i] = warp_sum(lrow[i]);
 
   auto store = [&](int row, const float (&o)[4], float m, float l) {   // lane: columns 4 lane..
-    const float inv = l > 0.f ? 1.f / l : 0.f;
+    const float inv = l == 0.f ? 0.f : 1.f / l;   // a sum of zero: no visible key (a NaN is kept)
     if (o_out) {
       const size_t at = ooff + static_cast<size_t>(row) * dv + 4 * lane;
       if (vec) {
@@ -657,7 +658,7 @@ __global__ void __launch_bounds__(NT, 1) simt_forward_kernel(const __grid_consta
       }
     }
     if (lane == 0)
-      lse_out[static_cast<size_t>(bh) * p.n_q + row] = l > 0.f ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
+      lse_out[static_cast<size_t>(bh) * p.n_q + row] = l == 0.f ? -INFINITY : (m + log2f(l)) * 0.6931471805599453f;
   };
   if (split <= 1) {
 #pragma unroll
@@ -687,9 +688,11 @@ __global__ void __launch_bounds__(NT, 1) simt_forward_kernel(const __grid_consta
       for (int i = 0; i < split; ++i) m = fmaxf(m, cluster_ld(cluster_map(at, rank0 + i) + 128 * 4));
       for (int i = 0; i < split; ++i) {
         const uint32_t from = cluster_map(at, rank0 + i);
-        const float mi = cluster_ld(from + 128 * 4), w = mi == -INFINITY ? 0.f : exp2f(mi - m);
+        const float mi = cluster_ld(from + 128 * 4), li = cluster_ld(from + 129 * 4);
+        if (li == 0.f) continue;   // a part without a visible key
+        const float w = mi == -INFINITY ? 1.f : exp2f(mi - m);   // (no maximum but a sum: NaN)
         const float4 x = cluster_ld4(from + 16 * lane);
-        l = fmaf(cluster_ld(from + 129 * 4), w, l);
+        l = fmaf(li, w, l);
         o[0] = fmaf(x.x, w, o[0]); o[1] = fmaf(x.y, w, o[1]); o[2] = fmaf(x.z, w, o[2]); o[3] = fmaf(x.w, w, o[3]);
       }
       store(m0 + r, o, m, l);

@@ -120,14 +120,20 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, 
 }
 
 // 2^x for two numbers on the FMA and ALU pipes, to relieve the special-function units (16 a clock and SM)
-// where they are what a kernel waits for.  x = n + f with n the nearest integer, |f| <= 1/2; 2^f is the
-// degree-5 polynomial with the smallest relative error there (Remez exchange, 7.5e-8; 2.1e-7 evaluated in
-// fp32, as ex2.approx: 2^-22), and n is added to the exponent field.  x <= 127; below -126 the result
-// is about 2^-126 or less, never a larger number.
+// where they are what a kernel waits for.  x = n + f with n the nearest integer, |f| <= 1/2; 2^f is a
+// degree-5 polynomial of small relative error there (Remez exchange; 1.3e-7 with the coefficients rounded as
+// written, 2.1e-7 evaluated in fp32, as ex2.approx: 2^-22), times 2^n put together from its exponent field.
+// x <= 127; below -126 the result is about 2^-126 or less, never a larger number; NaN stays NaN (a clamp that
+// keeps it, and a product: an integer added to the exponent of a NaN makes a number of it).
+__device__ __forceinline__ float clamp_exp2(float x) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(-126.f));
+  return r;
+}
 __device__ __forceinline__ float2 exp2_fma(float2 x) {
   constexpr float kMagic = 12582912.f;   // 1.5 * 2^23: adding it leaves the nearest integer in the low bits
-  x.x = fmaxf(x.x, -126.f);
-  x.y = fmaxf(x.y, -126.f);
+  x.x = clamp_exp2(x.x);
+  x.y = clamp_exp2(x.y);
   const float2 r = __fadd2_rn(x, make_float2(kMagic, kMagic));
   const float2 n = __fadd2_rn(r, make_float2(-kMagic, -kMagic));
   const float2 f = __ffma2_rn(n, make_float2(-1.f, -1.f), x);
@@ -137,9 +143,8 @@ __device__ __forceinline__ float2 exp2_fma(float2 x) {
   y = __ffma2_rn(y, f, c(0.2402212f));
   y = __ffma2_rn(y, f, c(0.69314694f));
   y = __ffma2_rn(y, f, c(1.0000001f));
-  y.x = __uint_as_float(__float_as_uint(y.x) + (__float_as_uint(r.x) << 23));
-  y.y = __uint_as_float(__float_as_uint(y.y) + (__float_as_uint(r.y) << 23));
-  return y;
+  return __fmul2_rn(y, make_float2(__uint_as_float((__float_as_uint(r.x) << 23) + 0x3f800000u),
+                                   __uint_as_float((__float_as_uint(r.y) << 23) + 0x3f800000u)));
 }
 
 // ---- split streamed axis: a cluster of `split` CTAs shares the streamed tiles of one stationary tile

@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) fw_kernel(const __grid_constant
           mbar_arrive(&bars->p_half[x]);
         }
       }
-            run_l += (sum[0].x + sum[1].x) + (sum[0].y + sum[1].y);
+      run_l += (sum[0].x + sum[1].x) + (sum[0].y + sum[1].y);
       if (OUT) {
         tmem_wait_st();
         tc_fence_before();
@@ -451,9 +451,10 @@ __global__ void __launch_bounds__(FW_THREADS, 1) fw_kernel(const __grid_constant
         bars->red[1][row] = run_l;
       }
     } else if (ok && live(x) && (!OUT || g_row - lane < p.n_q)) {
-      const float inv_l = run_l > 0.f ? 1.f / run_l : 0.f;
+      // a sum of zero: no visible key (a NaN is kept)
+      const float inv_l = run_l == 0.f ? 0.f : 1.f / run_l;
       if (g_row < p.n_q)
-        p.lse_out[static_cast<size_t>(head) * p.n_q + g_row] = run_l > 0.f ? (run_m + log2f(run_l)) * 0.6931471805599453f : -INFINITY;
+        p.lse_out[static_cast<size_t>(head) * p.n_q + g_row] = run_l == 0.f ? -INFINITY : (run_m + log2f(run_l)) * 0.6931471805599453f;
       if (OUT) {
         const size_t at = (static_cast<size_t>(head) * p.n_q + g_row) * p.d_v;
 #pragma unroll
@@ -509,11 +510,10 @@ __global__ void __launch_bounds__(FW_THREADS, 1) fw_kernel(const __grid_constant
 #pragma unroll
         for (int h = 0; h < V / 4; ++h) a[h] = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int q = 0; q < p.split; ++q) {
-          const float mq = cluster_ld(cluster_map(red + r * 4, q));
-          if (mq == -INFINITY) continue;   // a part without a visible key
-          const float w = ex2(mq - m);
-          l = fmaf(cluster_ld(cluster_map(red + (BM + r) * 4, q)), w, l);
-          if (OUT) {
+          const float mq = cluster_ld(cluster_map(red + r * 4, q)), lq = cluster_ld(cluster_map(red + (BM + r) * 4, q));
+          const float w = mq == -INFINITY ? 1.f : ex2(mq - m);   // (no maximum but a sum: NaN)
+          l = fmaf(lq, w, l);
+          if (OUT && lq != 0.f) {   // a part without a visible key has nothing to add
             const uint32_t from = cluster_map(stage + (r * C::kPitch + c) * 4, q);
 #pragma unroll
             for (int h = 0; h < V / 4; ++h) {
@@ -524,9 +524,9 @@ __global__ void __launch_bounds__(FW_THREADS, 1) fw_kernel(const __grid_constant
           }
         }
         const size_t g = static_cast<size_t>(head) * p.n_q + m0 + r;
-        if (c == 0) p.lse_out[g] = l > 0.f ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
+        if (c == 0) p.lse_out[g] = l == 0.f ? -INFINITY : (m + log2f(l)) * 0.6931471805599453f;
         if (OUT && c < p.d_v) {
-          const float inv_l = l > 0.f ? 1.f / l : 0.f;
+          const float inv_l = l == 0.f ? 0.f : 1.f / l;
           if constexpr (SPLIT)
             *reinterpret_cast<float4*>(static_cast<float*>(p.o) + g * p.d_v + c) = make_float4(a[0].x * inv_l, a[0].y * inv_l, a[0].z * inv_l, a[0].w * inv_l);
           else
