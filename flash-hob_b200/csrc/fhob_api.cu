@@ -330,6 +330,21 @@ int fhob_visible_tiles(int q_stationary, int m0, int rows, int tile, int n_q, in
   return FHOB_OK;
 }
 
+int fhob_cta_work(const FhobProblem* p, int64_t block, int32_t* pass, int32_t* item, int32_t* part, int32_t* parts) {
+  if (!p || !pass || !item || !part || !parts || block < 0 || p->bh <= 0 || p->n_q <= 0 || p->n_k <= 0) return FHOB_ERR_ARG;
+  PairGrid g;
+  const int st = use_tc(*p) ? tc_grid(*p, &g) : simt_grid(*p, &g);
+  if (st != FHOB_OK) return st;
+  if (block >= g.blocks) return FHOB_ERR_ARG;
+  const bool q_side = block < g.q_blocks;
+  *parts = q_side ? g.split_q : g.split_k;
+  const CtaWork w = cta_work(static_cast<int>(block) - (q_side ? 0 : g.q_blocks), *parts, q_side ? g.items_q : g.items_k);
+  *pass = !w.live ? 0 : (q_side ? 3 : 4);
+  *item = w.item;
+  *part = w.part;
+  return FHOB_OK;
+}
+
 int fhob_selftest_expired_wait(void* workspace, size_t workspace_bytes, void* stream) {
   if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255u) || workspace_bytes < sizeof(int))
     return FHOB_ERR_WORKSPACE;

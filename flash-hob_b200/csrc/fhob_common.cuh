@@ -165,6 +165,18 @@ void set_cuda_error_text(const char* text);
     }                                                       \
   } while (0)
 
+// Launch with query-tiled and key-tiled CTAs (pair_grid in tc_common.cuh): the first q_blocks CTAs are query-tiled.
+struct PairGrid {
+  int items_q, items_k;   // (head, stationary tile) pairs of either kind
+  int split_q, split_k;   // CTAs that share the streamed tiles of one such pair
+  int cluster;            // CTAs of a cluster (a multiple of the splits in use)
+  int q_blocks;
+  long long blocks;
+};
+// Grid of passes 3 and 4 of a whole problem; FHOB_ERR_SHAPE if it has too many CTAs
+int simt_grid(const FhobProblem& p, PairGrid* g);
+int tc_grid(const FhobProblem& p, PairGrid* g);
+
 // CUDA-core kernels (fp32 accumulate, any sizes): simt_kernels.cu
 int simt_pass(int pass, const FhobProblem& p, cudaStream_t s);
 int simt_forward(const FhobProblem& p, void* o_out, float* lse_out, cudaStream_t s);

@@ -211,12 +211,11 @@ __device__ __forceinline__ void simt_body(const SimtParams& p, int block) {
   const int group = threadIdx.x >> 7, tid = threadIdx.x & 127;
   const int ty = tid >> 3, tx = tid & 7;     // scores: rows 4 ty + i, streamed rows tx + 8 j
   const int ry = tid >> 4, cx = tid & 15;    // outputs: rows 8 ry + i, columns 4 cx.. and 64 + 4 cx..
-  // with few items the streamed axis is split over the CTAs of a cluster
+  // with few tiles a head the streamed axis is split over the CTAs of a cluster
   const int split = kQStat ? p.split_q : p.split_k;
-  int item = block / split;
-  const int begin_part = block - item * split;
-  const bool padding = item >= (kQStat ? p.items_q : p.items_k);   // the grid is padded to whole clusters
-  if (padding) item = 0;
+  const CtaWork work = cta_work(block, split, kQStat ? p.items_q : p.items_k);   // the grid is padded to whole clusters
+  const int item = work.item, begin_part = work.part;
+  const bool padding = !work.live;
   const int tile_no = item / p.bh, bh = item - tile_no * p.bh;   // causal: the longest tiles of all heads first
   const int tiles = ((kQStat ? p.n_q : p.n_k) + OM - 1) / OM;
   const int m0 = (kQStat ? tiles - 1 - tile_no : tile_no) * OM;
@@ -501,9 +500,9 @@ __global__ void __launch_bounds__(NT, 1) simt_pass_kernel(const __grid_constant_
 // rows of both the scores and the outputs, so a row's maximum and sum never leave the warp and P passes
 // through shared memory without a CTA barrier.  The warp's operand on the row side (Q, P) is the same
 // address for all lanes; of the other one (K, V) a thread reads one float4 per 32 multiply-adds.  K of the next
-// step arrives during P V, V during Q K^T.  Few items are split over clusters, as the operator's.
+// step arrives during P V, V during Q K^T.  Heads of few tiles are split over clusters, as the operator's.
 // fp32, D = 128, us, before (32 queries a CTA, two to four FMAs per word read) -> now:
-// 8 heads N = 1024 405 -> 131, 32 causal heads N = 512 294 -> 91, 4 heads 200 x 5000 (d_v 64) 1260 -> 115.
+// 8 heads N = 1024 405 -> 129, 32 causal heads N = 512 294 -> 90.  4 heads 200 x 5000, in two parts: 316.
 constexpr int FN = 128;
 constexpr int kForwardSmem = 4 * ((OM + 2 * FN) * OP + FN * PP);
 constexpr int kForwardPitch = 128 + 4;   // floats per staged row of a split problem: the outputs, maximum, sum
@@ -534,10 +533,9 @@ __global__ void __launch_bounds__(NT, 1) simt_forward_kernel(const __grid_consta
   float *qs = smem, *ks = qs + OM * OP, *vs = ks + FN * OP, *ps = vs + FN * OP;   // ps: [key][query]
   const int d = p.d, dv = p.dv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = p.split_q;
-  int item = blockIdx.x / split;
-  const int part = blockIdx.x - item * split;
-  const bool live = item < p.items_q;
-  if (!live) item = 0;
+  const CtaWork work = cta_work(blockIdx.x, split, p.items_q);
+  const int item = work.item, part = work.part;
+  const bool live = work.live;
   const int tile_no = item / p.bh, bh = item - tile_no * p.bh;   // causal: the longest tiles of all heads first
   const int m0 = ((p.n_q + OM - 1) / OM - 1 - tile_no) * OM, row0 = m0 + 8 * warp;
   const size_t qoff = static_cast<size_t>(bh) * p.n_q * d, ooff = static_cast<size_t>(bh) * p.n_q * dv;
@@ -720,36 +718,30 @@ inline int longest(int n, int tile, int rows, int window) {
 }
 
 // In streamed tiles (fp32, D = 128: 12 us in passes 3 and 4): what a CTA takes besides its tiles is about one
-// tile's time, meeting in a cluster about half of one.  Operator, fp32, D = 128, us, one CTA an item ->
-// split: 1 head 64x3000 2434 -> 332, 1 causal head N=2000 1706 -> 723, 4 heads 200x5000 (d_v 64) 3435 -> 898.
-constexpr SplitCost kSimtCost = {1.f, 0.5f, 0.5f};
+// tile's time, meeting in a cluster about half of one.  Operator, fp32, D = 128, us, unsplit -> split: 1 head
+// 64 x 3000 2497 -> 332, 4 heads 200 x 5000 4156 -> 2118; 64 heads 200 x 1000 2390 -> 2411.
+constexpr SplitCost kSimtCost = {1.f, 0.5f};
+
+PairGrid modes_grid(const FhobProblem& p, bool q_side, bool k_side) {
+  const int tiles_q = (p.n_q + OM - 1) / OM, tiles_k = (p.n_k + OM - 1) / OM;
+  return pair_grid(q_side ? static_cast<long long>(tiles_q) * p.bh : 0, split_parts(tiles_q, longest(p.n_k, ON, OM, p.window), kSimtCost),
+                   k_side ? static_cast<long long>(tiles_k) * p.bh : 0, split_parts(tiles_k, longest(p.n_q, ON, OM, p.window), kSimtCost));
+}
 
 template <typename T, int MODE_Q, int MODE_K>
-int launch_modes(SimtParams& p, bool q_side, bool k_side, cudaStream_t st) {
+int launch_modes(const FhobProblem& problem, SimtParams& p, bool q_side, bool k_side, cudaStream_t st) {
   constexpr auto kernel = simt_pass_kernel<T, MODE_Q, MODE_K>;
   constexpr int kQ = Tiles<MODE_Q>::SMEM_BYTES, kK = Tiles<MODE_K ? MODE_K : MODE_Q>::SMEM_BYTES, kSmem = kQ > kK ? kQ : kK;
   const int ok = allow_smem(kernel, kSmem);
   if (ok != FHOB_OK) return ok;
-  const long long items_q = q_side ? static_cast<long long>((p.n_q + OM - 1) / OM) * p.bh : 0;
-  const long long items_k = k_side ? static_cast<long long>((p.n_k + OM - 1) / OM) * p.bh : 0;
-  if (items_q + items_k > 0x7fffffffLL) return FHOB_ERR_SHAPE;
-  const SplitWork wq = {static_cast<int>(items_q), longest(p.n_k, ON, OM, p.window)};
-  const SplitWork wk = {static_cast<int>(items_k), longest(p.n_q, ON, OM, p.window)};
-  SplitChoice c = {1, 1, true};
-  if (may_split(p.n_q, p.n_k)) c = choose_split(kernel, kSmem, wq, wk, NT, kSimtCost);
-  auto go = [&](int q, int k, int cluster) -> int {
-    auto padded = [&](long long n) { return (n + cluster - 1) / cluster * cluster; };   // whole clusters for either kind
-    p.items_q = q; p.items_k = k;
-    p.split_q = c.a; p.split_k = c.b;
-    p.cluster = cluster;
-    p.q_blocks = static_cast<int>(padded(static_cast<long long>(q) * c.a));
-    const long long blocks = p.q_blocks + padded(static_cast<long long>(k) * c.b);
-    FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(blocks), NT, kSmem, cluster, st, p));
-    return FHOB_OK;
-  };
-  if (c.together) return go(wq.items, wk.items, c.a > c.b ? c.a : c.b);
-  const int first = go(wq.items, 0, c.a);
-  return first != FHOB_OK ? first : go(0, wk.items, c.b);
+  const PairGrid g = modes_grid(problem, q_side, k_side);
+  if (g.blocks > 0x7fffffffLL) return FHOB_ERR_SHAPE;
+  p.items_q = g.items_q; p.items_k = g.items_k;
+  p.split_q = g.split_q; p.split_k = g.split_k;
+  p.cluster = g.cluster;
+  p.q_blocks = g.q_blocks;
+  FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(g.blocks), NT, kSmem, g.cluster, st, p));
+  return FHOB_OK;
 }
 
 // `pass` as in the entry points; passes 1 and 2 are one sweep, whichever is asked for
@@ -759,10 +751,10 @@ int dispatch_pass(int pass, const FhobProblem& p, cudaStream_t st) {
   switch (pass) {
     case 1:
     case 2:
-    case 12: return launch_modes<T, 2, 0>(s, true, false, st);
-    case 3: return launch_modes<T, 3, 4>(s, true, false, st);
-    case 4: return launch_modes<T, 3, 4>(s, false, true, st);
-    case 34: return launch_modes<T, 3, 4>(s, true, true, st);
+    case 12: return launch_modes<T, 2, 0>(p, s, true, false, st);
+    case 3: return launch_modes<T, 3, 4>(p, s, true, false, st);
+    case 4: return launch_modes<T, 3, 4>(p, s, false, true, st);
+    case 34: return launch_modes<T, 3, 4>(p, s, true, true, st);
   }
   return FHOB_ERR_ARG;
 }
@@ -771,7 +763,7 @@ template <typename T>
 int launch_backward(const FhobProblem& p, void* dq, void* dk, void* dv, cudaStream_t st) {
   SimtParams s = make_params(p);
   s.dq2 = dq; s.dk2 = dk; s.dv2 = dv;
-  return launch_modes<T, 5, 6>(s, true, true, st);
+  return launch_modes<T, 5, 6>(p, s, true, true, st);
 }
 
 // The forward reads rows element by element if they are not whole, aligned 16-byte pieces.
@@ -786,14 +778,18 @@ int launch_forward(const FhobProblem& p, void* o_out, float* lse_out, cudaStream
   const long long items = static_cast<long long>((p.n_q + OM - 1) / OM) * p.bh;
   if (items > 0x7fffffffLL) return FHOB_ERR_SHAPE;
   s.items_q = static_cast<int>(items);
-  s.split_q = s.cluster = 1;
-  if (may_split(p.n_q, p.n_k))
-    s.split_q = s.cluster = choose_split(kernel, kForwardSmem, SplitWork{s.items_q, longest(p.n_k, FN, OM, p.window)}, SplitWork{0, 0}, NT, kSimtCost).a;
+  s.split_q = s.cluster = split_parts((p.n_q + OM - 1) / OM, longest(p.n_k, FN, OM, p.window), kSimtCost);
+  if (items * s.split_q > 0x7fffffffLL) return FHOB_ERR_SHAPE;
   FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(items * s.split_q), NT, kForwardSmem, s.cluster, st, s, o_out, lse_out, vec));
   return FHOB_OK;
 }
 
 }  // namespace
+
+int simt_grid(const FhobProblem& p, PairGrid* g) {
+  *g = modes_grid(p, true, true);
+  return g->blocks > 0x7fffffffLL ? FHOB_ERR_SHAPE : FHOB_OK;
+}
 
 int simt_backward(const FhobProblem& p, void* dq, void* dk, void* dv, cudaStream_t st) {
   if (p.d > 128 || head_dim_v(p) > 128) return FHOB_ERR_SHAPE;

@@ -111,13 +111,9 @@ __device__ __forceinline__ void bw_body(const BwParams& p, int block) {
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = KSIDE ? p.split_k : p.split_q;
-  int item = block, part = 0;
-  if (split > 1) {
-    item = block / split;
-    part = block - item * split;
-  }
-  const bool live = item < (KSIDE ? p.items_k : p.items_q);   // the grid is padded to whole clusters
-  if (!live) item = 0;
+  const CtaWork work = cta_work(block, split, KSIDE ? p.items_k : p.items_q);   // the grid is padded to whole clusters
+  const int item = work.item, part = work.part;
+  const bool live = work.live;
   const int tiles_per_head = KSIDE ? p.tiles_k : p.tiles_q;
   const int head = item / tiles_per_head;
   const int tile_in_head = item - head * tiles_per_head;
@@ -538,22 +534,18 @@ int bw_launch(const FhobProblem& p, void* dq, void* dk, void* dv, cudaStream_t s
   tp.items_k = tp.tiles_k * p.bh;
   const int st = allow_smem(kernel, kSmem);
   if (st != FHOB_OK) return st;
-  SplitChoice c = {1, 1, true};
-  if (may_split(p.n_q, p.n_k))
-    c = choose_split(kernel, kSmem, SplitWork{tp.items_q, (p.n_k + CQ::BN - 1) / CQ::BN}, SplitWork{tp.items_k, (p.n_q + CK::BN - 1) / CK::BN});
-  auto go = [&](int items_q, int items_k, int cluster) -> int {
-    // whole clusters for either half, so that the parts of an item are neighbours in one cluster
-    auto padded = [&](long long n) { return (n + cluster - 1) / cluster * cluster; };
-    tp.split_q = c.a; tp.split_k = c.b;
-    tp.cluster = cluster;
-    tp.q_blocks = static_cast<int>(padded(static_cast<long long>(items_q) * c.a));
-    const long long blocks = tp.q_blocks + padded(static_cast<long long>(items_k) * c.b);
-    FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(blocks), NTHREADS, kSmem, cluster, s, tp));
+  auto go = [&](bool q_side, bool k_side) -> int {
+    const PairGrid g = pair_grid(q_side ? tp.items_q : 0, tc_parts(p.n_q, p.n_k), k_side ? tp.items_k : 0, tc_parts(p.n_k, p.n_q));
+    if (g.blocks > 0x7fffffffLL) return FHOB_ERR_SHAPE;
+    tp.split_q = g.split_q; tp.split_k = g.split_k;
+    tp.cluster = g.cluster;
+    tp.q_blocks = g.q_blocks;
+    FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(g.blocks), NTHREADS, kSmem, g.cluster, s, tp));
     return FHOB_OK;
   };
-  if (c.together) return go(tp.items_q, tp.items_k, c.a > c.b ? c.a : c.b);
-  const int st1 = go(tp.items_q, 0, c.a);
-  return st1 != FHOB_OK ? st1 : go(0, tp.items_k, c.b);
+  if (!launch_apart(pair_grid(tp.items_q, tc_parts(p.n_q, p.n_k), tp.items_k, tc_parts(p.n_k, p.n_q)))) return go(true, true);
+  const int first = go(true, false);
+  return first != FHOB_OK ? first : go(false, true);
 }
 
 template <bool F16>

@@ -150,6 +150,22 @@ __device__ __forceinline__ float2 exp2_fma(float2 x) {
 // ---- split streamed axis: a cluster of `split` CTAs shares the streamed tiles of one stationary tile
 // and adds up its results through distributed shared memory, in rank order (so bits do not vary).
 
+// What CTA `block` of a kind of CTAs does: part `part` of item `item`, or nothing.
+struct CtaWork {
+  int item, part;
+  bool live;   // false: the CTA only fills up a cluster (item 0 stands in; nothing may be stored)
+};
+__host__ __device__ __forceinline__ CtaWork cta_work(int block, int split, int items) {
+  CtaWork w = {block, 0, true};
+  if (split > 1) {
+    w.item = block / split;
+    w.part = block - w.item * split;
+  }
+  w.live = w.item < items;
+  if (!w.live) w.item = 0;
+  return w;
+}
+
 // Streamed tiles of part `part` of `split` of the range [begin, end).
 __device__ __forceinline__ void split_range(int part, int split, int& begin, int& end) {
   const int n = end - begin, b = begin;
@@ -351,96 +367,67 @@ int allow_smem(K kernel, int bytes) {
   return FHOB_OK;
 }
 
-// How many CTAs share the streamed tiles of an item (a head's 128-row tile), for one or two kinds of
-// item that need not wait for each other.
-struct SplitWork {
-  int items, tiles;   // items of this kind, streamed tiles of the longest one
-};
-struct SplitChoice {
-  int a, b;
-  bool together;   // one launch for both kinds (clusters are of one size in a launch)
-};
-constexpr int kMaxSplit = 8;   // the portable cluster size
-
-// CTAs the device runs at once in clusters of `c` of a kernel that has an SM to itself: clusters do not
-// straddle GPCs, so some SMs stay idle (a B200 with 148 SMs: 132 in clusters of 4 or 6, 120 in clusters
-// of 8).  Asked once per device and host thread.
-template <class K>
-int cluster_slots(K kernel, int smem, int c, int threads = NTHREADS) {
+// SMs of the current device: how many CTAs run at once of a kernel that has an SM to itself.  0: not known.
+int sm_count() {
   constexpr int kDevices = 64;
-  static thread_local int table[kDevices][kMaxSplit + 1] = {};
+  static thread_local int table[kDevices] = {};
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices || c < 1 || c > kMaxSplit) return 0;
-  int& slots = table[dev][c];
-  if (slots == 0) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = c;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.gridDim = dim3(c * 64);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-    slots = n > 0 ? n * c : -1;   // -1: not available
-  }
-  return slots > 0 ? slots : 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return 0;
+  if (table[dev] == 0 && cudaDeviceGetAttribute(&table[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) table[dev] = 0;
+  return table[dev];
 }
 
-// A head whose sequences both have 4096 rows or more is never split: jobs of that size are cut over
-// GPUs by heads, and a head's bits must not depend on which heads it is launched with (the number of
-// parts is a number of partial sums).
-bool may_split(int n_q, int n_k) { return n_q < 4096 || n_k < 4096; }
-
-// Splitting pays while the items leave SMs idle.  Times are in streamed tiles: a CTA takes about `fixed`
-// tiles' time besides its own (launch, prologue, first loads, epilogue: 6 to 9 us against 1 to 1.7 us a
-// tile of the tensor-core kernels), `cluster` more in a cluster (its CTAs start together and meet twice), and
-// a second launch costs `launch`.  Measured with 16 heads, 100 queries, 6000 keys (16 items of 94 tiles, 752 of 2): sweep
-// 102 -> 29 us; passes 3 and 4 205 us in one unsplit launch.
+// How many CTAs of a cluster share the streamed tiles of one stationary tile of a head.  That is also the
+// number of partial sums its results are added up from, so it is worked out from one head alone: the bits
+// of a head must not depend on the heads it is launched with (batches are cut over GPUs and into ranges).
+// Two conditions, because nothing is known of the other heads:
+//  - the head's stationary tiles together take at most one cluster of the portable size, 8 CTAs: a layer
+//    of 16 heads is then still one wave (a B200 runs 132 CTAs at once in clusters of 4, 120 in clusters of 8);
+//  - where there are heads enough to fill the GPU unsplit, the parts cost at most a quarter more.  In
+//    streamed tiles, a CTA takes about `fixed` besides its own (launch, prologue, first loads, epilogue: 6
+//    to 9 us against 1 to 1.7 us a 64-row tile of the tensor-core kernels) and `cluster` more in a cluster (its
+//    CTAs start together and meet twice).
+// Operator, bf16, D = 64, 100 x 6000, us, unsplit / 4 parts / 8: 4 heads 153 / 50 / 38, 16 heads 156 / 95 / 109,
+// 256 heads 959 / 1070 / 1247.
+constexpr int kMaxParts = 8;
 struct SplitCost {
-  float fixed = 5.f, cluster = 1.f, launch = 1.f;
+  float fixed = 5.f, cluster = 1.f;
 };
-template <class K>
-SplitChoice choose_split(K kernel, int smem, const SplitWork& wa, const SplitWork& wb, int threads = NTHREADS,
-                         const SplitCost& cost = SplitCost{}) {
-  SplitChoice best = {1, 1, true};
-  const int sms = cluster_slots(kernel, smem, 1, threads);
-  auto fills = [&](const SplitWork& w) { return w.items == 0 || w.items >= sms; };
-  if (fills(wa) && fills(wb)) return best;
-  auto item_time = [&](const SplitWork& w, int split, int cluster) {
-    return w.items == 0 ? 0.f : (w.tiles + split - 1) / split + cost.fixed + (cluster > 1 ? cost.cluster : 0.f);
-  };
-  auto wave_time = [&](int sa, int sb, int cluster, const SplitWork& a, const SplitWork& b) {
-    const float slots = static_cast<float>(cluster_slots(kernel, smem, cluster, threads));
-    if (slots == 0.f) return 1e30f;
-    const float ta = item_time(a, sa, cluster), tb = item_time(b, sb, cluster), longest = ta > tb ? ta : tb;
-    const float ctas = static_cast<float>(a.items) * sa + static_cast<float>(b.items) * sb;
-    // one wave takes as long as its longest CTA; more CTAs fill the slots as they come free
-    return ctas <= slots ? longest : (a.items * sa * ta + b.items * sb * tb) / slots + 0.5f * longest;
-  };
-  const SplitWork none = {0, 0};
-  float best_time = wave_time(1, 1, 1, wa, wb);
-  for (int sa = 1; sa <= kMaxSplit && (sa == 1 || sa <= wa.tiles); ++sa)
-    for (int sb = 1; sb <= kMaxSplit && (sb == 1 || sb <= wb.tiles); ++sb) {
-      if ((sa > 1 && wa.items == 0) || (sb > 1 && wb.items == 0)) continue;
-      const int most = sa > sb ? sa : sb, least = sa > sb ? sb : sa;
-      if (most % least == 0) {
-        const float t = wave_time(sa, sb, most, wa, wb);
-        if (t < best_time) { best_time = t; best = {sa, sb, true}; }
-      }
-      if (wa.items && wb.items) {
-        const float t = wave_time(sa, 1, sa, wa, none) + wave_time(1, sb, sb, none, wb) + cost.launch;
-        if (t < best_time) { best_time = t; best = {sa, sb, false}; }
-      }
-    }
-  return best;
+inline int split_parts(int stationary_tiles, int streamed_tiles, const SplitCost& cost = SplitCost{}) {
+  const float unsplit = static_cast<float>(streamed_tiles) + cost.fixed;
+  int parts = kMaxParts;
+  while (parts > 1 && (stationary_tiles > kMaxParts / parts ||
+                       static_cast<float>(streamed_tiles) + parts * (cost.fixed + cost.cluster) > 1.25f * unsplit))
+    parts >>= 1;
+  return parts;
 }
+// The tensor-core kernels: 128-row stationary tiles, streamed rows in units of 64.
+inline int tc_parts(int n_stat, int n_strm) { return split_parts((n_stat + BM - 1) / BM, (n_strm + 63) / 64); }
 
 }  // namespace
+
+// Grid of a launch that holds query-tiled and key-tiled CTAs (of which either may have none): the CTAs of
+// an item (a stationary tile of a head) are neighbours in one cluster, and each kind is padded to whole clusters.
+inline PairGrid pair_grid(long long items_q, int split_q, long long items_k, int split_k) {
+  PairGrid g;
+  g.items_q = static_cast<int>(items_q);
+  g.items_k = static_cast<int>(items_k);
+  g.split_q = split_q;
+  g.split_k = split_k;
+  g.cluster = 1;
+  if (items_q > 0 && split_q > g.cluster) g.cluster = split_q;
+  if (items_k > 0 && split_k > g.cluster) g.cluster = split_k;   // both are powers of two
+  auto padded = [&](long long n) { return (n + g.cluster - 1) / g.cluster * g.cluster; };
+  g.q_blocks = static_cast<int>(padded(items_q * split_q));
+  g.blocks = g.q_blocks + padded(items_k * split_k);
+  return g;
+}
+// Clusters of 4 or 8 leave SMs idle that single CTAs would use: an unsplit kind of many CTAs gets a launch of
+// its own.  (us, one launch -> two, operator as above in clusters of 8: 256 heads 1560 -> 1247, 16 heads 109 -> 109,
+// 4 heads 38 -> 48; in clusters of 2, 32 heads 100 x 2000 D = 128, 93 -> 110.)
+inline bool launch_apart(const PairGrid& g) {
+  const int unsplit = g.split_q == 1 ? g.items_q : (g.split_k == 1 ? g.items_k : 0);
+  return g.cluster >= 4 && unsplit > 4 * sm_count();
+}
+
 }  // namespace fhob

@@ -578,17 +578,18 @@ int fw_launch(const FhobProblem& p, void* o_out, float* lse_out, int* status, cu
   tp.heads = (!SPLIT && p.layout) ? p.layout->heads : p.bh;
   tp.d_v = dv;
   tp.scale = p.scale;
-  // Two query tiles a CTA hide each other's latency and share K and V; a tile takes as long alone, so
-  // when single tiles fit the GPU at once, a CTA has one (and the keys are split if that leaves SMs idle).
   const int tiles = (p.n_q + BM - 1) / BM;
   if (static_cast<long long>(tiles) * p.bh > 0x7fffffffLL) return FHOB_ERR_SHAPE;
-  tp.q_tiles = static_cast<long long>(tiles) * p.bh <= cluster_slots(kernel, C::SMEM_BYTES, 1) ? 1 : 2;
+  // A head of one query tile may split its keys (a second tile would cost the parts more than they save).
+  tp.split = tiles == 1 ? tc_parts(p.n_q, p.n_k) : 1;
+  // Two query tiles a CTA hide each other's latency and share K and V; a tile takes as long alone, so
+  // when single tiles fit the GPU at once, a CTA has one.  (The bits are the same.)
+  tp.q_tiles = tiles == 1 || static_cast<long long>(tiles) * p.bh <= sm_count() ? 1 : 2;
   tp.groups = (tiles + tp.q_tiles - 1) / tp.q_tiles;
   tp.items = tp.groups * p.bh;
-  tp.split = 1;
-  if (tp.q_tiles == 1 && may_split(p.n_q, p.n_k))
-    tp.split = choose_split(kernel, C::SMEM_BYTES, SplitWork{tp.items, (p.n_k + C::BN - 1) / C::BN}, SplitWork{0, 0}).a;
-  FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(tp.items * tp.split), FW_THREADS, C::SMEM_BYTES, tp.split, s, tp));
+  const long long blocks = static_cast<long long>(tp.items) * tp.split;
+  if (blocks > 0x7fffffffLL) return FHOB_ERR_SHAPE;
+  FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(blocks), FW_THREADS, C::SMEM_BYTES, tp.split, s, tp));
   return FHOB_OK;
 }
 

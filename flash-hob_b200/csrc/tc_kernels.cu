@@ -421,7 +421,7 @@ __device__ __forceinline__ float row_dot(const void* o, const void* d_o, int c0,
 }
 
 // One pass over one 128-row tile of one head; `block` numbers the (head, tile, part) triples of the pass.
-// With few tiles the streamed axis is split over the CTAs of a cluster (see choose_split); each computes its
+// With few tiles a head the streamed axis is split over the CTAs of a cluster (see split_parts); each computes its
 // part's sums and the cluster adds them up.
 template <int PASS, int DQK, int DV, int BN, int FUSED, bool F16, bool SPLIT>
 __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
@@ -441,13 +441,9 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_per_head = kQStat ? p.tiles_q : p.tiles_k;
   const int split = kQStat ? p.split_q : p.split_k;
-  int item = block, part = 0;
-  if (split > 1) {
-    item = block / split;
-    part = block - item * split;
-  }
-  const bool live = item < (kQStat ? p.items_q : p.items_k);   // the grid is padded to whole clusters
-  if (!live) item = 0;
+  const CtaWork work = cta_work(block, split, kQStat ? p.items_q : p.items_k);   // the grid is padded to whole clusters
+  const int item = work.item, part = work.part;
+  const bool live = work.live;
   const int head = item / tiles_per_head;
   const int tile_in_head = item - head * tiles_per_head;
   // causal: longest tiles first (late queries in passes 1-3, early keys in pass 4)
@@ -1058,10 +1054,13 @@ int first_live_query(const FhobProblem& p) {
   return (p.causal && p.n_q > p.n_k) ? p.n_q - p.n_k : 0;
 }
 
+bool tc_items_fit(const FhobProblem& p) {   // both passes together stay below 2^31 items
+  return (static_cast<long long>(p.n_q > p.n_k ? p.n_q : p.n_k) + BM - 1) / BM * p.bh <= 0x3fffffffLL;
+}
+
 template <bool F16, bool SPLIT>
 int fill_params(const FhobProblem& p, TcParams& tp) {
-  const long long most_items = static_cast<long long>((p.n_q > p.n_k ? p.n_q : p.n_k) + BM - 1) / BM * p.bh;
-  if (most_items > 0x3fffffffLL) return FHOB_ERR_SHAPE;   // both passes together stay below 2^31 CTAs
+  if (!tc_items_fit(p)) return FHOB_ERR_SHAPE;
   RowVectors rv = row_vectors(p);
   const void* mats[kMaps] = {p.q, p.ddq, p.d_o, p.k, p.ddk, p.v, p.ddv};
   const int ids[kMaps] = {kTenQ, kTenDDQ, kTenDO, kTenK, kTenDDK, kTenV, kTenDDV};
@@ -1106,6 +1105,7 @@ int fill_params(const FhobProblem& p, TcParams& tp) {
 
 template <class K>
 int launch(K kernel, const TcParams& tp, long long blocks, int smem, cudaStream_t s) {
+  if (blocks > 0x7fffffffLL) return FHOB_ERR_SHAPE;
   const int st = allow_smem(kernel, smem);
   if (st != FHOB_OK) return st;
   FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(blocks), NTHREADS, smem, tp.cluster, s, tp));
@@ -1116,11 +1116,7 @@ template <int PASS, int DQK, int DV, int BN, int FUSED, bool F16, bool SPLIT>
 int launch_pass(TcParams& tp, cudaStream_t s) {
   constexpr auto kernel = tc_pass_kernel<PASS, DQK, DV, BN, FUSED, F16, SPLIT>;
   constexpr int kSmem = Cfg<PASS, DQK, DV, BN>::SMEM_BYTES;
-  if (FUSED && may_split(tp.n_q, tp.n_k)) {
-    const int st = allow_smem(kernel, kSmem);
-    if (st != FHOB_OK) return st;
-    tp.split_q = tp.cluster = choose_split(kernel, kSmem, SplitWork{tp.items_q, (tp.n_k + BN - 1) / BN}, SplitWork{0, 0}).a;
-  }
+  if (FUSED) tp.split_q = tp.cluster = tc_parts(tp.n_q, tp.n_k);
   return launch(kernel, tp, static_cast<long long>(tp.items_q) * tp.split_q, kSmem, s);
 }
 
@@ -1130,24 +1126,15 @@ int launch_34(TcParams& tp, bool pass3, bool pass4, cudaStream_t s) {
   constexpr auto kernel = tc_pass34_kernel<DQK, DV, F16, SPLIT>;
   constexpr int kSmem3 = Cfg<3, DQK, DV, 64>::SMEM_BYTES, kSmem4 = Cfg<4, DQK, DV, 64>::SMEM_BYTES;
   constexpr int kSmem = kSmem3 > kSmem4 ? kSmem3 : kSmem4;
-  const SplitWork w3 = {pass3 ? tp.items_q : 0, (tp.n_k + 63) / 64}, w4 = {pass4 ? tp.items_k : 0, (tp.n_q + 63) / 64};
-  SplitChoice c = {1, 1, true};
-  if (may_split(tp.n_q, tp.n_k)) {
-    const int st = allow_smem(kernel, kSmem);
-    if (st != FHOB_OK) return st;
-    c = choose_split(kernel, kSmem, w3, w4);
+  const PairGrid g = pair_grid(pass3 ? tp.items_q : 0, tc_parts(tp.n_q, tp.n_k), pass4 ? tp.items_k : 0, tc_parts(tp.n_k, tp.n_q));
+  if (pass3 && pass4 && launch_apart(g)) {
+    const int st = launch_34<DQK, DV, F16, SPLIT>(tp, true, false, s);
+    return st != FHOB_OK ? st : launch_34<DQK, DV, F16, SPLIT>(tp, false, true, s);
   }
-  auto go = [&](int items3, int items4, int cluster) {
-    // whole clusters for either pass, so that the parts of an item are neighbours in one cluster
-    auto padded = [&](long long n) { return (n + cluster - 1) / cluster * cluster; };
-    tp.split_q = c.a; tp.split_k = c.b;
-    tp.cluster = cluster;
-    tp.q_blocks = static_cast<int>(padded(static_cast<long long>(items3) * c.a));
-    return launch(kernel, tp, tp.q_blocks + padded(static_cast<long long>(items4) * c.b), kSmem, s);
-  };
-  if (c.together) return go(w3.items, w4.items, c.a > c.b ? c.a : c.b);
-  const int st = go(w3.items, 0, c.a);
-  return st != FHOB_OK ? st : go(0, w4.items, c.b);
+  tp.split_q = g.split_q; tp.split_k = g.split_k;
+  tp.cluster = g.cluster;
+  tp.q_blocks = g.q_blocks;
+  return launch(kernel, tp, g.blocks, kSmem, s);
 }
 
 // `pass`: 1, 2, 3, 4 alone, 12 = passes 1 and 2 in one sweep, kWholeOperator = the sweep, then passes 3 and 4
@@ -1232,6 +1219,13 @@ int tc_split_inputs(const FhobProblem& p, cudaStream_t s, int which) {
   if (blocks > 0x7fffffffL) return FHOB_ERR_SHAPE;
   FHOB_CUDA_OK(launch_pdl(split_rows_kernel, dim3(static_cast<unsigned>(blocks), count), 256, 0, 1, s, jobs));
   return FHOB_OK;
+}
+
+int tc_grid(const FhobProblem& p, PairGrid* g) {
+  if (!tc_items_fit(p)) return FHOB_ERR_SHAPE;
+  const int tq = (p.n_q + BM - 1) / BM, tk = (p.n_k + BM - 1) / BM;
+  *g = pair_grid(tq * p.bh, tc_parts(p.n_q, p.n_k), tk * p.bh, tc_parts(p.n_k, p.n_q));
+  return g->blocks > 0x7fffffffLL ? FHOB_ERR_SHAPE : FHOB_OK;
 }
 
 int tc_pass(int pass, const FhobProblem& p, cudaStream_t s) {

@@ -17,7 +17,7 @@ SYMBOLS = (
     "fhob_prepass", "fhob_pass1", "fhob_pass2", "fhob_pass12", "fhob_pass3", "fhob_pass4", "fhob_row_stats",
     "fhob_read_status", "fhob_forward", "fhob_backward", "fhob_bwdbwd_static_scratch",
     "fhob_selftest_expired_wait", "fhob_visible_tiles", "fhob_static_scratch_status",
-    "fhob_workspace_bytes_problem",
+    "fhob_workspace_bytes_problem", "fhob_cta_work",
 )
 STATIC_SCRATCH_MAX_ROWS = 262144
 
@@ -77,6 +77,8 @@ def load() -> C.CDLL:
     lib.fhob_backward.argtypes = [P, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
     lib.fhob_visible_tiles.restype = C.c_int
     lib.fhob_visible_tiles.argtypes = [C.c_int] * 8 + [C.POINTER(C.c_int), C.POINTER(C.c_int)]
+    lib.fhob_cta_work.restype = C.c_int
+    lib.fhob_cta_work.argtypes = [P, C.c_int64] + [C.POINTER(C.c_int32)] * 4
     lib.fhob_selftest_expired_wait.restype = C.c_int
     lib.fhob_selftest_expired_wait.argtypes = [C.c_void_p, C.c_size_t, C.c_void_p]
     lib.fhob_static_scratch_status.restype = C.c_int

@@ -222,6 +222,16 @@ int fhob_visible_tiles(int q_stationary, int m0, int rows, int tile, int n_q, in
                        int* t_begin, int* t_end);
 
 /*
+ * The CTA-to-work rule of passes 3 and 4 in one launch (host evaluation, no GPU
+ * needed): CTA `block` works for pass *pass (3 query-tiled, 4 key-tiled, 0 = it only fills up a cluster) on
+ * part *part of *parts of item *item; the items of a pass are the (head, stationary tile) pairs, and the
+ * streamed tiles of one are cut into *parts, a number that depends on n_q, n_k, window and the kernel family
+ * alone.  FHOB_ERR_ARG for a block beyond the grid.  Reads the sizes of the problem, impl, dtype and the
+ * workspace, no pointers.  Exposed so that the rule can be checked exhaustively; the reference has no counterpart.
+ */
+int fhob_cta_work(const FhobProblem* p, int64_t block, int32_t* pass, int32_t* item, int32_t* part, int32_t* parts);
+
+/*
  * Self-test of the bounded device waits.  Queues one warp whose only wait is
  * on an mbarrier nothing ever arrives on; after about a second the wait gives
  * up, ORs FHOB_ERR_TIMEOUT into the status word at the start of `workspace`

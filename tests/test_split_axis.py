@@ -1,6 +1,8 @@
 """Problems with few 128-row tiles: the streamed axis is split over the CTAs of a cluster."""
 from __future__ import annotations
 
+import ctypes as C
+
 import pytest
 import torch
 
@@ -11,8 +13,8 @@ from oracle import attn_oracle as O
 # one item of one tile to many items; parts of unequal length; more parts than one pass has tiles for
 SHAPES = [(1, 1, 64), (1, 100, 130), (1, 129, 700), (3, 100, 1000), (1, 1, 4096), (5, 300, 64), (3, 640, 3000), (16, 100, 6000)]
 # Passes 3 and 4 in one launch of clusters, one of them split and the other not, with a number of items of
-# the other that leaves a cluster with CTAs that have no item (47 key tiles a head in clusters of 8, ...)
-PADDED = [(3, 100, 6000), (4, 100, 6000), (2, 640, 6000), (5, 100, 4000), (3, 6000, 100), (4, 4000, 100)]
+# the other that leaves a cluster with CTAs that have no item (3 x 47 key tiles in clusters of 4, 3 x 17 in clusters of 2, ...)
+PADDED = [(3, 100, 6000), (3, 100, 2100), (1, 200, 11000), (3, 6000, 100), (3, 2100, 100), (1, 11000, 200)]
 
 
 @pytest.mark.gpu
@@ -37,3 +39,76 @@ def test_split_matches_oracle(bh, nq, nk, dtype, d, tol):
         grads = fhob.attention_backward(x["q"], x["k"], x["v"], o, x["do"], lse, scale, is_causal=causal)
         for n, g, r in zip(("dq", "dk", "dv"), grads, O.attn_bwd(ref[0], ref[1], ref[2], ref[3], scale, causal)):
             assert O.rel_err(g.cpu(), r) < tol, (n, causal)
+
+
+# one to many tiles a head on either side, with and without parts; windows; both families of kernels
+INVARIANT = [(9, 100, 3000, False, None), (9, 2048, 2048, True, None), (8, 1024, 1024, False, None), (7, 300, 300, True, 64),
+             (16, 100, 6000, True, 700), (6, 640, 3000, False, None), (12, 64, 1500, True, None), (5, 3000, 100, False, None)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 64), (torch.bfloat16, 128), (torch.float32, 64), (torch.float32, 96)])
+@pytest.mark.parametrize("bh,nq,nk,causal,window", INVARIANT)
+def test_bits_of_a_head_do_not_depend_on_the_heads_it_is_launched_with(bh, nq, nk, causal, window, dtype, d):
+    import fhob
+    x = make_inputs(bh, nq, nk, d, seed=nq + nk, dtype=dtype, device="cuda")
+    kw = dict(is_causal=causal, sliding_window=window)
+
+    def calls(lo, hi):
+        t = {n: v[lo:hi].contiguous() for n, v in x.items()}
+        o, lse = fhob.attention_forward(t["q"], t["k"], t["v"], 0.1, **kw)
+        alone = fhob.produce_L(t["q"], t["k"], causal, 0.1, window)
+        first = fhob.attention_backward(t["q"], t["k"], t["v"], o, t["do"], lse, 0.1, **kw)
+        second = fhob.flash_bwdbwd(t["q"], t["k"], t["v"], o, t["do"], t["ddq"], t["ddk"], t["ddv"], lse, 0.1, **kw)
+        return (o, lse, alone, *first, *second)
+
+    whole = calls(0, bh)
+    for lo, hi in ((0, 1), (bh - 2, bh)):
+        for n, a, b in zip(("o", "lse", "L", "dq", "dk", "dv", "dq2", "dk2", "dv2", "ddo"), whole, calls(lo, hi)):
+            assert torch.equal(a[lo:hi], b), (n, lo)
+
+
+def _ctas(family, bh, nq, nk, window=0):
+    """What the CTAs of the launch of passes 3 and 4 do: [(pass, item, part, parts)] in grid order."""
+    from fhob import _lib
+    lib = _lib.load()
+    p = _lib.FhobProblem()
+    p.bh, p.n_q, p.n_k, p.d, p.causal, p.window = bh, nq, nk, 64, int(window > 0), window
+    p.dtype, p.impl = _lib.FHOB_BF16, _lib.IMPL[family]
+    out = [C.c_int32() for _ in range(4)]
+    ctas = []
+    while lib.fhob_cta_work(C.byref(p), len(ctas), *(C.byref(x) for x in out)) == 0:
+        ctas.append(tuple(x.value for x in out))
+    return ctas
+
+
+WALK = [(bh, nq, nk) for bh in (1, 2, 3, 5, 7) for nq, nk in
+        [(1, 1), (64, 64), (100, 6000), (6000, 100), (640, 6000), (129, 700), (300, 3000), (500, 2000), (3000, 513), (256, 256), (513, 8192)]]
+
+
+@pytest.mark.parametrize("family,rows", [("tcgen05", 128), ("simt", 64)])
+@pytest.mark.parametrize("bh,nq,nk", WALK)
+def test_every_part_of_every_tile_has_one_cta(family, rows, bh, nq, nk):
+    ctas = _ctas(family, bh, nq, nk)
+    parts = {}
+    for kind, n in ((3, nq), (4, nk)):
+        mine = [c for c in ctas if c[0] == kind]
+        split = {c[3] for c in mine}
+        assert len(split) == 1
+        parts[kind] = split.pop()
+        assert sorted((c[1], c[2]) for c in mine) == [(i, s) for i in range(bh * -(-n // rows)) for s in range(parts[kind])]
+    cluster = max(parts.values())
+    assert cluster <= 8 and len(ctas) % cluster == 0
+    for i, c in enumerate(ctas):   # the parts of an item are neighbours in one cluster, in order
+        if c[0] and c[2]:
+            assert i % cluster and ctas[i - 1][:3] == (c[0], c[1], c[2] - 1)
+    alone = _ctas(family, 1, nq, nk)
+    assert {c[0]: c[3] for c in alone if c[0]} == parts   # a head's own
+
+
+def test_some_walked_shapes_have_idle_ctas_beside_an_unsplit_pass():
+    hit = 0
+    for bh, nq, nk in WALK:
+        ctas = _ctas("tcgen05", bh, nq, nk)
+        hit += any(c[0] == 0 and c[3] == 1 for c in ctas)
+    assert hit >= 3
