@@ -710,13 +710,6 @@ SimtParams make_params(const FhobProblem& p) {
   return s;
 }
 
-// Streamed tiles of `tile` rows that the longest item of `rows` stationary rows sees.
-inline int longest(int n, int tile, int rows, int window) {
-  const int all = (n + tile - 1) / tile;
-  const long long seen = window > 0 ? (static_cast<long long>(rows) + window - 2) / tile + 2 : all;
-  return seen < all ? static_cast<int>(seen) : all;
-}
-
 // In streamed tiles (fp32, D = 128: 12 us in passes 3 and 4): what a CTA takes besides its tiles is about one
 // tile's time, meeting in a cluster about half of one.  Operator, fp32, D = 128, us, unsplit -> split: 1 head
 // 64 x 3000 2497 -> 332, 4 heads 200 x 5000 4156 -> 2118; 64 heads 200 x 1000 2390 -> 2411.

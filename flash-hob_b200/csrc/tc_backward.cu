@@ -535,7 +535,7 @@ int bw_launch(const FhobProblem& p, void* dq, void* dk, void* dv, cudaStream_t s
   const int st = allow_smem(kernel, kSmem);
   if (st != FHOB_OK) return st;
   auto go = [&](bool q_side, bool k_side) -> int {
-    const PairGrid g = pair_grid(q_side ? tp.items_q : 0, tc_parts(p.n_q, p.n_k), k_side ? tp.items_k : 0, tc_parts(p.n_k, p.n_q));
+    const PairGrid g = pair_grid(q_side ? tp.items_q : 0, tc_parts(p.n_q, p.n_k, p.window), k_side ? tp.items_k : 0, tc_parts(p.n_k, p.n_q, p.window));
     if (g.blocks > 0x7fffffffLL) return FHOB_ERR_SHAPE;
     tp.split_q = g.split_q; tp.split_k = g.split_k;
     tp.cluster = g.cluster;
@@ -543,7 +543,7 @@ int bw_launch(const FhobProblem& p, void* dq, void* dk, void* dv, cudaStream_t s
     FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(g.blocks), NTHREADS, kSmem, g.cluster, s, tp));
     return FHOB_OK;
   };
-  if (!launch_apart(pair_grid(tp.items_q, tc_parts(p.n_q, p.n_k), tp.items_k, tc_parts(p.n_k, p.n_q)))) return go(true, true);
+  if (!launch_apart(pair_grid(tp.items_q, tc_parts(p.n_q, p.n_k, p.window), tp.items_k, tc_parts(p.n_k, p.n_q, p.window)))) return go(true, true);
   const int first = go(true, false);
   return first != FHOB_OK ? first : go(false, true);
 }

@@ -401,8 +401,15 @@ inline int split_parts(int stationary_tiles, int streamed_tiles, const SplitCost
     parts >>= 1;
   return parts;
 }
+// Streamed tiles of `tile` rows that the longest item of `rows` stationary rows sees.
+inline int longest(int n, int tile, int rows, int window) {
+  const int all = (n + tile - 1) / tile;
+  const long long seen = window > 0 ? (static_cast<long long>(rows) + window - 2) / tile + 2 : all;
+  return seen < all ? static_cast<int>(seen) : all;
+}
+
 // The tensor-core kernels: 128-row stationary tiles, streamed rows in units of 64.
-inline int tc_parts(int n_stat, int n_strm) { return split_parts((n_stat + BM - 1) / BM, (n_strm + 63) / 64); }
+inline int tc_parts(int n_stat, int n_strm, int window) { return split_parts((n_stat + BM - 1) / BM, longest(n_strm, 64, BM, window)); }
 
 }  // namespace
 

@@ -581,7 +581,7 @@ int fw_launch(const FhobProblem& p, void* o_out, float* lse_out, int* status, cu
   const int tiles = (p.n_q + BM - 1) / BM;
   if (static_cast<long long>(tiles) * p.bh > 0x7fffffffLL) return FHOB_ERR_SHAPE;
   // A head of one query tile may split its keys (a second tile would cost the parts more than they save).
-  tp.split = tiles == 1 ? tc_parts(p.n_q, p.n_k) : 1;
+  tp.split = tiles == 1 ? tc_parts(p.n_q, p.n_k, p.window) : 1;
   // Two query tiles a CTA hide each other's latency and share K and V; a tile takes as long alone, so
   // when single tiles fit the GPU at once, a CTA has one.  (The bits are the same.)
   tp.q_tiles = tiles == 1 || static_cast<long long>(tiles) * p.bh <= sm_count() ? 1 : 2;

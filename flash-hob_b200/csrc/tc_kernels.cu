@@ -1116,7 +1116,7 @@ template <int PASS, int DQK, int DV, int BN, int FUSED, bool F16, bool SPLIT>
 int launch_pass(TcParams& tp, cudaStream_t s) {
   constexpr auto kernel = tc_pass_kernel<PASS, DQK, DV, BN, FUSED, F16, SPLIT>;
   constexpr int kSmem = Cfg<PASS, DQK, DV, BN>::SMEM_BYTES;
-  if (FUSED) tp.split_q = tp.cluster = tc_parts(tp.n_q, tp.n_k);
+  if (FUSED) tp.split_q = tp.cluster = tc_parts(tp.n_q, tp.n_k, tp.window);
   return launch(kernel, tp, static_cast<long long>(tp.items_q) * tp.split_q, kSmem, s);
 }
 
@@ -1126,7 +1126,7 @@ int launch_34(TcParams& tp, bool pass3, bool pass4, cudaStream_t s) {
   constexpr auto kernel = tc_pass34_kernel<DQK, DV, F16, SPLIT>;
   constexpr int kSmem3 = Cfg<3, DQK, DV, 64>::SMEM_BYTES, kSmem4 = Cfg<4, DQK, DV, 64>::SMEM_BYTES;
   constexpr int kSmem = kSmem3 > kSmem4 ? kSmem3 : kSmem4;
-  const PairGrid g = pair_grid(pass3 ? tp.items_q : 0, tc_parts(tp.n_q, tp.n_k), pass4 ? tp.items_k : 0, tc_parts(tp.n_k, tp.n_q));
+  const PairGrid g = pair_grid(pass3 ? tp.items_q : 0, tc_parts(tp.n_q, tp.n_k, tp.window), pass4 ? tp.items_k : 0, tc_parts(tp.n_k, tp.n_q, tp.window));
   if (pass3 && pass4 && launch_apart(g)) {
     const int st = launch_34<DQK, DV, F16, SPLIT>(tp, true, false, s);
     return st != FHOB_OK ? st : launch_34<DQK, DV, F16, SPLIT>(tp, false, true, s);
@@ -1224,7 +1224,7 @@ int tc_split_inputs(const FhobProblem& p, cudaStream_t s, int which) {
 int tc_grid(const FhobProblem& p, PairGrid* g) {
   if (!tc_items_fit(p)) return FHOB_ERR_SHAPE;
   const int tq = (p.n_q + BM - 1) / BM, tk = (p.n_k + BM - 1) / BM;
-  *g = pair_grid(tq * p.bh, tc_parts(p.n_q, p.n_k), tk * p.bh, tc_parts(p.n_k, p.n_q));
+  *g = pair_grid(tq * p.bh, tc_parts(p.n_q, p.n_k, p.window), tk * p.bh, tc_parts(p.n_k, p.n_q, p.window));
   return g->blocks > 0x7fffffffLL ? FHOB_ERR_SHAPE : FHOB_OK;
 }
 

@@ -41,6 +41,25 @@ def test_split_matches_oracle(bh, nq, nk, dtype, d, tol):
             assert O.rel_err(g.cpu(), r) < tol, (n, causal)
 
 
+# one head and two; a window of a few tiles of a long sequence (not split), one of half of it (two parts)
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,d,tol", [(torch.bfloat16, 64, 2e-2), (torch.bfloat16, 128, 2e-2), (torch.float32, 64, 1e-4), (torch.float32, 96, 1e-4)])
+@pytest.mark.parametrize("bh,nq,nk,window", [(1, 100, 6000, 64), (2, 100, 8000, 4000), (1, 3000, 3000, 64)])
+def test_split_with_a_window_matches_oracle(bh, nq, nk, window, dtype, d, tol):
+    import fhob
+    x = make_inputs(bh, nq, nk, d, seed=nq + nk, dtype=dtype, device="cuda")
+    ref = [t.double().cpu() for t in x.values()]
+    kw = dict(is_causal=True, sliding_window=window)
+    o, lse = fhob.attention_forward(x["q"], x["k"], x["v"], 0.1, **kw, check=True)
+    assert O.rel_err(o.cpu(), O.attn_fwd(*ref[:3], 0.1, True, window)) < tol
+    got = fhob.flash_bwdbwd(x["q"], x["k"], x["v"], o, x["do"], x["ddq"], x["ddk"], x["ddv"], lse, 0.1, **kw, check=True)
+    for n, g, r in zip(("dq2", "dk2", "dv2", "ddo"), got, O.bwdbwd_closed_form(*ref, 0.1, True, sliding_window_length=window)):
+        assert O.rel_err(g.cpu(), r) < tol, n
+    grads = fhob.attention_backward(x["q"], x["k"], x["v"], o, x["do"], lse, 0.1, **kw)
+    for n, g, r in zip(("dq", "dk", "dv"), grads, O.attn_bwd(*ref[:4], 0.1, True, window)):
+        assert O.rel_err(g.cpu(), r) < tol, n
+
+
 # one to many tiles a head on either side, with and without parts; windows; both families of kernels
 INVARIANT = [(9, 100, 3000, False, None), (9, 2048, 2048, True, None), (8, 1024, 1024, False, None), (7, 300, 300, True, 64),
              (16, 100, 6000, True, 700), (6, 640, 3000, False, None), (12, 64, 1500, True, None), (5, 3000, 100, False, None)]
@@ -112,3 +131,12 @@ def test_some_walked_shapes_have_idle_ctas_beside_an_unsplit_pass():
         ctas = _ctas("tcgen05", bh, nq, nk)
         hit += any(c[0] == 0 and c[3] == 1 for c in ctas)
     assert hit >= 3
+
+
+@pytest.mark.parametrize("family", ("tcgen05", "simt"))
+def test_a_window_bounds_the_number_of_parts(family):
+    """Parts are of the tiles an item sees: a window of a few tiles leaves nothing to split."""
+    def parts(window):
+        return {c[0]: c[3] for c in _ctas(family, 1, 100, 8000, window)}[3]
+    assert parts(0) > 1 and parts(64) == 1
+    assert 1 < parts(4000) <= parts(0) and parts(8000) == parts(0)
