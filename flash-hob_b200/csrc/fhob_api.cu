@@ -370,17 +370,16 @@ int fhob_forward(const FhobProblem* p, void* o_out, float* lse_out, void* stream
     if (!layout_ok(l, mats, 3, p->dtype == FHOB_F32 ? 4 : 2)) return FHOB_ERR_ALIGN;
   }
   if (p->impl == FHOB_IMPL_TCGEN05 && !tc_ok) return FHOB_ERR_SHAPE;
-  if (p->impl != FHOB_IMPL_SIMT && tc_ok) {
-    int* status = static_cast<int*>(p->workspace);
-    if (status) {
-      if ((reinterpret_cast<uintptr_t>(p->workspace) & 255u) || p->workspace_bytes < sizeof(int)) return FHOB_ERR_WORKSPACE;
-    } else {
-      int st = own_status_word(&status);
-      if (st != FHOB_OK) return st;
-    }
-    return tc_forward(*p, o_out, lse_out, status, s);
+  const bool tc = p->impl != FHOB_IMPL_SIMT && tc_ok;
+  int* status = static_cast<int*>(p->workspace);
+  if (!status) {
+    int st = own_status_word(&status);
+    if (st != FHOB_OK) return st;
+  } else if ((reinterpret_cast<uintptr_t>(p->workspace) & 255u) || p->workspace_bytes < sizeof(int)) {
+    if (tc) return FHOB_ERR_WORKSPACE;
+    status = nullptr;   // the CUDA-core kernel only clears the word: it does without one
   }
-  return simt_forward(*p, o_out, lse_out, s);
+  return tc ? tc_forward(*p, o_out, lse_out, status, s) : simt_forward(*p, o_out, lse_out, status, s);
 }
 
 int fhob_backward(const FhobProblem* p, void* dq, void* dk, void* dv, void* stream) {

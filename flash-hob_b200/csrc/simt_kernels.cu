@@ -526,9 +526,12 @@ __device__ __forceinline__ void loads_commit() { asm volatile("cp.async.commit_g
 __device__ __forceinline__ void loads_landed_but_last() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 template <typename T>
-__global__ void __launch_bounds__(NT, 1) simt_forward_kernel(const __grid_constant__ SimtParams p, void* o_out, float* lse_out, bool vec) {
+__global__ void __launch_bounds__(NT, 1) simt_forward_kernel(const __grid_constant__ SimtParams p, void* o_out, float* lse_out, int* status, bool vec) {
   pdl_wait();
-  if (threadIdx.x == 0) pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    pdl_launch_dependents();
+    if (blockIdx.x == 0 && status) *status = 0;   // every call starts clean
+  }
   extern __shared__ float smem[];
   float *qs = smem, *ks = qs + OM * OP, *vs = ks + FN * OP, *ps = vs + FN * OP;   // ps: [key][query]
   const int d = p.d, dv = p.dv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -761,7 +764,7 @@ int launch_backward(const FhobProblem& p, void* dq, void* dk, void* dv, cudaStre
 
 // The forward reads rows element by element if they are not whole, aligned 16-byte pieces.
 template <typename T>
-int launch_forward(const FhobProblem& p, void* o_out, float* lse_out, cudaStream_t st) {
+int launch_forward(const FhobProblem& p, void* o_out, float* lse_out, int* status, cudaStream_t st) {
   constexpr auto kernel = simt_forward_kernel<T>;
   const int ok = allow_smem(kernel, kForwardSmem);
   if (ok != FHOB_OK) return ok;
@@ -773,7 +776,7 @@ int launch_forward(const FhobProblem& p, void* o_out, float* lse_out, cudaStream
   s.items_q = static_cast<int>(items);
   s.split_q = s.cluster = split_parts((p.n_q + OM - 1) / OM, longest(p.n_k, FN, OM, p.window), kSimtCost);
   if (items * s.split_q > 0x7fffffffLL) return FHOB_ERR_SHAPE;
-  FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(items * s.split_q), NT, kForwardSmem, s.cluster, st, s, o_out, lse_out, vec));
+  FHOB_CUDA_OK(launch_pdl(kernel, static_cast<unsigned>(items * s.split_q), NT, kForwardSmem, s.cluster, st, s, o_out, lse_out, status, vec));
   return FHOB_OK;
 }
 
@@ -798,11 +801,11 @@ int simt_pass(int pass, const FhobProblem& p, cudaStream_t st) {
   return dispatch_pass<__nv_bfloat16>(pass, p, st);
 }
 
-int simt_forward(const FhobProblem& p, void* o_out, float* lse_out, cudaStream_t st) {
+int simt_forward(const FhobProblem& p, void* o_out, float* lse_out, int* status, cudaStream_t st) {
   if (p.d > 128 || head_dim_v(p) > 128) return FHOB_ERR_SHAPE;
-  if (p.dtype == FHOB_F32) return launch_forward<float>(p, o_out, lse_out, st);
-  if (p.dtype == FHOB_F16) return launch_forward<__half>(p, o_out, lse_out, st);
-  return launch_forward<__nv_bfloat16>(p, o_out, lse_out, st);
+  if (p.dtype == FHOB_F32) return launch_forward<float>(p, o_out, lse_out, status, st);
+  if (p.dtype == FHOB_F16) return launch_forward<__half>(p, o_out, lse_out, status, st);
+  return launch_forward<__nv_bfloat16>(p, o_out, lse_out, status, st);
 }
 
 }  // namespace fhob

@@ -102,3 +102,29 @@ def test_forward_matches_oracle(bh, nq, nk, d, dv, causal, window):
         if need_o:
             assert O.rel_err(o[:, dead:], O.attn_fwd(ql, k.double(), v.double(), scale, causal, w)) < 1e-5
             assert (o[:, :dead] == 0).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("impl,dtype,d", [("auto", "fp32", 128), ("simt", "bf16", 64), ("auto", "bf16", 64), ("auto", "fp32", 64)])
+def test_forward_clears_the_status_word(impl, dtype, d):
+    """Whatever the workspace held before the call; both families of kernels."""
+    import ctypes as C
+    from fhob import _lib
+    lib = _lib.load()
+    t = {"fp32": torch.float32, "bf16": torch.bfloat16}[dtype]
+    q, k, v, o = (torch.randn(2, n, d, device="cuda").to(t) for n in (70, 90, 90, 70))
+    lse = torch.empty(2, 70, device="cuda")
+    p = _lib.FhobProblem()
+    p.bh, p.n_q, p.n_k, p.d, p.scale, p.impl = 2, 70, 90, d, 0.1, _lib.IMPL[impl]
+    p.dtype = {"fp32": _lib.FHOB_F32, "bf16": _lib.FHOB_BF16}[dtype]
+    p.q, p.k, p.v = q.data_ptr(), k.data_ptr(), v.data_ptr()
+    ws = torch.full((lib.fhob_workspace_bytes_problem(C.byref(p)),), 255, dtype=torch.uint8, device="cuda")
+    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert lib.fhob_forward(C.byref(p), C.c_void_p(o.data_ptr()), C.c_void_p(lse.data_ptr()), s) == 0
+    assert lib.fhob_read_status(C.byref(p), s) == 0
+    ws.fill_(255)   # the CUDA-core kernels never needed a workspace that would do for the others
+    if impl == "simt":
+        p.workspace = ws.data_ptr() + 8
+        assert lib.fhob_forward(C.byref(p), C.c_void_p(o.data_ptr()), C.c_void_p(lse.data_ptr()), s) == 0
+        assert (ws == 255).all()
