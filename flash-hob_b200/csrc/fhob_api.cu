@@ -116,6 +116,16 @@ int own_status_word(int** out) {
   return FHOB_OK;
 }
 
+// Held while a call queues its kernels, which hand results to one another through the workspace: host threads
+// that share a stream may share a workspace, and then one call's kernels must not come between another's.
+// Workspaces at different addresses seldom share a lock, so a full launch queue holds up its own users.
+std::mutex& workspace_lock(const void* workspace) {
+  constexpr unsigned kLocks = 64;
+  static std::mutex locks[kLocks];
+  const uintptr_t a = reinterpret_cast<uintptr_t>(workspace) >> 8;
+  return locks[(a ^ (a >> 12)) % kLocks];
+}
+
 // strides of the first `count` matrices of a layout (those given): positive rows, everything 16-byte aligned
 bool layout_ok(const FhobLayout& l, const void* const* mats, int count, size_t es) {
   const long long align = 16 / static_cast<long long>(es);
@@ -284,6 +294,7 @@ int fhob_bwdbwd(const FhobProblem* p, void* stream) {
   int st = validate(p, true, true, true);
   if (st != FHOB_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  std::lock_guard<std::mutex> together(workspace_lock(p->workspace));
   // tensor cores: dd and b come out of one sweep (sum_j P dP = D makes b linear in sums that need no
   // dd), which also computes D and clears the status word, so there is no pre-pass
   if (use_tc(*p)) return tc_operator(*p, s);
@@ -379,6 +390,7 @@ int fhob_forward(const FhobProblem* p, void* o_out, float* lse_out, void* stream
     if (tc) return FHOB_ERR_WORKSPACE;
     status = nullptr;   // the CUDA-core kernel only clears the word: it does without one
   }
+  std::lock_guard<std::mutex> together(workspace_lock(p->workspace));   // fp32 on the tensor cores: the hi/lo copies
   return tc ? tc_forward(*p, o_out, lse_out, status, s) : simt_forward(*p, o_out, lse_out, status, s);
 }
 
@@ -387,6 +399,7 @@ int fhob_backward(const FhobProblem* p, void* dq, void* dk, void* dv, void* stre
   int st = validate(p, false, false);
   if (st != FHOB_OK) return st;
   if (!aligned16(dq) || !aligned16(dk) || !aligned16(dv)) return FHOB_ERR_ALIGN;
+  std::lock_guard<std::mutex> together(workspace_lock(p->workspace));
   st = run_prepass(p, stream, false);  // stores -L*log2(e) and -D in the workspace
   if (st != FHOB_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);

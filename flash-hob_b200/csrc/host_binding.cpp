@@ -119,7 +119,8 @@ bool fill_lse(Call& c, const Tensor& lse) {
   return (reinterpret_cast<uintptr_t>(c.p.lse) & 15u) == 0;
 }
 
-// The stream and its workspace, from the dict the Python path uses too (needs the GIL).  Memory
+// The stream and its workspace, from the dict the Python path uses too (needs the GIL).  Threads on one stream
+// share it: the library queues the kernels of a call without another's between them.  Memory
 // allocated while a stream is captured belongs to the graph: that is left to the Python path.
 bool take_workspace(Call& c, Tensor& keep) {
   if (at::cuda::currentStreamCaptureStatusMayInitCtx() != at::cuda::CaptureStatus::None) return false;

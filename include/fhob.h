@@ -10,7 +10,10 @@
  * Every entry point takes plain device pointers and sizes, launches on the
  * CUDA stream it is given and returns an int status (0 = ok).  No entry point
  * allocates device memory unless its comment says so; scratch is a caller
- * provided workspace of fhob_workspace_bytes() bytes.
+ * provided workspace of fhob_workspace_bytes() bytes.  fhob_bwdbwd,
+ * fhob_forward and fhob_backward queue all their kernels without another
+ * such call's on the same workspace coming between, so host threads that
+ * share a stream may share a workspace; on different streams they may not.
  *
  * Layout: every matrix is row-major (BH, N, D) with the batch and head axes
  * folded into BH like the reference does (fhog/triton_bwdbwd.py:577), rows
