@@ -9,6 +9,7 @@ CUDA kernels, and a missing library is an error rather than a fallback.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from typing import Optional, Tuple
 
 import torch
@@ -319,11 +320,13 @@ def flash_bwdbwd(Q, K, V, O, dO, ddQ, ddK, ddV, L, scale, *, is_causal: bool = F
     if workspace is not None:
         raise ValueError("workspace= is only supported for device tensors")
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    return _run_host((Q, K, V, O, dO, ddQ, ddK, ddV), L, scale, is_causal, impl, check is None or bool(check), dev,
-                     window=sliding_window, out=out)
+    with _host_locks.setdefault(dev.index, threading.Lock()):   # a call ends synchronised: the next finds the sets idle
+        return _run_host((Q, K, V, O, dO, ddQ, ddK, ddV), L, scale, is_causal, impl, check is None or bool(check), dev,
+                         window=sliding_window, out=out)
 
 
 _copy_streams: dict = {}
+_host_locks: dict = {}  # one host-buffer call at a time and device: its copy streams and staging sets are shared
 _staging: dict = {}     # (device, heads per range, shapes) -> ring of device staging sets of the host-buffer path
 HOST_STAGES = 3
 HOST_RANGE_BYTES = 192 << 20   # input bytes staged per head range on the host-buffer path (measured best of 48-768 MB)

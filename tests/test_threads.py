@@ -55,3 +55,19 @@ def test_threads_on_one_stream_get_their_own_results(dtype, d, caller):
     for r, results in zip(ref, got):
         for g in results:
             assert all(torch.equal(a, b) for a, b in zip(g, r))
+
+
+@pytest.mark.gpu
+def test_threads_with_host_tensors_get_their_own_results():
+    """Calls of one shape stage through the same device buffers."""
+    import fhob
+    jobs, ref = [], []
+    for seed in (1, 2, 3):
+        x = make_inputs(8, 256, 256, 64, seed=seed, dtype=torch.bfloat16, device="cuda")
+        o, lse = fhob.attention_forward(x["q"], x["k"], x["v"], 0.1)
+        args = [t.cpu().pin_memory() for t in (x["q"], x["k"], x["v"], o, x["do"], x["ddq"], x["ddk"], x["ddv"], lse)]
+        jobs.append(lambda args=args: fhob.flash_bwdbwd(*args, 0.1))
+        ref.append(jobs[-1]())
+    for r, results in zip(ref, _in_threads(jobs, 20)):
+        for g in results:
+            assert all(torch.equal(a, b) for a, b in zip(g, r))
