@@ -26,10 +26,12 @@ namespace {
 // 128 elements) takes kPrepassRows query rows of one head, their loads all issued before the sums:
 // D = sum_d dO*O, stored as k1 = -D, and nlc = -L*log2(e).
 // Block 0 also clears the status word, so every operator call starts clean.
+// Plain pointers: o and lse may be what the kernel in front writes while this one starts, and the compiler may
+// take a load through a const __restrict__ pointer for one of memory that does not change, and move it to
+// before the wait.
 constexpr int kPrepassRows = 4;
 template <typename T>
-__global__ void prepass_kernel(const T* __restrict__ o, const T* __restrict__ d_o, const float* __restrict__ lse,
-                               float* __restrict__ nlc, float* __restrict__ k1, int* status, unsigned blocks_per_head, int d,
+__global__ void prepass_kernel(const T* o, const T* d_o, const float* lse, float* nlc, float* k1, int* status, unsigned blocks_per_head, int d,
                                int n_q, int first_live_query, View vo, View vdo, long long lse_head,
                                long long lse_batch, int lanes) {
   ptx::pdl_wait();
@@ -48,11 +50,14 @@ __global__ void prepass_kernel(const T* __restrict__ o, const T* __restrict__ d_
   // a query the causal mask leaves without any visible key (n_k < n_q): every P of its row is
   // masked to zero in the passes, so the row contributes nothing and its dQ2 and ddO are zero.
   // Its saved L (-inf) and O (0 or NaN, depending on who produced them) are not looked at.
+  const float* lse_h = lse + static_cast<long long>(hb) * lse_batch + static_cast<long long>(hh) * lse_head;
   uint4 a[kPrepassRows], b[kPrepassRows];
+  float l[kPrepassRows];
 #pragma unroll
   for (int r = 0; r < kPrepassRows; ++r) {
     const int qi = q0 + r * groups;
     a[r] = b[r] = make_uint4(0u, 0u, 0u, 0u);
+    l[r] = c == 0 && qi < n_q && qi >= first_live_query ? lse_h[qi] : 0.f;
     if (o != nullptr && c < d && qi < n_q && qi >= first_live_query) {
       a[r] = *reinterpret_cast<const uint4*>(po + qi * vo.row);
       b[r] = *reinterpret_cast<const uint4*>(pd + qi * vdo.row);
@@ -60,7 +65,6 @@ __global__ void prepass_kernel(const T* __restrict__ o, const T* __restrict__ d_
   }
   float* nlc_head = nlc + static_cast<long>(bh) * row_stride(n_q);
   float* k1_head = k1 + static_cast<long>(bh) * row_stride(n_q);
-  const float* lse_h = lse + static_cast<long long>(hb) * lse_batch + static_cast<long long>(hh) * lse_head;
 #pragma unroll
   for (int r = 0; r < kPrepassRows; ++r) {
     const int qi = q0 + r * groups;
@@ -76,7 +80,7 @@ __global__ void prepass_kernel(const T* __restrict__ o, const T* __restrict__ d_
       k1_head[qi] = 0.f;
       continue;
     }
-    nlc_head[qi] = -lse_h[qi] * kLog2e;
+    nlc_head[qi] = -l[r] * kLog2e;
     // no O: D comes out of the sweep that yields dd and b (sum_j P dP), which then writes k1
     if (o != nullptr) k1_head[qi] = -acc;
   }
