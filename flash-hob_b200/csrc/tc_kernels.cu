@@ -143,7 +143,7 @@ struct Bars {
   uint64_t q_full[2];   // passes 3, 4 deep: dS/dS2 written into group-A stage [i]
   uint64_t out_full;
   uint64_t s_ready;      // passes 3, 4: the stacked product [S | Q.ddK^T] of a tile has finished
-  uint64_t chain_go;     // passes 3, 4: chain 1 has issued its products of this round (chain 2 may follow)
+  uint64_t chain_go[2];  // passes 3, 4: chain 1 has issued its products of this round (chain 2 may follow), in turn
   uint64_t teardown[2];
   uint32_t tmem_base;
   int abort_flag;
@@ -477,7 +477,8 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
       mbar_init(&bars->q_full[i], EW_THREADS);
     }
     mbar_init(&bars->out_full, 2);
-    mbar_init(&bars->chain_go, 1);
+    mbar_init(&bars->chain_go[0], 1);
+    mbar_init(&bars->chain_go[1], 1);
     mbar_init(&bars->s_ready, 1);
     mbar_init(&bars->teardown[0], 1);
     mbar_init(&bars->teardown[1], 1);
@@ -689,9 +690,11 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
           commit(&bars->strm_free[it % C::NSLOT]);
           // Chain 1's group A of the next tile gates the next elementwise half, while chain 2's
           // group B is needed half a tile later: chain 2 lets chain 1 issue first, so the tensor
-          // pipe runs them in that order.
+          // pipe runs them in that order.  Two barriers in turn: chain 1's next signal only waits for the
+          // first elementwise half of the next tile, so it may come before chain 2 has looked at this one,
+          // and a barrier that is two phases on looks as if it had not moved.  (The third waits for chain 2.)
           if (chain == 1) {
-            ok = wait_all(&bars->chain_go, it & 1);
+            ok = wait_all(&bars->chain_go[it & 1], (it >> 1) & 1);
             if (!ok) break;
           }
           if (it + 1 < n_iter) {
@@ -699,7 +702,7 @@ __device__ __forceinline__ void tc_pass_body(const TcParams& p, int block) {
             if (!ok) break;
             commit(&bars->s_full[chain]);
           }
-          if (chain == 0) mbar_arrive(&bars->chain_go);
+          if (chain == 0) mbar_arrive(&bars->chain_go[it & 1]);
         }
       }
       if (ok) {
