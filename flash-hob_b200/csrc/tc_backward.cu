@@ -31,17 +31,21 @@ constexpr int BW_RING = 5;      // most slots of a ring
 // Two head dims: the first stationary and the first streamed tile are q/k-side tensors (DQK columns), the
 // second ones v-side tensors (DV columns).  BQ: Q, dO | K, V.  BK: K, V | Q, dO.
 // SPLIT: fp32 operands as bf16 hi + lo pairs, rows [hi(64) | lo(64)] = the two boxes of a 128-wide tile, three
-// products per contraction (see tc_kernels.cu); 64 columns a result.
+// products per contraction (see tc_kernels.cu); 64 columns a result.  A result's accumulator has 128 columns:
+// hi.hi in the first 64, hi.lo and lo.hi in the others, added up at the end.  The tensor core cuts off low bits
+// every time it adds to an accumulator, so the two small terms must not be added to the large one tile by
+// tile: with all three in 64 columns dV of 8 causal heads N = 2048 is off by 1.25e-5, this way by 7.1e-6.
 template <bool KSIDE, int DQK, int DV, bool SPLIT>
 struct BwCfg {
-  static constexpr int OUT0 = SPLIT ? 64 : DQK;                          // TMEM columns of dQ | dK
-  static constexpr int OUT1 = KSIDE ? (SPLIT ? 64 : DV) : 0;             // dV
+  static constexpr int OUT0 = DQK;                                       // TMEM columns of dQ | dK
+  static constexpr int OUT1 = KSIDE ? DV : 0;                            // dV
   static constexpr int OUT_COLS = OUT0 + OUT1;
+  static constexpr int W0 = SPLIT ? 64 : OUT0, W1 = SPLIT && KSIDE ? 64 : OUT1;   // columns of the results
   // 128 streamed rows a tile if S and two dP of that width fit beside the results
   static constexpr int BN = OUT_COLS + 3 * 128 <= TMEM_COLS && !(SPLIT && KSIDE) ? 128 : 64;
   // split P and dS do not fit dP's columns together: P goes over S then, and S has as many stages as dP
   static constexpr bool P_OVER_S = SPLIT && KSIDE;
-  static constexpr int ND = BN == 128 ? 2 : 3;
+  static constexpr int ND = BN == 128 || P_OVER_S ? 2 : 3;
   static constexpr int NS = P_OVER_S ? ND : 1;
   static constexpr int S_COL = OUT_COLS, DP_COL = OUT_COLS + NS * BN;
   static constexpr int STAT0 = BM * DQK * 2, STAT1 = BM * DV * 2;
@@ -53,9 +57,9 @@ struct BwCfg {
   static constexpr int N1_FIT = ROOM / (SLOT0 + SLOT1), N1 = N1_FIT > BW_RING ? BW_RING : N1_FIT;
   static constexpr int N0_FIT = (ROOM - N1 * SLOT1) / SLOT0, N0 = N0_FIT > BW_RING ? BW_RING : N0_FIT;
   static constexpr int SMEM_BYTES = STAT0 + STAT1 + N0 * SLOT0 + N1 * SLOT1 + BW_TAIL;
-  static constexpr int kPitch = OUT_COLS + 4;                            // floats per row of the staging area (split streamed axis)
+  static constexpr int kPitch = W0 + W1 + 4;                             // floats per row of the staging area (split streamed axis)
   static_assert(DP_COL + ND * BN <= TMEM_COLS, "TMEM budget");
-  static_assert(N0 >= 2 && N1 >= ND, "slots of a ring: the issuing thread is ND tiles ahead with dP");
+  static_assert(N0 >= 2 && N0 >= NS && N1 >= ND, "slots of a ring: the issuing thread is ND tiles ahead with dP, NS with S");
   static_assert(BM * kPitch * 4 <= SMEM_BYTES - BW_TAIL, "staging area");
 };
 
@@ -201,6 +205,7 @@ __device__ __forceinline__ void bw_body(const BwParams& p, int block) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(BM, BN, false, false, F16);
       constexpr uint32_t idesc_o0 = umma_idesc_bf16(BM, C::OUT0, false, true, F16);                 // dQ | dK
       constexpr uint32_t idesc_o1 = umma_idesc_bf16(BM, C::OUT1 ? C::OUT1 : 64, false, true, F16);  // dV
+      constexpr uint32_t idesc_o64 = umma_idesc_bf16(BM, 64, false, true, F16);                     // split operands: the hi box alone
       constexpr int kStatBox = BM * 128, kBox = BN * 128;
       const uint32_t stat0 = umma_desc_lo(smem_u32(smem), 16), stat1 = stat0 + (C::STAT0 >> 4);
       const uint32_t r0 = umma_desc_lo(smem_u32(ring0), 16), r1 = umma_desc_lo(smem_u32(ring1), 16);
@@ -240,10 +245,7 @@ __device__ __forceinline__ void bw_body(const BwParams& p, int block) {
       auto outputs = [&](uint32_t out, uint32_t a, int lo, uint32_t tile, uint32_t idesc, bool accumulate) {
         const uint32_t b = tile - (1u << 16) + (static_cast<uint32_t>(kBox >> 4) << 16);
         gemm_ts<BN>(out, a, b, idesc, accumulate);
-        if constexpr (SPLIT) {
-          gemm_ts<BN>(out, a, b + (kBox >> 4), idesc, true);   // hi . lo
-          gemm_ts<BN>(out, a + lo, b, idesc, true);            // lo . hi
-        }
+        if constexpr (SPLIT) gemm_ts<BN>(out + 64, a + lo, b, idesc_o64, true);   // hi . [hi | lo] above, lo . hi here
       };
       wait(&bars->stat_full, 0);
       for (int t = 0; ok && t < C::ND && t < n_iter; ++t) {
@@ -423,23 +425,17 @@ __device__ __forceinline__ void bw_body(const BwParams& p, int block) {
     tc_fence_after();
     if (split > 1) {
       float* dst = reinterpret_cast<float*>(smem) + row * C::kPitch;   // every tile has been read: out_full follows the last product
-      stage_row<C::OUT0 / 2>(dst + half * (C::OUT0 / 2), lane_base + half * (C::OUT0 / 2), n_iter > 0);
-      if constexpr (KSIDE) stage_row<C::OUT1 / 2>(dst + C::OUT0 + half * (C::OUT1 / 2), lane_base + C::OUT0 + half * (C::OUT1 / 2), n_iter > 0);
+      stage_row<C::W0 / 2, SPLIT>(dst + half * (C::W0 / 2), lane_base + half * (C::W0 / 2), n_iter > 0);
+      if constexpr (KSIDE) stage_row<C::W1 / 2, SPLIT>(dst + C::W0 + half * (C::W1 / 2), lane_base + C::OUT0 + half * (C::W1 / 2), n_iter > 0);
     } else if (ok && live) {
       // `width` columns from TMEM column col0 on; dS was stored without the scale
       auto store_out = [&](auto width, int d_mem, uint32_t col0, void* base, float mul) {
-        constexpr int W = decltype(width)::value;   // columns of the accumulator; d_mem <= W of them exist in memory
+        constexpr int W = decltype(width)::value;   // columns of the result; d_mem <= W of them exist in memory
         const size_t at = (static_cast<size_t>(head) * n_stat + g_row) * d_mem;
 #pragma unroll
         for (int c = half * (W / 2); c < (half + 1) * (W / 2); c += 16) {
           uint32_t v[16];
-          if (n_iter > 0) {
-            tmem_ld16(lane_base + col0 + c, v);
-            tmem_wait_ld();
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = 0u;
-          }
+          load_result<SPLIT>(lane_base + col0 + c, n_iter > 0, v);
           if (g_row >= n_stat) continue;
           if constexpr (SPLIT) {
 #pragma unroll
@@ -459,8 +455,8 @@ __device__ __forceinline__ void bw_body(const BwParams& p, int block) {
           }
         }
       };
-      store_out(std::integral_constant<int, C::OUT0>{}, p.d, 0, KSIDE ? p.dk : p.dq, p.scale);
-      if constexpr (KSIDE) store_out(std::integral_constant<int, C::OUT1>{}, p.d_v, C::OUT0, p.dv, 1.f);
+      store_out(std::integral_constant<int, C::W0>{}, p.d, 0, KSIDE ? p.dk : p.dq, p.scale);
+      if constexpr (KSIDE) store_out(std::integral_constant<int, C::W1>{}, p.d_v, C::OUT0, p.dv, 1.f);
     }
   }
 
@@ -470,8 +466,8 @@ __device__ __forceinline__ void bw_body(const BwParams& p, int block) {
     cluster_sync();
     const int tid = threadIdx.x - EW_WARP0 * 32, rank0 = static_cast<int>(cluster_rank()) - part;
     if (split > 1 && live && tid >= 0) {
-      reduce_store<C::OUT0, SPLIT, F16>(smem_u32(smem), C::kPitch, 0, rank0, part, split, tid, KSIDE ? p.dk : p.dq, head, m0, n_stat, p.d, p.scale);
-      if constexpr (KSIDE) reduce_store<C::OUT1, SPLIT, F16>(smem_u32(smem), C::kPitch, C::OUT0, rank0, part, split, tid, p.dv, head, m0, n_stat, p.d_v, 1.f);
+      reduce_store<C::W0, SPLIT, F16>(smem_u32(smem), C::kPitch, 0, rank0, part, split, tid, KSIDE ? p.dk : p.dq, head, m0, n_stat, p.d, p.scale);
+      if constexpr (KSIDE) reduce_store<C::W1, SPLIT, F16>(smem_u32(smem), C::kPitch, C::W0, rank0, part, split, tid, p.dv, head, m0, n_stat, p.d_v, 1.f);
     }
     cluster_sync();   // the others are done with this CTA's shared memory
   }

@@ -173,19 +173,32 @@ __device__ __forceinline__ void split_range(int part, int split, int& begin, int
   end = b + static_cast<int>(static_cast<long long>(n) * (part + 1) / split);
 }
 
-// This thread's W fp32 accumulator columns (TMEM addresses taddr..) of its row -> staging area.
-template <int W>
+// 16 fp32 columns of this thread's row of a finished result at TMEM address taddr (zeros if there was nothing
+// to add up).  HALVES: the result is the sum of two accumulators, 64 columns apart (split operands).
+template <bool HALVES>
+__device__ __forceinline__ void load_result(uint32_t taddr, bool any, uint32_t (&v)[16]) {
+  if (any) {
+    [[maybe_unused]] uint32_t w[16];
+    tmem_ld16(taddr, v);
+    if constexpr (HALVES) tmem_ld16(taddr + 64, w);
+    tmem_wait_ld();
+    if constexpr (HALVES) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = 0u;
+  }
+}
+
+// This thread's W fp32 result columns (TMEM addresses taddr..) of its row -> staging area.
+template <int W, bool HALVES = false>
 __device__ __forceinline__ void stage_row(float* dst, uint32_t taddr, bool any) {
 #pragma unroll
   for (int c = 0; c < W; c += 16) {
     uint32_t v[16];
-    if (any) {
-      tmem_ld16(taddr + c, v);
-      tmem_wait_ld();
-    } else {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = 0u;
-    }
+    load_result<HALVES>(taddr + c, any, v);
 #pragma unroll
     for (int j = 0; j < 16; j += 4)
       *reinterpret_cast<uint4*>(dst + c + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);

@@ -102,14 +102,15 @@ __device__ __forceinline__ void fw_split_pack(float x, float y, uint32_t& hi, ui
 }
 
 // fp32 problems (SPLIT): every fp32 operand as bf16 hi + lo, rows [hi(64) | lo(64)] = the two boxes of a
-// 128-wide tile; a contraction is hi.hi + hi.lo + lo.hi (see tc_kernels.cu).  Head dims up to 64.
+// 128-wide tile; a contraction is hi.hi + hi.lo + lo.hi (see tc_kernels.cu).  Head dims up to 64.  The small
+// terms of P V have an accumulator of their own (see BwCfg in tc_backward.cu).
 template <int DQK, int DV, bool F16, bool SPLIT, bool OUT>
 __global__ void __launch_bounds__(FW_THREADS, 1) fw_kernel(const __grid_constant__ FwParams p) {
   using C = FwCfg<DQK, DV, OUT>;
   static_assert(!SPLIT || (DQK == 128 && DV == 128 && !F16), "split fp32 operands are [hi(64) | lo(64)] bf16 rows");
   constexpr int BN = C::BN, kStages = C::STAGES;
   constexpr bool kHalves = OUT && BN == 128;   // P handed over in two halves
-  constexpr int kO = SPLIT ? 64 : DV;   // columns of an O accumulator
+  constexpr int kO = DV, kRes = SPLIT ? 64 : DV;   // columns of an O accumulator (split: [hi.hi | hi.lo + lo.hi]) and of O
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* ring = smem + 2 * C::Q_BYTES;
   FwBars* bars = reinterpret_cast<FwBars*>(ring + C::NSLOT * C::SLOT_BYTES);
@@ -229,6 +230,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) fw_kernel(const __grid_constant
     if (n_tiles > 0 && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(BM, BN, false, false, F16);
       constexpr uint32_t idesc_o = umma_idesc_bf16(BM, kO, false, true, F16);
+      constexpr uint32_t idesc_o64 = umma_idesc_bf16(BM, 64, false, true, F16);   // split operands: the hi box alone
       constexpr int kBox = BM * 128;
       const uint32_t q_lo = umma_desc_lo(smem_u32(smem), 16), ring_lo = umma_desc_lo(smem_u32(ring), 16);
       constexpr uint32_t kQ16 = C::Q_BYTES >> 4, kSlot16 = C::SLOT_BYTES >> 4;
@@ -267,22 +269,22 @@ __global__ void __launch_bounds__(FW_THREADS, 1) fw_kernel(const __grid_constant
         tc_fence_after();
         // MN-major: leading byte offset = distance between the tile's 64-column boxes
         const uint32_t b = ring_lo + slot * kSlot16 - (1u << 16) + (static_cast<uint32_t>((BN * 128) >> 4) << 16);
-        auto pv = [&](uint32_t a_cols, uint32_t b_off, int k0, int k1, bool accumulate) {
+        auto pv = [&](int k0, int k1, bool accumulate) {
 #pragma unroll
           for (int ks = k0; ks < k1; ++ks)
-            umma_ts_split(o_cols(x), s_cols(x, stage) + a_cols + 8 * ks, b + ((b_off + ks * 2048) >> 4), kDescHi, idesc_o,
-                          accumulate || ks > k0 ? 1u : 0u);
+            umma_ts_split(o_cols(x), s_cols(x, stage) + 8 * ks, b + ((ks * 2048) >> 4), kDescHi, idesc_o, accumulate || ks > k0 ? 1u : 0u);
         };
         constexpr int kFirst = kHalves ? BN / 32 : BN / 16;
-        pv(0, 0, 0, kFirst, it > 0);
+        pv(0, kFirst, it > 0);
         if (kHalves) {
           if (!wait(&bars->p_full[x][stage], it & 1)) return;
           tc_fence_after();
-          pv(0, 0, kFirst, BN / 16, true);
+          pv(kFirst, BN / 16, true);
         }
-        if (SPLIT) {   // P_hi . V_lo, P_lo . V_hi
-          pv(0, BN * 128, 0, BN / 16, true);
-          pv(BN / 2, 0, 0, BN / 16, true);
+        if (SPLIT) {   // above P_hi . [V_hi | V_lo]; here P_lo . V_hi on top of the second half
+#pragma unroll
+          for (int ks = 0; ks < BN / 16; ++ks)
+            umma_ts_split(o_cols(x) + 64, s_cols(x, stage) + BN / 2 + 8 * ks, b + ((ks * 2048) >> 4), kDescHi, idesc_o64, 1u);
         }
         umma_commit(&bars->o_done[x]);
         if (t + 1 == end[x]) umma_commit(&bars->out_full[x]);
@@ -446,7 +448,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) fw_kernel(const __grid_constant
     if (p.split > 1) {
       // this part's row: unscaled O, reference maximum and sum (query tile A only)
       if (x == 0) {
-        if (OUT) stage_row<kO>(reinterpret_cast<float*>(smem) + row * C::kPitch, o_addr, n_iter > 0);
+        if (OUT) stage_row<kRes, SPLIT>(reinterpret_cast<float*>(smem) + row * C::kPitch, o_addr, n_iter > 0);
         bars->red[0][row] = run_m;
         bars->red[1][row] = run_l;
       }
@@ -458,15 +460,9 @@ __global__ void __launch_bounds__(FW_THREADS, 1) fw_kernel(const __grid_constant
       if (OUT) {
         const size_t at = (static_cast<size_t>(head) * p.n_q + g_row) * p.d_v;
 #pragma unroll
-        for (int c = 0; c < kO; c += 16) {
+        for (int c = 0; c < kRes; c += 16) {
           uint32_t v[16];
-          if (n_iter > 0) {
-            tmem_ld16(o_addr + c, v);
-            tmem_wait_ld();
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = 0u;
-          }
+          load_result<SPLIT>(o_addr + c, n_iter > 0, v);
           if (g_row < p.n_q) {
             if constexpr (SPLIT) {
 #pragma unroll
@@ -498,7 +494,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) fw_kernel(const __grid_constant
     cluster_sync();
     const int tid = threadIdx.x - FW_EW_WARP0 * 32, m0 = m_of(0);
     if (tid >= 0) {
-      constexpr int V = SPLIT ? 4 : 8, PIECES = OUT ? kO / V : 1;
+      constexpr int V = SPLIT ? 4 : 8, PIECES = OUT ? kRes / V : 1;
       const int rows = (BM + p.split - 1) / p.split;
       const uint32_t stage = smem_u32(smem), red = smem_u32(&bars->red[0][0]);
       for (int i = tid; i < rows * PIECES; i += EW_THREADS) {
