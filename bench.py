@@ -65,12 +65,13 @@ EXEC_OVER_ALG = sum(GEMM_UNITS.values()) / 12.0
 # dram__bytes_read.sum + dram__bytes_write.sum per head of one launch of each pass at N_Q=4096,
 # N_K=8192, D=128, from an ncu capture of a 16-head case (every head has its own tensors, so the
 # traffic of a launch grows in proportion to its heads).
-DRAM_BYTES_PER_HEAD = {("cfg5", "pass12"): 190.32e6 / 16, ("cfg5", "pass3"): 213.21e6 / 16,
-                       ("cfg5", "pass4"): 229.11e6 / 16}
-# template arguments: pass, head dim of q/k, head dim of v, streamed rows, fused dd+b sweep, fp16 storage,
-# split fp32 operands
+DRAM_BYTES_PER_HEAD = {("cfg5", "pass12"): 207.12e6 / 16, ("cfg5", "pass3"): 207.02e6 / 16,
+                       ("cfg5", "pass4"): 229.58e6 / 16}
+# template arguments: [pass,] head dim of q/k, head dim of v, [streamed rows, fused dd+b sweep,] fp16 storage, split
+# fp32 operands.  A call launches passes 3 and 4 together; the per-pass figures come from a launch of either alone.
 KERNEL_NAMES = {"pass12": "tc_pass_kernel<2, {d}, {d}, 64, 1, 0, 0>",
-                "pass3": "tc_pass_kernel<3, {d}, {d}, 64, 0, 0, 0>", "pass4": "tc_pass_kernel<4, {d}, {d}, 64, 0, 0, 0>"}
+                "pass3": "tc_pass34_kernel<{d}, {d}, 0, 0> (pass 3 alone)",
+                "pass4": "tc_pass34_kernel<{d}, {d}, 0, 0> (pass 4 alone)"}
 METRIC = "double_backward_attention_tflops"
 
 _JSON_FD = None
@@ -101,6 +102,11 @@ def pairs(w):
         assert w["n_q"] == w["n_k"]
         return w["n_q"] * (w["n_q"] + 1) // 2
     return w["n_q"] * w["n_k"]
+
+
+def launches_per_call(w):
+    """Kernels of one operator call: the sweep, passes 3 and 4 together; fp32: the split copies in front."""
+    return 3 if w.get("dtype") == "f32" else 2
 
 
 def f_alg(w, heads=None):
@@ -808,7 +814,7 @@ def main():
         passes=passes, roofline=roofline, parity_of_timed_outputs=dict(
             max_rel_err_vs_fp64_oracle=parity, head="last head of rank 0's shard", tolerance=2e-2),
         producers=producers, cpu_baseline=cpu_baseline, e2e=e2e, clocks=clocks,
-        gpu_launches=4 * args.steps * rounds, peak_mem_bytes=peak_mem,
+        gpu_launches=launches_per_call(w) * args.steps * rounds, peak_mem_bytes=peak_mem,
         other_configs=extras, mem_sweep=sweep, competitor_triton=competitor)
     emit(line)
     if world > 1:

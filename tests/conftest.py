@@ -28,6 +28,20 @@ def pytest_collection_modifyitems(config, items):
             item.add_marker(skip)
 
 
+@pytest.fixture(autouse=True)
+def no_expired_wait(request):
+    """A bounded device wait that ran out in a call whose status nobody read leaves wrong results: fail the test
+    after the last call on each workspace."""
+    yield
+    if "gpu" not in request.keywords or not torch.cuda.is_available():
+        return
+    from fhob import _lib, ops
+    for (device, stream), ws in ops._workspaces.items():
+        torch.cuda.synchronize(device)
+        status = int(ws[:4].view(torch.int32))   # (memory that no call has cleared yet may hold anything)
+        assert not (0 <= status < 512 and status & _lib.ERR_TIMEOUT), f"status {status} on stream {stream:#x}"
+
+
 def make_inputs(bh, nq, nk, d, seed, dtype=torch.float32, device="cpu", cot_scale=1.0, on_device=False):
     """Seven seeded N(0,1) tensors with bf16-representable values.
 

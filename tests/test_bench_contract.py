@@ -3,6 +3,7 @@ the flop accounting of the workloads."""
 from __future__ import annotations
 
 import json
+import re
 import subprocess
 import sys
 
@@ -41,3 +42,10 @@ def test_reference_arm_prints_one_contract_line():
     assert j["cpu_baseline"]["value"] == j["value"] == j["e2e"]["value"] > 0
     assert j["e2e"]["h2d_bytes_per_step"] == 0 and j["e2e"]["d2h_bytes_per_step"] == 0
 
+
+def test_kernels_named_by_the_bench_are_those_of_the_library():
+    source = (ROOT / "flash-hob_b200" / "csrc" / "tc_kernels.cu").read_text()
+    for name in bench.KERNEL_NAMES.values():
+        assert re.search(r"__global__[^;{]*\b" + name.split("<")[0] + r"\(", source), name
+    assert bench.launches_per_call(bench.WORKLOADS["cfg5"]) == 2
+    assert bench.launches_per_call(bench.WORKLOADS["cfg1"]) == 3
