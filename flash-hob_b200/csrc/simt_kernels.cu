@@ -714,9 +714,11 @@ SimtParams make_params(const FhobProblem& p) {
 }
 
 // In streamed tiles (fp32, D = 128: 12 us in passes 3 and 4): what a CTA takes besides its tiles is about one
-// tile's time, meeting in a cluster about half of one.  Operator, fp32, D = 128, us, unsplit -> split: 1 head
-// 64 x 3000 2497 -> 332, 4 heads 200 x 5000 4156 -> 2118; 64 heads 200 x 1000 2390 -> 2411.
-constexpr SplitCost kSimtCost = {1.f, 0.5f};
+// tile's time, meeting in a cluster about half of one.  That is little enough for
+// heads of any number of tiles to be split in two from about 1000 streamed rows on.  Operator, fp32, D = 128, us,
+// unsplit -> split: 1 head 64 x 3000 2497 -> 332, 4 heads 200 x 5000 4156 -> 1086, 1 causal head N = 2000 1719 -> 897;
+// 8 heads N = 1024 1326 -> 1337, 64 heads 9333 -> 9596, causal 5174 -> 5371.
+constexpr SplitCost kSimtCost = {1.f, 0.5f, 1.f / 16};
 
 PairGrid modes_grid(const FhobProblem& p, bool q_side, bool k_side) {
   const int tiles_q = (p.n_q + OM - 1) / OM, tiles_k = (p.n_k + OM - 1) / OM;

@@ -405,13 +405,15 @@ int sm_count() {
 constexpr int kMaxParts = 8;
 struct SplitCost {
   float fixed = 5.f, cluster = 1.f;
+  float any = 0.f;   // heads of any number of tiles are split if that costs at most this much
 };
 inline int split_parts(int stationary_tiles, int streamed_tiles, const SplitCost& cost = SplitCost{}) {
   const float unsplit = static_cast<float>(streamed_tiles) + cost.fixed;
   int parts = kMaxParts;
-  while (parts > 1 && (stationary_tiles > kMaxParts / parts ||
-                       static_cast<float>(streamed_tiles) + parts * (cost.fixed + cost.cluster) > 1.25f * unsplit))
-    parts >>= 1;
+  for (; parts > 1; parts >>= 1) {
+    const float more = streamed_tiles + parts * (cost.fixed + cost.cluster) - unsplit;
+    if (more <= (stationary_tiles <= kMaxParts / parts ? 0.25f : cost.any) * unsplit) break;
+  }
   return parts;
 }
 // Streamed tiles of `tile` rows that the longest item of `rows` stationary rows sees.
